@@ -370,9 +370,9 @@ size_t nectb_train_workspace_bytes(const NectbGeometry* geometry, const NectbHas
  * repeats a pixel) and the backward runs in rounds of equal ray counts
  * (NectbTuning::staged_rounds, 4 by default);
  * each round's tensor-core pass writes dL/d(encoding) of its samples (fp32,
- * num_points_per_ray * n_levels * n_features per ray) and scatter passes over
- * level groups apply it to grid_grad with the gradient slice of each group
- * resident in L2.  The rounds' part is capped at 16 GiB (plus the ray list).
+ * num_points_per_ray, rounded up to a multiple of 4, * n_levels * n_features
+ * per ray) and a scatter over level groups applies it to grid_grad with the
+ * gradient slice of each group resident in L2.  The rounds' part is capped at 16 GiB (plus the ray list).
  * It also includes an encoding store: the forward writes each sample's bf16
  * MLP input row (n_levels * n_features * 2 bytes) there and the backward
  * reads it back instead of gathering the tables a second time (identical
@@ -546,11 +546,13 @@ int nectb_selftest_bounded_wait(unsigned int* error_word, uint32_t max_tries, vo
 /* Launch shapes and scheduling of the mixed training path, process-wide:
  * warpgroups per SM of the forward (1..6), blocks per SM of the tensor-core
  * backward (1..3; the three-layer model's kernel takes at most 2),
- * of the gradient scatter (0 = as many as fit), the rounds the recommended
- * staging is sized for (nectb_train_staging_bytes, 1..64), the largest fp32
- * gradient slice one scatter pass covers, and the samples-per-cell
- * thresholds above which runs of samples along a ray are merged before their
- * reductions (3D and 4D grids), and time_slice: 1 lets a mixed 4D training
+ * of the gradient scatter (0..8, without effect: the staged scatter launches a
+ * warp per work item), the most rounds the recommended staging is sized for
+ * (nectb_train_staging_bytes, 1..64; fewer where a round would stage less
+ * than 1 GiB), the largest fp32 gradient slice the staged scatter works on at
+ * a time, and the samples-per-cell thresholds above which the single-pass
+ * backward merges runs of samples along a ray before their reductions (3D and
+ * 4D grids), and time_slice: 1 lets a mixed 4D training
  * step with staging interpolate the fp16 table at the batch's t once (a 3D
  * slice per level, fp16) and run the 3D kernels on it, the gradient being
  * spread back to the two time vertices afterwards; the slice's fp16 rounding

@@ -1,9 +1,9 @@
 """Launch shapes and scheduling of the mixed training path, tuned per workload.
 
 The library's tunables (NectbTuning, include/nectb.h): blocks per SM of the
-forward, of the tensor-core backward and of the gradient scatter, the rounds
-of the two-pass backward, the gradient slice one scatter pass covers and the
-run-merging thresholds.  None changes results beyond fp32 reassociation.
+forward and of the tensor-core backward, the rounds of the two-pass backward
+and the gradient slice its scatter works on at a time (the run-merging
+thresholds belong to the single-pass backward and are not searched).  None changes results beyond fp32 reassociation.
 ``tune`` runs coordinate descent over them on real training steps of the
 caller's workload (CUDA-event timing on the training stream), keeps the
 fastest setting in the library and returns it; the model and optimizer state
@@ -27,11 +27,8 @@ FIELDS = ("forward_blocks_per_sm", "backward_blocks_per_sm", "scatter_blocks_per
 SPACE = {
     "forward_blocks_per_sm": (4, 5, 6),
     "backward_blocks_per_sm": (2, 3),
-    "scatter_blocks_per_sm": (0, 2, 3),
     "staged_rounds": (4, 8, 16),
     "scatter_group_bytes": (24 << 20, 48 << 20, 96 << 20),
-    "run_threshold_3d": (0.5, 0.75, 1.0),
-    "run_threshold_4d": (0.75, 1.5, 3.0),
 }
 
 

@@ -417,4 +417,184 @@ __device__ __forceinline__ void scatter_warp(const GridDev& g, float* __restrict
   }
 }
 
+// Reduces (fp32 add, relaxed, device scope) the even vertex's sums e into entry
+// ie where xe is non-zero and the odd vertex's sums o into entry io where xo
+// is, and clears those sums; with two features, both in one 16-byte reduction
+// where their entries form an aligned pair.  Predicated, without branches:
+// the lanes of a warp rarely agree on which vertices to reduce.
+template <int F>
+__device__ __forceinline__ void reduce_row(float* base, uint32_t ie, uint32_t io, uint32_t xe, uint32_t xo, float* e,
+                                           float* o) {
+  static_assert(F == 2 || F == 4, "F must be 2 or 4");
+  if constexpr (F == 2) {
+    asm volatile(
+        "{\n\t.reg .pred pe, po, pp, ps, q;\n\t.reg .b32 t;\n\t.reg .b64 ap, ae, ao;\n\t"
+        ".reg .f32 x0, x1, x2, x3;\n\t"
+        "setp.ne.u32 pe, %7, 0;\n\tsetp.ne.u32 po, %8, 0;\n\tand.pred q, pe, po;\n\t"
+        "xor.b32 t, %5, %6;\n\tsetp.eq.and.u32 pp, t, 1, q;\n\t"
+        "and.b32 t, %5, 1;\n\tsetp.ne.u32 ps, t, 0;\n\t"
+        "selp.f32 x0, %2, %0, ps;\n\tselp.f32 x1, %3, %1, ps;\n\t"
+        "selp.f32 x2, %0, %2, ps;\n\tselp.f32 x3, %1, %3, ps;\n\t"
+        "and.b32 t, %5, -2;\n\tmad.wide.u32 ap, t, 8, %4;\n\t"
+        "mad.wide.u32 ae, %5, 8, %4;\n\tmad.wide.u32 ao, %6, 8, %4;\n\t"
+        "@pp red.relaxed.gpu.global.add.v4.f32 [ap], {x0, x1, x2, x3};\n\t"
+        "setp.ne.and.u32 q, %7, 0, !pp;\n\t"
+        "@q red.relaxed.gpu.global.add.v2.f32 [ae], {%0, %1};\n\t"
+        "setp.ne.and.u32 q, %8, 0, !pp;\n\t"
+        "@q red.relaxed.gpu.global.add.v2.f32 [ao], {%2, %3};\n\t"
+        "selp.f32 %0, 0f00000000, %0, pe;\n\tselp.f32 %1, 0f00000000, %1, pe;\n\t"
+        "selp.f32 %2, 0f00000000, %2, po;\n\tselp.f32 %3, 0f00000000, %3, po;\n\t}\n"
+        : "+f"(e[0]), "+f"(e[1]), "+f"(o[0]), "+f"(o[1])
+        : "l"(base), "r"(ie), "r"(io), "r"(xe), "r"(xo)
+        : "memory");
+  } else {
+    auto one = [&](uint32_t i, uint32_t x, float* v) {
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t.reg .b64 a;\n\tsetp.ne.u32 p, %6, 0;\n\tmad.wide.u32 a, %5, 16, %4;\n\t"
+          "@p red.relaxed.gpu.global.add.v4.f32 [a], {%0, %1, %2, %3};\n\t"
+          "selp.f32 %0, 0f00000000, %0, p;\n\tselp.f32 %1, 0f00000000, %1, p;\n\t"
+          "selp.f32 %2, 0f00000000, %2, p;\n\tselp.f32 %3, 0f00000000, %3, p;\n\t}\n"
+          : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3])
+          : "l"(base), "r"(i), "r"(x)
+          : "memory");
+    };
+    one(ie, xe, e);
+    one(io, xo, o);
+  }
+}
+
+// One thread's march over points of one level: the gradient sums of the eight
+// vertices of its current cell stay in registers and a vertex is reduced into
+// the table once, when the march leaves it.  Slot r * 2 + b holds the vertex
+// whose axis-0 coordinate has parity b and whose axis-1 and axis-2 coordinates
+// have parities r & 1 and r >> 1: a cell's vertices have distinct parities, and
+// a step to a neighbouring cell replaces exactly the slots of the vertices left
+// behind, so nothing moves between registers.  Correct for points in any order;
+// few reductions when consecutive points lie in the same or adjacent cells
+// (consecutive samples of a ray).  D = 4: t (the last coordinate) is the same
+// for every point, the sums are spatial and each goes to both time vertices.
+template <int D, int F, bool kHashed>
+struct CellMarch {
+  uint32_t m1, m2, mask;
+  int res;
+  float* base;              // the level's first gradient entry
+  uint32_t t0 = 0, t1 = 0;  // D = 4: index terms of the two time vertices
+  float wt0 = 1.f, wt1 = 0.f;
+  bool any = false;         // a cell is held
+  // the vertex coordinates of the current cell: even and odd, per axis
+  int v[3][2];
+  float acc[8][F];
+
+  __device__ __forceinline__ CellMarch(const GridDev& g, int l, float* grad, float t) {
+    mask = g.hash_mask;
+    m1 = kHashed ? kPrime1 : g.stride[l][1];
+    m2 = kHashed ? kPrime2 : g.stride[l][2];
+    res = g.res[l][0];
+    base = grad + g.offset[l] * F;
+    if constexpr (D == 4) {
+      const int r = g.res[l][3];
+      const float pt = __fmul_rn(t, (float)r);   // as level_corners
+      int ct = (int)floorf(pt);
+      ct = ct < 0 ? 0 : (ct > r - 1 ? r - 1 : ct);
+      wt1 = pt - (float)ct;
+      wt0 = 1.f - wt1;
+      const uint32_t m3 = kHashed ? kPrime3 : g.stride[l][3];
+      t0 = (uint32_t)ct * m3;
+      t1 = t0 + m3;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k][0] = v[k][1] = 0;
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+#pragma unroll
+      for (int f = 0; f < F; ++f) acc[s][f] = 0.f;
+  }
+
+  // Entry of vertex v0 in the row with index term h.
+  __device__ __forceinline__ uint32_t entry(int v0, uint32_t h) const {
+    return kHashed ? (((uint32_t)v0 ^ h) & mask) : (uint32_t)v0 + h;
+  }
+
+  // Reduces and clears the slots whose vertex changes: x[k][b] is non-zero where
+  // axis k's vertex of parity b does.
+  __device__ __forceinline__ void leave(const uint32_t (*x)[2]) {
+    const uint32_t h1[2] = {(uint32_t)v[1][0] * m1, (uint32_t)v[1][1] * m1};
+    const uint32_t h2[2] = {(uint32_t)v[2][0] * m2, (uint32_t)v[2][1] * m2};
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const uint32_t h = kHashed ? h1[r & 1] ^ h2[r >> 1] : h1[r & 1] + h2[r >> 1];
+      const uint32_t xe = x[0][0] | x[1][r & 1] | x[2][r >> 1], xo = x[0][1] | x[1][r & 1] | x[2][r >> 1];
+      float* e = acc[2 * r];
+      float* o = acc[2 * r + 1];
+      if constexpr (D == 4) {
+        float a[F], b[F];
+        const uint32_t g0 = kHashed ? h ^ t0 : h + t0, g1 = kHashed ? h ^ t1 : h + t1;
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+          a[f] = wt0 * e[f];
+          b[f] = wt0 * o[f];
+        }
+        reduce_row<F>(base, entry(v[0][0], g0), entry(v[0][1], g0), xe, xo, a, b);
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+          a[f] = wt1 * e[f];
+          b[f] = wt1 * o[f];
+          e[f] = xe ? 0.f : e[f];
+          o[f] = xo ? 0.f : o[f];
+        }
+        reduce_row<F>(base, entry(v[0][0], g1), entry(v[0][1], g1), xe, xo, a, b);
+      } else {
+        reduce_row<F>(base, entry(v[0][0], h), entry(v[0][1], h), xe, xo, e, o);
+      }
+    }
+  }
+
+  // Adds d (dL/d of the level's F features) at point x.
+  __device__ __forceinline__ void add(const float* x, const float* d) {
+    uint32_t ch[3][2], moved = 0;
+    int n[3][2];
+    float w[3][2];   // per axis: the weights of the even and the odd vertex
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float p = __fmul_rn(x[k], (float)res);   // as level_corners
+      int ci = (int)floorf(p);
+      ci = ci < 0 ? 0 : (ci > res - 1 ? res - 1 : ci);
+      const float f = p - (float)ci, u = 1.f - f;
+      w[k][0] = (ci & 1) ? f : u;
+      w[k][1] = (ci & 1) ? u : f;
+      n[k][0] = (ci + 1) & ~1;
+      n[k][1] = ci | 1;
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        ch[k][b] = (uint32_t)(n[k][b] ^ v[k][b]);
+        moved |= ch[k][b];
+      }
+    }
+    if (moved != 0u || !any) {
+      if (any) leave(ch);
+      any = true;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        v[k][0] = n[k][0];
+        v[k][1] = n[k][1];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        const float wc = w[0][b] * w[1][r & 1] * w[2][r >> 1];
+#pragma unroll
+        for (int f = 0; f < F; ++f) acc[2 * r + b][f] = fmaf(wc, d[f], acc[2 * r + b][f]);
+      }
+  }
+
+  // Reduces what the march still holds.
+  __device__ __forceinline__ void finish() {
+    const uint32_t all[3][2] = {{1u, 1u}, {1u, 1u}, {1u, 1u}};
+    if (any) leave(all);
+    any = false;
+  }
+};
+
 }  // namespace nectb

@@ -225,6 +225,7 @@ int train_entry(const NectbGeometry* geometry, const NectbHashGrid* grid, const 
     return set_error(NECTB_ERR_WORKSPACE, "workspace of %zu bytes < required %zu", workspace_size, need);
   TrainArgs a;
   a.n_pixels = P * sub;
+  a.n_cols = geometry->nDetector[1];
   a.perm = batch->random_ray_index;
   a.perm_len = batch->random_ray_index_len;
   a.start = batch->starting_ray_index;
@@ -409,7 +410,7 @@ namespace {
 // rays over P (virtual) pixels: ray order and offsets, the staged rounds, the
 // encoding store (when enabled) and a 4D grid's time slice.
 size_t staging_bytes(const NectbHashGrid* grid, int R, int P, int S) {
-  const size_t per_ray = (size_t)S * grid->n_levels * grid->n_features * sizeof(float);
+  const size_t per_ray = (size_t)ray_slots(S) * grid->n_levels * grid->n_features * sizeof(float);
   const NectbTuning tune = current_tuning();
   const size_t row_bytes = (size_t)input_padded(grid->n_levels * grid->n_features) * 2;  // bf16 MLP input row
   const size_t rows = tune.encoding_store ? std::min<size_t>({(size_t)R * S, kEncodingStoreCap / row_bytes,

@@ -35,6 +35,7 @@ struct TrainArgs {
   int64_t start;
   int num_rays;
   int n_pixels;  // nDetector[0] * nDetector[1]
+  int n_cols = 1;  // nDetector[1]
   int S;
   float angle;
   float t;
@@ -70,12 +71,20 @@ enum : unsigned int { kFlagDuplicatePixels = 1u };
 // staging is sized for NectbTuning::staged_rounds, 4 by default).
 constexpr int kMaxStagedRounds = 64;
 constexpr size_t kStagingCap = size_t(16) << 30;  // largest staging buffer recommended
+// A round staging less than this leaves part of the GPU idle in the scatter:
+// batches below it take one round (24,999 rays x 100 samples: the scatter of a
+// step 1.12 ms in four rounds of four level passes, 0.58 ms in one launch).
+constexpr size_t kStagedRoundMin = size_t(1) << 30;
 constexpr int kOrderBlock = 1024;                  // threads of the ray-order kernels
 
 // Stored encodings: the forward writes each sample's bf16 MLP input row, which
 // the backward reads back instead of gathering the tables again.  Largest
 // store the recommended staging size includes.
 constexpr size_t kEncodingStoreCap = size_t(80) << 30;
+
+// Staged samples per ray: S rounded up so that each run of four samples of a
+// ray's features is 16-byte aligned.
+__host__ __device__ inline int ray_slots(int S) { return (S + 3) & ~3; }
 
 inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 inline int order_blocks(int R, int P) { return (std::max(R, P) + kOrderBlock - 1) / kOrderBlock; }
@@ -139,6 +148,7 @@ struct StageLayout {
 };
 
 inline size_t staged_round_bytes(int R, int rounds, size_t per_ray) {
+  rounds = (int)std::max<int64_t>(1, std::min<int64_t>(rounds, (int64_t)((size_t)R * per_ray / kStagedRoundMin)));
   const int64_t per_round = (R + rounds - 1) / rounds;
   return std::min((size_t)per_round * per_ray, kStagingCap / per_ray * per_ray);
 }
@@ -168,8 +178,10 @@ inline StageLayout stage_layout(const Workspace& ws, int R, int P, int S, size_t
       L.xstore = reinterpret_cast<uint4*>(p + ob);
     }
   }
-  L.stage = reinterpret_cast<float*>(p + ob + xbytes);
-  L.per_round = std::min<int64_t>((int64_t)((avail - xbytes) / per_ray), R);
+  // 16-byte aligned rows whatever the caller's workspace pointer
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p + ob + xbytes), pad = ((at + 15) & ~uintptr_t(15)) - at;
+  L.stage = reinterpret_cast<float*>(at + pad);
+  L.per_round = avail < xbytes + pad ? 0 : std::min<int64_t>((int64_t)((avail - xbytes - pad) / per_ray), R);
   if (L.per_round <= 0 || (R + L.per_round - 1) / L.per_round > kMaxStagedRounds) {
     L.per_round = 0;
     L.xstore = nullptr;
@@ -303,13 +315,13 @@ __device__ __forceinline__ int next_ray(unsigned int* cursor, const int32_t* __r
 // or batch positions when the batch repeats a pixel): per-block counts, one
 // block scanning them, and the per-block compaction, so pixel order is kept.
 __global__ void order_count_kernel(const int32_t* __restrict__ slot, const RayRec* __restrict__ recs,
-                                   const unsigned int* __restrict__ ctrl, int R, int P,
+                                   const unsigned int* __restrict__ ctrl, int R, int P, int cols, int sub,
                                    unsigned int* __restrict__ block_sums,
                                    unsigned long long* __restrict__ block_samples);
 __global__ void order_scan_kernel(unsigned int* __restrict__ block_sums, unsigned long long* __restrict__ block_samples,
                                   int n_blocks, unsigned int* __restrict__ ctrl);
 __global__ void order_compact_kernel(const int32_t* __restrict__ slot, const RayRec* __restrict__ recs,
-                                     const unsigned int* __restrict__ ctrl, int R, int P,
+                                     const unsigned int* __restrict__ ctrl, int R, int P, int cols, int sub,
                                      const unsigned int* __restrict__ block_sums,
                                      const unsigned long long* __restrict__ block_samples,
                                      int32_t* __restrict__ order, uint64_t* __restrict__ offs);

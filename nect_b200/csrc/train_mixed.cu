@@ -36,7 +36,16 @@ namespace nectb {
 namespace {
 
 constexpr int kMixThreads = 128;
-constexpr int kScatterThreads = 256;
+// Staged scatter: a warp marches over segments of kScatterSegment samples.  A
+// segment's end reduces the 8 vertices it holds, so longer segments reduce less,
+// shorter ones give small batches more warps: 262,144 rays x 512 took 45.2 /
+// 43.9 / 43.7 ms a step with 16 / 32 / 64 samples, 24,999 rays x 100 took 2.43 /
+// 2.55 / 2.67 ms (before the passes became one launch).
+constexpr int kScatterThreads = 128;
+constexpr int kScatterSegment = 32;
+#ifndef UNR
+#define UNR 1
+#endif
 // Per-warp ray cursor shared by the mixed kernels.
 struct RayCursor {
   int ray = -1;
@@ -282,7 +291,7 @@ fwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
 
 // Staged mode (kStaged): instead of scattering, dL/d(encoding) of every sample
 // is written to the staging buffer, level-major: stage[(l * slots + s) * F + f]
-// with s = (scheduling index - lo) * S + sample, for the rays whose
+// with s = (scheduling index - lo) * ray_slots(S) + sample, for the rays whose
 // scheduling index lies in [lo, hi); scatter_stage_kernel applies it.
 //
 // TMEM (BW columns): [0, T) the transient result of every layer and gradient
@@ -515,7 +524,7 @@ bwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
     tc::tmem_wait_ld();
     if constexpr (kStaged) {
       if (valid) {
-        float* dst = stage + ((int64_t)(cur.sched - lo) * a.S + i) * F;
+        float* dst = stage + ((int64_t)(cur.sched - lo) * ray_slots(a.S) + i) * F;
 #pragma unroll
         for (int l = 0; l < L; ++l) {
           // evict-first: each staged value is read once, by the scatter pass
@@ -818,7 +827,7 @@ bwd_lean_kernel(GridDev grid, const __half* __restrict__ table, const float* __r
       break;
     }
     {
-      float* dst = stage + ((int64_t)(cur.sched - lo) * a.S + i) * F;
+      float* dst = stage + ((int64_t)(cur.sched - lo) * ray_slots(a.S) + i) * F;
 #pragma unroll
       for (int c = 0; c < IN / 16; ++c) {
         float dx[16];
@@ -875,32 +884,89 @@ bwd_lean_kernel(GridDev grid, const __half* __restrict__ table, const float* __r
   }
 }
 
-// Applies staged encoding gradients of the rays with scheduling index in
-// [lo, hi) to the fp32 gradient table, levels [l0, l1) only: a pass touches a
-// slice of the gradient table small enough to stay in L2.  Warp per 32
-// consecutive samples of a ray (the backward's order, so runs of equal cells
-// are merged the same way); no shared memory or TMEM, so many warps per SM
-// keep many reductions in flight.
-template <int D, int F>
-__global__ void __launch_bounds__(kScatterThreads)
-scatter_stage_kernel(GridDev grid, TrainArgs a, const RayRec* __restrict__ recs, const int32_t* __restrict__ slot,
-                     unsigned int* __restrict__ ctrl, const float* __restrict__ stage, int64_t slots, int lo, int hi,
-                     int l0, int l1, float* __restrict__ table_grad, const int32_t* __restrict__ order) {
-  const bool by_pixel = !(ctrl[3] & kFlagDuplicatePixels);
-  const unsigned int n_valid = ctrl[6];
-  const int lane = threadIdx.x & 31;
-  RayCursor cur;
-  while (next_chunk(cur, recs, ctrl + 5, slot, a, by_pixel, lane, lo, hi, order, n_valid)) {
-    const int i = cur.base + lane;
-    float p[4] = {0.f, 0.f, 0.f, 0.f};
-    bool valid = false;
-    if (i < cur.rec.count) valid = sample_point(cur.rec, i, p);
-    if (D == 4) p[3] = a.t;
-    const float* dsrc = stage + ((int64_t)(cur.sched - lo) * a.S + i) * F;
-    scatter_warp<D, F, true>(grid, table_grad, p, valid, dsrc, slots * F, 1,
-                             run_levels(grid, cur.rec.dx, cur.rec.dy, cur.rec.dz, a.run_threshold), l0, l1);
-    cur.base += 32;
+// Level groups of the staged scatter: consecutive levels whose fp32 gradient
+// slices add up to at most the tuning's scatter_group_bytes (48 MiB by default).
+struct LevelGroups {
+  int n;
+  int start[NECTB_MAX_LEVELS + 1];
+};
+
+// One lane's march over samples [i, end) of a ray at level l.
+template <int D, int F, bool kHashed>
+__device__ __forceinline__ void scatter_segment(const GridDev& grid, int l, const RayRec& rec, float t,
+                                                const float* __restrict__ src, int i, int end,
+                                                float* __restrict__ table_grad) {
+  CellMarch<D, F, kHashed> march(grid, l, table_grad, t);
+  float cur[4 * F];   // four samples' features; sample by sample they move down
+  float4 next[F];
+#pragma unroll
+  for (int v = 0; v < F; ++v) next[v] = __ldcs(reinterpret_cast<const float4*>(src) + v);
+  while (i < end) {
+#pragma unroll
+    for (int v = 0; v < F; ++v) {
+      cur[4 * v] = next[v].x;
+      cur[4 * v + 1] = next[v].y;
+      cur[4 * v + 2] = next[v].z;
+      cur[4 * v + 3] = next[v].w;
+    }
+    src += 4 * F;
+    if (i + 4 < end) {
+#pragma unroll
+      for (int v = 0; v < F; ++v) next[v] = __ldcs(reinterpret_cast<const float4*>(src) + v);
+    }
+#pragma unroll 2   // all four do not fit the instruction cache: 43.5 against 41.4 ms a step
+    for (int q = 0; q < 4; ++q, ++i) {
+      float p[4], d[F];
+#pragma unroll
+      for (int f = 0; f < F; ++f) d[f] = cur[f];
+#pragma unroll
+      for (int j = 0; j < 3 * F; ++j) cur[j] = cur[j + F];
+      if (i < end && sample_point(rec, i, p)) march.add(p, d);
+    }
   }
+  march.finish();
+}
+
+// Applies the staged encoding gradients of the rays ranked [lo, hi) to the fp32
+// gradient table.  A warp takes 32 consecutive ranks (vertical neighbours of the
+// detector, strip_slot), one segment of samples and one level; each lane marches
+// over its ray's samples with the cell's vertex sums in registers (CellMarch).
+// The blocks run through the level groups in order, so the gradient slice in use
+// stays small enough for the L2, in one launch.
+// Bound by instruction issue on the coarse levels and by the L2's reduction
+// requests on the fine ones (issue slots 59 %, L2 tag requests 56 % over all
+// levels).  512 x 512 rays x 512 samples, 16 x 2 levels: 29.7 -> 17.2 ms a step
+// against one warp per 32 consecutive samples with runs of equal cells merged by
+// shuffles; 24,999 rays x 100 samples 1.23 -> 0.58 ms.  Five blocks of 96
+// registers an SM; six (80, spilled) cost 1.0 ms a step.
+template <int D, int F>
+__global__ void __launch_bounds__(kScatterThreads, F == 2 ? 5 : 4)
+scatter_stage_kernel(GridDev grid, LevelGroups groups, TrainArgs a, const RayRec* __restrict__ recs,
+                     const unsigned int* __restrict__ ctrl, const float* __restrict__ stage, int64_t slots,
+                     int ray_slots, int lo, int hi, int segs, float* __restrict__ table_grad,
+                     const int32_t* __restrict__ order) {
+  const unsigned int parts = (unsigned)((hi - lo + 31) >> 5) * (unsigned)segs;   // (32 rays, segment) pairs
+  unsigned int item = blockIdx.x * (kScatterThreads / 32) + (threadIdx.x >> 5);
+  int gi = 0, nl = groups.start[1] - groups.start[0];
+  while (item >= parts * (unsigned)nl) {
+    item -= parts * (unsigned)nl;
+    if (++gi >= groups.n) return;
+    nl = groups.start[gi + 1] - groups.start[gi];
+  }
+  const int lane = threadIdx.x & 31;
+  const int l = groups.start[gi] + (int)(item % (unsigned)nl);
+  const unsigned int part = item / (unsigned)nl;
+  const unsigned int rank = (unsigned)lo + part / (unsigned)segs * 32u + lane;
+  if (rank >= min((unsigned)hi, ctrl[6])) return;
+  const RayRec rec = load_ray(recs, order[rank]);
+  const int i = (int)(part % (unsigned)segs) * kScatterSegment;
+  const int end = min(i + kScatterSegment, rec.count);
+  if (i >= end) return;
+  const float* src = stage + (l * slots + (int64_t)(rank - lo) * ray_slots + i) * F;
+  if ((grid.hashed_bits >> l) & 1u)
+    scatter_segment<D, F, true>(grid, l, rec, a.t, src, i, end, table_grad);
+  else
+    scatter_segment<D, F, false>(grid, l, rec, a.t, src, i, end, table_grad);
 }
 
 // Builds the fp16 time slice of every level (grid y = level): slice entry k
@@ -957,9 +1023,6 @@ __global__ void time_spread_kernel(TimeSlice s, const float* __restrict__ g3, fl
   }
 }
 
-
-// Level groups of the staged scatter: consecutive levels whose fp32 gradient
-// slices add up to at most the tuning's scatter_group_bytes (48 MiB by default).
 template <int D, int F, int L, int H, int ACT>
 int run_mixed(const NectbGeometry& geo, const GridDev& grid, const __half* table, const float* W,
               const TrainArgs& args, Workspace ws, int out_act, float* table_grad, float* W_grad, float* y_pred,
@@ -1053,15 +1116,15 @@ int run_mixed(const NectbGeometry& geo, const GridDev& grid, const __half* table
   // input rows with their zero padding), then dL/d(encoding) of one round of
   // per_round rays
   const StageLayout SL = stage_layout(ws, R, a.n_pixels, a.S, Shape::INP * sizeof(__nv_bfloat16),
-                                      (size_t)a.S * IN * sizeof(float), tune.staged_rounds,
+                                      (size_t)ray_slots(a.S) * IN * sizeof(float), tune.staged_rounds,
                                       tune.encoding_store != 0 && !shares_sms);
   auto run_order = [&]() -> int {
     ProfScope ps(kProfOrder, s);
     const int n_blocks = order_blocks(R, a.n_pixels);
-    order_count_kernel<<<n_blocks, kOrderBlock, 0, s>>>(ws.slot, ws.rays, ws.counters, R, a.n_pixels, SL.block_sums,
+    order_count_kernel<<<n_blocks, kOrderBlock, 0, s>>>(ws.slot, ws.rays, ws.counters, R, a.n_pixels, a.n_cols, a.sub, SL.block_sums,
                                                         SL.block_samples);
     order_scan_kernel<<<1, kOrderBlock, 0, s>>>(SL.block_sums, SL.block_samples, n_blocks, ws.counters);
-    order_compact_kernel<<<n_blocks, kOrderBlock, 0, s>>>(ws.slot, ws.rays, ws.counters, R, a.n_pixels, SL.block_sums,
+    order_compact_kernel<<<n_blocks, kOrderBlock, 0, s>>>(ws.slot, ws.rays, ws.counters, R, a.n_pixels, a.n_cols, a.sub, SL.block_sums,
                                                           SL.block_samples, SL.order, SL.offs);
     return launch_status("order kernels");
   };
@@ -1100,21 +1163,22 @@ int run_mixed(const NectbGeometry& geo, const GridDev& grid, const __half* table
   const int64_t per_round = SL.per_round;
   float* stage = SL.stage;
   const int32_t* order = SL.order;
-  // two passes per round of Q ordered rays: the tensor-core backward stages
-  // dL/d(encoding), then one scatter pass per level group
-  int group_start[NECTB_MAX_LEVELS + 1], n_groups = 0;
+  // two passes per round of ordered rays: the tensor-core backward stages
+  // dL/d(encoding), then the scatter applies it level group by level group
+  LevelGroups groups;
+  groups.n = 0;
   {
     size_t acc = 0;
     for (int l = 0; l < grid.n_levels; ++l) {
       const int64_t next = l + 1 < grid.n_levels ? grid.offset[l + 1] : grid.total_entries;
       const size_t bytes = (size_t)(next - grid.offset[l]) * F * sizeof(float);
       if (l == 0 || acc + bytes > group_bytes) {
-        group_start[n_groups++] = l;
+        groups.start[groups.n++] = l;
         acc = 0;
       }
       acc += bytes;
     }
-    group_start[n_groups] = grid.n_levels;
+    groups.start[groups.n] = grid.n_levels;
   }
   // tensor-core pass of a round: the lean kernel for two hidden layers over at
   // most 64 inputs (up to three blocks per SM), else the general one (two)
@@ -1127,37 +1191,42 @@ int run_mixed(const NectbGeometry& geo, const GridDev& grid, const __half* table
     cudaFuncSetAttribute(bwd_mixed_kernel<D, F, L, H, true, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)bsmem);
   auto ks = scatter_stage_kernel<D, F>;
-  int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ks, kScatterThreads, 0);
-  if (tune.scatter_blocks_per_sm > 0) per_sm = std::min(per_sm, tune.scatter_blocks_per_sm);
-  const int sblocks = sms * std::max(per_sm, 1);
-  const int64_t slots = per_round * a.S;
+  const int segs = (int)ceil_div(a.S, kScatterSegment);
+  const int64_t slots = per_round * ray_slots(a.S);
+  // a round stages in launches of at most R / staged_rounds rays: the weight
+  // gradients gather in the tensor cores' accumulators for the length of a
+  // launch and in fp32 memory between launches, and the accumulators lose about
+  // 2e-8 of the sum per product (three times the launch length: 3e-5)
+  const int64_t chunk = (R + tune.staged_rounds - 1) / tune.staged_rounds;
   for (int64_t lo = 0; lo < R; lo += per_round) {
     const int hi = (int)std::min<int64_t>(R, lo + per_round);
-    if (int rc = cuda_status(cudaMemsetAsync(ws.counters + 1, 0, sizeof(unsigned int), s), "memset cursor")) return rc;
-    {
-      ProfScope ps(kProfBackward, s);
-      if constexpr (kLean)
-        bwd_lean_kernel<D, F, ACT><<<lblocks, kMixThreads, lsmem, s>>>(gt, table, W, a, ws.rays, ws.slot,
-                                                                       ws.counters, out_act, W_grad, (int)lo, hi,
-                                                                       stage, slots, order, SL.offs, SL.xstore,
-                                                                       SL.xcap);
-      else
-        bwd_mixed_kernel<D, F, L, H, true, ACT><<<blocks, kMixThreads, bsmem, s>>>(
-            gt, table, W, a, ws.rays, ws.slot, ws.counters, out_act, table_grad, W_grad, (int)lo, hi, stage, slots,
-            order, SL.offs, SL.xstore, SL.xcap);
-    }
-    if (int rc = launch_status("bwd_mixed_kernel")) return rc;
-    for (int gi = 0; gi < n_groups; ++gi) {
-      if (int rc = cuda_status(cudaMemsetAsync(ws.counters + 5, 0, sizeof(unsigned int), s), "memset cursor"))
+    for (int64_t c0 = lo; c0 < hi; c0 += chunk) {
+      const int c1 = (int)std::min<int64_t>(hi, c0 + chunk);
+      if (int rc = cuda_status(cudaMemsetAsync(ws.counters + 1, 0, sizeof(unsigned int), s), "memset cursor"))
         return rc;
       {
-        ProfScope ps(kProfScatter, s);
-        ks<<<sblocks, kScatterThreads, 0, s>>>(grid, a, ws.rays, ws.slot, ws.counters, stage, slots, (int)lo, hi,
-                                               group_start[gi], group_start[gi + 1], table_grad, order);
+        ProfScope ps(kProfBackward, s);
+        float* at = stage + (c0 - lo) * ray_slots(a.S) * F;
+        if constexpr (kLean)
+          bwd_lean_kernel<D, F, ACT><<<lblocks, kMixThreads, lsmem, s>>>(gt, table, W, a, ws.rays, ws.slot,
+                                                                         ws.counters, out_act, W_grad, (int)c0, c1,
+                                                                         at, slots, order, SL.offs, SL.xstore,
+                                                                         SL.xcap);
+        else
+          bwd_mixed_kernel<D, F, L, H, true, ACT><<<blocks, kMixThreads, bsmem, s>>>(
+              gt, table, W, a, ws.rays, ws.slot, ws.counters, out_act, table_grad, W_grad, (int)c0, c1, at, slots,
+              order, SL.offs, SL.xstore, SL.xcap);
       }
-      if (int rc = launch_status("scatter_stage_kernel")) return rc;
+      if (int rc = launch_status("bwd_mixed_kernel")) return rc;
     }
+    {
+      ProfScope ps(kProfScatter, s);
+      const int64_t warps = ceil_div(hi - lo, 32) * segs * grid.n_levels;
+      ks<<<(unsigned)ceil_div(warps, kScatterThreads / 32), kScatterThreads, 0, s>>>(
+          grid, groups, a, ws.rays, ws.counters, stage, slots, ray_slots(a.S), (int)lo, hi, segs, table_grad,
+          order);
+    }
+    if (int rc = launch_status("scatter_stage_kernel")) return rc;
   }
   return NECTB_OK;
 }

@@ -79,10 +79,21 @@ __global__ void ray_prep_kernel(NectbGeometry g, TrainArgs a, RayRec* __restrict
   }
 }
 
+// Slot of scheduling index idx: the detector in strips of 32 rows, a strip
+// column by column, so that 32 consecutive rays are vertical neighbours.
+// Their paths differ along axis 0 only (the rotation axis), whose vertices
+// share sectors of the tables.
+__device__ __forceinline__ int strip_slot(int idx, int P, int cols, int sub) {
+  const int rows = P / (cols * sub), strip = idx / (32 * cols * sub);
+  const int h = min(32, rows - 32 * strip), rem = idx - strip * 32 * cols * sub;
+  const int cj = rem / h, row = 32 * strip + rem - cj * h;   // cj = column * sub + sub-angle
+  return row * cols * sub + cj;
+}
+
 __device__ __forceinline__ bool ordered_valid(const int32_t* __restrict__ slot, const RayRec* __restrict__ recs,
-                                              bool by_pixel, int idx, int n, int* ray) {
+                                              bool by_pixel, int idx, int n, int cols, int sub, int* ray) {
   if (idx >= n) return false;
-  const int r = by_pixel ? slot[idx] : idx;
+  const int r = by_pixel ? slot[strip_slot(idx, n, cols, sub)] : idx;
   *ray = r;
   return r >= 0 && recs[r].count > 0;
 }
@@ -119,13 +130,15 @@ __device__ __forceinline__ T block_scan(T v, T* warp_sums, T* total) {
 
 __global__ void __launch_bounds__(kOrderBlock)
 order_count_kernel(const int32_t* __restrict__ slot, const RayRec* __restrict__ recs,
-                   const unsigned int* __restrict__ ctrl, int R, int P, unsigned int* __restrict__ block_sums,
+                   const unsigned int* __restrict__ ctrl, int R, int P, int cols, int sub,
+                   unsigned int* __restrict__ block_sums,
                    unsigned long long* __restrict__ block_samples) {
   __shared__ unsigned int ws[33];
   __shared__ unsigned long long ws64[33];
   const bool by_pixel = !(ctrl[3] & kFlagDuplicatePixels);
   int ray = -1;
-  const bool v = ordered_valid(slot, recs, by_pixel, blockIdx.x * kOrderBlock + threadIdx.x, by_pixel ? P : R, &ray);
+  const bool v = ordered_valid(slot, recs, by_pixel, blockIdx.x * kOrderBlock + threadIdx.x, by_pixel ? P : R, cols, sub,
+                               &ray);
   unsigned int total;
   unsigned long long samples;
   block_scan<unsigned int>(v ? 1u : 0u, ws, &total);
@@ -163,14 +176,16 @@ order_scan_kernel(unsigned int* __restrict__ block_sums, unsigned long long* __r
 
 __global__ void __launch_bounds__(kOrderBlock)
 order_compact_kernel(const int32_t* __restrict__ slot, const RayRec* __restrict__ recs,
-                     const unsigned int* __restrict__ ctrl, int R, int P, const unsigned int* __restrict__ block_sums,
+                     const unsigned int* __restrict__ ctrl, int R, int P, int cols, int sub,
+                     const unsigned int* __restrict__ block_sums,
                      const unsigned long long* __restrict__ block_samples, int32_t* __restrict__ order,
                      uint64_t* __restrict__ offs) {
   __shared__ unsigned int ws[33];
   __shared__ unsigned long long ws64[33];
   const bool by_pixel = !(ctrl[3] & kFlagDuplicatePixels);
   int ray = -1;
-  const bool v = ordered_valid(slot, recs, by_pixel, blockIdx.x * kOrderBlock + threadIdx.x, by_pixel ? P : R, &ray);
+  const bool v = ordered_valid(slot, recs, by_pixel, blockIdx.x * kOrderBlock + threadIdx.x, by_pixel ? P : R, cols, sub,
+                               &ray);
   unsigned int total;
   unsigned long long samples;
   const unsigned int rank = block_scan<unsigned int>(v ? 1u : 0u, ws, &total);
