@@ -4,7 +4,7 @@
 
 #include "common.cuh"
 #include "hashgrid.cuh"
-#include "mlp_simt.cuh"
+#include "mlp_tile.cuh"
 
 namespace nectb {
 
@@ -65,42 +65,35 @@ __global__ void encode_kernel(GridDev g, const T* __restrict__ table, const floa
   encode_point<D, F, T>(g, table, p, out + i * (int64_t)g.n_levels * F);
 }
 
-// One thread per point: encode into a shared-memory column, then the SIMT MLP.
-constexpr int kModelThreads = 128;
+// Tiles of 128 points: encode, then the fp32 MLP (mlp_tile.cuh).
+constexpr int kModelSamples = 128;
 
-template <int D, int F, typename T, int IN, int H>
-__global__ void __launch_bounds__(kModelThreads) model_forward_kernel(GridDev g, const T* __restrict__ table,
-                                                                      const float* __restrict__ W,
-                                                                      const float* __restrict__ x, int64_t n,
-                                                                      float t, const float* __restrict__ t_dev,
-                                                                      int act, int out_act,
-                                                                      float* __restrict__ sigma) {
-  constexpr int LD = kModelThreads + 4;
+template <int D, int F, typename T, int L, int H>
+__global__ void __launch_bounds__(kTileThreads)
+model_forward_kernel(GridDev g, const T* __restrict__ table, const float* __restrict__ W, const float* __restrict__ x,
+                     int64_t n, float t, const float* __restrict__ t_dev, int act, int out_act,
+                     float* __restrict__ sigma) {
+  constexpr int IN = L * F, NT = kModelSamples, LD = NT + 4;
   extern __shared__ float4 smem4[];
   float* smem = reinterpret_cast<float*>(smem4);
   const SimtWeights sw = stage_weights<IN, H, false>(W, smem);
-  float* xe = smem + simt_weight_floats<IN, H, false>() + threadIdx.x;
-  float* hid = xe + IN * LD;  // two [64][LD] buffers, alternating between layers
+  TilePoints<NT>* pts = reinterpret_cast<TilePoints<NT>*>(smem + simt_weight_floats<IN, H, false>());
+  float* buf = reinterpret_cast<float*>(pts + 1);
   if (D == 4 && t_dev) t = *t_dev;   // the broadcast timestep, read on the device
-  __syncthreads();
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    float p[4];
+  const int s = threadIdx.x;
+  for (int64_t c0 = (int64_t)blockIdx.x * NT; c0 < n; c0 += (int64_t)gridDim.x * NT) {  // block-uniform
+    const bool valid = s < NT && c0 + s < n;
+    if (s < NT) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) p[k] = x[i * 3 + k];
-    if (D == 4) p[3] = t;
-    encode_point<D, F, T>(g, table, p, xe, LD);
-    float z;
-    if (H == 1) {
-      z = gemv_dot<IN, LD>(sw.WT[0], xe, sw.wout, act);
-    } else {
-      gemv_cols<IN, kWidth, LD>(sw.WT[0], xe, hid, act);
-#pragma unroll
-      for (int k = 1; k < H - 1; ++k)
-        gemv_cols<kWidth, kWidth, LD>(sw.WT[k], hid + ((k - 1) & 1) * kWidth * LD, hid + (k & 1) * kWidth * LD,
-                                      act);
-      z = gemv_dot<kWidth, LD>(sw.WT[H - 1], hid + ((H - 2) & 1) * kWidth * LD, sw.wout, act);
+      for (int k = 0; k < 3; ++k) pts->p[k * NT + s] = valid ? x[(c0 + s) * 3 + k] : 0.f;
+      pts->valid[s] = valid ? 1 : 0;
     }
-    sigma[i] = act_fwd(z, out_act);
+    __syncthreads();
+    encode_tile<D, F, L, NT, kTileThreads, T>(g, table, pts->p, pts->valid, t, buf);
+    __syncthreads();
+    tile_hidden<IN, H, NT, kTileThreads>(sw, buf, buf, act);
+    __syncthreads();
+    if (valid) sigma[c0 + s] = act_fwd(dot_col<kWidth, LD>(sw.wout, buf + s), out_act);
   }
 }
 
@@ -132,17 +125,16 @@ template <int D, int F, typename T, int L, int H>
 int launch_model(const GridDev& g, const void* params, const float* W, const float* x, int64_t n, float t,
                  const float* t_dev, int act, int out_act, float* sigma, cudaStream_t s) {
   constexpr int IN = L * F;
-  auto k = model_forward_kernel<D, F, T, IN, H>;
-  const size_t smem = (size_t)(simt_weight_floats<IN, H, false>() +
-                               (IN + simt_hidden_buffers<H>() * kWidth) * (kModelThreads + 4)) * sizeof(float);
+  auto k = model_forward_kernel<D, F, T, L, H>;
+  const size_t smem = tile_forward_smem<IN, H, kModelSamples>();
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int dev = 0, sms = 148, per_sm = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kModelThreads, smem);
-  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, kModelThreads), (int64_t)sms * std::max(per_sm, 1)));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kTileThreads, smem);
+  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, kModelSamples), (int64_t)sms * std::max(per_sm, 1)));
   ProfScope ps(kProfModel, s);
-  k<<<blocks, kModelThreads, smem, s>>>(g, (const T*)params, W, x, n, t, t_dev, act, out_act, sigma);
+  k<<<blocks, kTileThreads, smem, s>>>(g, (const T*)params, W, x, n, t, t_dev, act, out_act, sigma);
   return launch_status("model_forward_kernel");
 }
 

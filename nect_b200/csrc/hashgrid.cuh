@@ -148,54 +148,34 @@ struct Feat<4, __half> {
   }
 };
 
-// Encodes one point: out[(l*F + f) * stride] for all levels.  x has D
-// coordinates in [0,1].
+// Encodes one point at level l: acc[f] (fused multiply-adds over the corners in
+// order).  x has D coordinates in [0,1].
+template <int D, int F, typename T>
+__device__ __forceinline__ void encode_level(const GridDev& g, const T* __restrict__ table, int l, const float* x,
+                                             float* acc) {
+  LevelCorners<D> lc;
+  level_corners<D>(g, l, x, lc);
+  float vals[1 << D][F];
+#pragma unroll
+  for (int c = 0; c < (1 << D); ++c) Feat<F, T>::load(table, g.offset[l] + lc.idx[c], vals[c]);
+#pragma unroll
+  for (int f = 0; f < F; ++f) acc[f] = 0.f;
+#pragma unroll
+  for (int c = 0; c < (1 << D); ++c)
+#pragma unroll
+    for (int f = 0; f < F; ++f) acc[f] = fmaf(lc.w[c], vals[c][f], acc[f]);
+}
+
+// Encodes one point: out[(l*F + f) * stride] for all levels.
 template <int D, int F, typename T>
 __device__ __forceinline__ void encode_point(const GridDev& g, const T* __restrict__ table, const float* x,
                                              float* out, int stride = 1) {
 #pragma unroll 1
   for (int l = 0; l < g.n_levels; ++l) {
-    LevelCorners<D> lc;
-    level_corners<D>(g, l, x, lc);
-    float vals[1 << D][F];
-#pragma unroll
-    for (int c = 0; c < (1 << D); ++c) Feat<F, T>::load(table, g.offset[l] + lc.idx[c], vals[c]);
     float acc[F];
-#pragma unroll
-    for (int f = 0; f < F; ++f) acc[f] = 0.f;
-#pragma unroll
-    for (int c = 0; c < (1 << D); ++c)
-#pragma unroll
-      for (int f = 0; f < F; ++f) acc[f] = fmaf(lc.w[c], vals[c][f], acc[f]);
+    encode_level<D, F, T>(g, table, l, x, acc);
 #pragma unroll
     for (int f = 0; f < F; ++f) out[(l * F + f) * stride] = acc[f];
-  }
-}
-
-// Gradient scatter of one point: grad[offset + idx][f] += w * dout[(l*F + f) * stride].
-template <int D, int F>
-__device__ __forceinline__ void scatter_point(const GridDev& g, float* __restrict__ grad, const float* x,
-                                              const float* dsrc, int stride = 1) {
-#pragma unroll 1
-  for (int l = 0; l < g.n_levels; ++l) {
-    LevelCorners<D> lc;
-    level_corners<D>(g, l, x, lc);
-    float d[F];
-#pragma unroll
-    for (int f = 0; f < F; ++f) d[f] = dsrc[(l * F + f) * stride];
-#pragma unroll
-    for (int c = 0; c < (1 << D); ++c) {
-      float* dst = grad + (g.offset[l] + lc.idx[c]) * F;
-      if constexpr (F == 2) {
-        atomicAdd(reinterpret_cast<float2*>(dst), make_float2(lc.w[c] * d[0], lc.w[c] * d[1]));
-      } else if constexpr (F == 4) {
-        atomicAdd(reinterpret_cast<float4*>(dst),
-                  make_float4(lc.w[c] * d[0], lc.w[c] * d[1], lc.w[c] * d[2], lc.w[c] * d[3]));
-      } else {
-#pragma unroll
-        for (int f = 0; f < F; ++f) atomicAdd(dst + f, lc.w[c] * d[f]);
-      }
-    }
   }
 }
 
@@ -240,6 +220,31 @@ __device__ __forceinline__ void red_entry(float* dst, const float* v) {
   else
 #pragma unroll
     for (int f = 0; f < F; ++f) atomicAdd(dst + f, v[f]);
+}
+
+// Adds one point's gradient d of level l to its corners' entries.
+template <int D, int F>
+__device__ __forceinline__ void scatter_level(const GridDev& g, float* __restrict__ grad, int l, const float* x,
+                                              const float* d) {
+  LevelCorners<D> lc;
+  level_corners<D>(g, l, x, lc);
+  float* base = grad + g.offset[l] * F;
+#pragma unroll
+  for (int c = 0; c < (1 << D); c += 2) {
+    if constexpr (F == 2) {
+      red_pair_f2(base, lc.idx[c], lc.idx[c + 1], lc.w[c] * d[0], lc.w[c] * d[1], lc.w[c + 1] * d[0],
+                  lc.w[c + 1] * d[1]);
+    } else {
+      float v0[F], v1[F];
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        v0[f] = lc.w[c] * d[f];
+        v1[f] = lc.w[c + 1] * d[f];
+      }
+      red_entry<F>(base + (int64_t)lc.idx[c] * F, v0);
+      red_entry<F>(base + (int64_t)lc.idx[c + 1] * F, v1);
+    }
+  }
 }
 
 // fp32 value of a gradient element held as fp32 or bf16.

@@ -1,12 +1,8 @@
 // fp32 SIMT pieces of the bias-free MLP (tiny-cuda-nn FullyFusedMLP
 // semantics, as configured by MLPNetConfig in nect/config.py:115-135).
 //
-// Each thread owns one sample.  Its activation vectors live in shared memory
-// as column t of [features][NT] arrays (thread t touches only its column, so
-// per-sample work needs no barriers and accesses are bank-conflict free).
-// Layer products run over 32-output groups: 32 accumulators in registers, the
-// input element from the thread's column, the weight row as broadcast float4
-// loads.  Loops over groups are not unrolled, which keeps the code small.
+// A sample's vectors are columns of [features][LD] arrays in shared memory; the
+// layer products over a tile of samples are in mlp_tile.cuh.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -60,70 +56,6 @@ __device__ __forceinline__ float act_grad_a(float a, int kind) {
     default:
       return 1.f;
   }
-}
-
-// out[o*LD] = act(sum_k M[k][o] * in[k*LD]) for o < N.  M is [K][N] row-major
-// (shared or global memory, rows 16-byte aligned); in/out point at this
-// thread's column of [.][LD] arrays.  When N is not a multiple of 32 the last
-// group of 32 outputs reads past the end of each row of M into the next row
-// (or the next array: M must be followed by at least 32 - N % 32 floats) and
-// stores only the outputs below N.
-template <int K, int N, int LD>
-__device__ __forceinline__ void gemv_cols(const float* __restrict__ M, const float* __restrict__ in,
-                                          float* __restrict__ out, int act) {
-  static_assert(N % 4 == 0, "rows of M must be 16-byte aligned");
-  const int t = 0;
-#pragma unroll 1
-  for (int og = 0; og < N; og += 32) {
-    float acc[32];
-#pragma unroll
-    for (int o = 0; o < 32; ++o) acc[o] = 0.f;
-#pragma unroll 2
-    for (int k = 0; k < K; ++k) {
-      const float xk = in[k * LD + t];
-      const float4* w = reinterpret_cast<const float4*>(M + k * N + og);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float4 v = w[q];
-        acc[4 * q + 0] = fmaf(v.x, xk, acc[4 * q + 0]);
-        acc[4 * q + 1] = fmaf(v.y, xk, acc[4 * q + 1]);
-        acc[4 * q + 2] = fmaf(v.z, xk, acc[4 * q + 2]);
-        acc[4 * q + 3] = fmaf(v.w, xk, acc[4 * q + 3]);
-      }
-    }
-#pragma unroll
-    for (int o = 0; o < 32; ++o)
-      if (N % 32 == 0 || og + o < N) out[(og + o) * LD + t] = act_fwd(acc[o], act);
-  }
-}
-
-// Last layer fused with the output product: returns sum_o w[o] * act(sum_k M[k][o] * in[k]).
-template <int K, int LD>
-__device__ __forceinline__ float gemv_dot(const float* __restrict__ M, const float* __restrict__ in,
-                                          const float* __restrict__ w, int act) {
-  float z = 0.f;
-#pragma unroll 1
-  for (int og = 0; og < kWidth; og += 32) {
-    float acc[32];
-#pragma unroll
-    for (int o = 0; o < 32; ++o) acc[o] = 0.f;
-#pragma unroll 2
-    for (int k = 0; k < K; ++k) {
-      const float xk = in[k * LD];
-      const float4* m = reinterpret_cast<const float4*>(M + k * kWidth + og);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float4 v = m[q];
-        acc[4 * q + 0] = fmaf(v.x, xk, acc[4 * q + 0]);
-        acc[4 * q + 1] = fmaf(v.y, xk, acc[4 * q + 1]);
-        acc[4 * q + 2] = fmaf(v.z, xk, acc[4 * q + 2]);
-        acc[4 * q + 3] = fmaf(v.w, xk, acc[4 * q + 3]);
-      }
-    }
-#pragma unroll
-    for (int o = 0; o < 32; ++o) z = fmaf(w[og + o], act_fwd(acc[o], act), z);
-  }
-  return z;
 }
 
 // sum_k w[k] * in[k * LD]
@@ -213,13 +145,6 @@ __device__ __forceinline__ SimtWeights stage_weights(const float* __restrict__ W
   sw.wout = wo;
   for (int k = H; k < kMaxHidden; ++k) sw.WT[k] = sw.W[k] = nullptr;
   return sw;
-}
-
-// Hidden activations of the SIMT forward kernels: two [64][LD] buffers that
-// consecutive layers alternate between.
-template <int H>
-__host__ __device__ constexpr int simt_hidden_buffers() {
-  return H - 1 < 2 ? H - 1 : 2;
 }
 
 }  // namespace nectb

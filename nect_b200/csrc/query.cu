@@ -13,6 +13,7 @@
 #include <algorithm>
 
 #include "mixed_common.cuh"
+#include "mlp_tile.cuh"
 #include "train_common.cuh"
 
 namespace nectb {
@@ -182,22 +183,21 @@ query_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* 
   }
 }
 
+// fp32: a chunk is a tile of 128 points (mlp_tile.cuh).
 template <int D, int F, typename T, int L, int H>
-__global__ void __launch_bounds__(kQThreads)
+__global__ void __launch_bounds__(kTileThreads)
 query_plain_kernel(GridDev grid, const T* __restrict__ table, const float* __restrict__ W,
                    const NectbQueryItem* __restrict__ items, int n_items, int64_t total_chunks,
                    unsigned int* __restrict__ counter, int act, int out_act) {
-  constexpr int IN = L * F;
-  constexpr int LD = kQThreads + 4;
+  constexpr int IN = L * F, NT = 128, LD = NT + 4;
   extern __shared__ float4 smem4[];
   float* smem = reinterpret_cast<float*>(smem4);
   const SimtWeights sw = stage_weights<IN, H, false>(W, smem);
-  float* xe = smem + simt_weight_floats<IN, H, false>() + threadIdx.x;
-  float* hid = xe + IN * LD;  // two [64][LD] buffers, alternating between layers
+  TilePoints<NT>* pts = reinterpret_cast<TilePoints<NT>*>(smem + simt_weight_floats<IN, H, false>());
+  float* buf = reinterpret_cast<float*>(pts + 1);
   __shared__ long long s_chunk;
   __shared__ int s_item;
   const int t = threadIdx.x;
-  __syncthreads();
   while (true) {
     if (t == 0) {
       const long long c = (long long)atomicAdd(counter, 1u);
@@ -207,23 +207,22 @@ query_plain_kernel(GridDev grid, const T* __restrict__ table, const float* __res
     __syncthreads();
     const long long chunk = s_chunk;
     if (chunk >= total_chunks) break;
-    const QPoint q = query_point(items[s_item], chunk, t);
-    if (q.valid) {
-      encode_point<D, F, T>(grid, table, q.p, xe, LD);
-      float z;
-      if (H == 1) {
-        z = gemv_dot<IN, LD>(sw.WT[0], xe, sw.wout, act);
-      } else {
-        gemv_cols<IN, kWidth, LD>(sw.WT[0], xe, hid, act);
+    const NectbQueryItem& it = items[s_item];
+    QPoint q;
+    q.valid = false;
+    if (t < NT) {
+      q = query_point(it, chunk, t);
 #pragma unroll
-        for (int k = 1; k < H - 1; ++k)
-          gemv_cols<kWidth, kWidth, LD>(sw.WT[k], hid + ((k - 1) & 1) * kWidth * LD, hid + (k & 1) * kWidth * LD,
-                                        act);
-        z = gemv_dot<kWidth, LD>(sw.WT[H - 1], hid + ((H - 2) & 1) * kWidth * LD, sw.wout, act);
-      }
-      *q.dst = fmaf(act_fwd(z, out_act), q.scale, q.offset);
+      for (int k = 0; k < 3; ++k) pts->p[k * NT + t] = q.p[k];
+      pts->valid[t] = q.valid ? 1 : 0;
     }
+    const float tval = it.t;
     __syncthreads();
+    encode_tile<D, F, L, NT, kTileThreads, T>(grid, table, pts->p, pts->valid, tval, buf);
+    __syncthreads();
+    tile_hidden<IN, H, NT, kTileThreads>(sw, buf, buf, act);
+    __syncthreads();
+    if (q.valid) *q.dst = fmaf(act_fwd(dot_col<kWidth, LD>(sw.wout, buf + t), out_act), q.scale, q.offset);
   }
 }
 
@@ -255,15 +254,14 @@ int launch_query_plain(const GridDev& g, const void* table, const float* W, cons
                        int64_t chunks, unsigned int* counter, int act, int oact, int max_blocks, cudaStream_t s) {
   constexpr int IN = L * F;
   auto k = query_plain_kernel<D, F, T, L, H>;
-  const size_t smem =
-      (size_t)(simt_weight_floats<IN, H, false>() + (IN + simt_hidden_buffers<H>() * kWidth) * (kQThreads + 4)) * 4;
+  const size_t smem = tile_forward_smem<IN, H, 128>();
   set_smem(k, smem, true);
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kQThreads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kTileThreads, smem);
   int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(chunks, (int64_t)sm_count() * std::max(per_sm, 1)));
   if (max_blocks > 0) blocks = std::min(blocks, max_blocks);
   ProfScope ps(kProfModel, s);
-  k<<<blocks, kQThreads, smem, s>>>(g, (const T*)table, W, items, n, chunks, counter, act, oact);
+  k<<<blocks, kTileThreads, smem, s>>>(g, (const T*)table, W, items, n, chunks, counter, act, oact);
   return launch_status("query_plain_kernel");
 }
 

@@ -3,18 +3,18 @@
 //
 // Three launches per batch:
 //   1. ray_prep_kernel   warp per ray: entry/exit, count, measured value.
-//   2. fwd_plain_kernel  warp per ray: regenerate each sample, encode, MLP,
-//                        warp-shuffle sum along the ray -> y_pred, loss,
+//   2. fwd_plain_kernel  blocks step through tiles of 128 samples (32
+//                        consecutive samples of each of four rays): encode,
+//                        MLP, warp-shuffle sum along the ray -> y_pred, loss,
 //                        dL/dsigma for the ray.
-//   3. bwd_plain_kernel  blocks of NT threads step through tiles of NT
-//                        samples: re-encode, forward, backward through the
-//                        MLP, fp32 weight-gradient tile products accumulated
-//                        in registers, table gradients by float2/float4
+//   3. bwd_plain_kernel  the same tiles: re-encode, forward, backward through
+//                        the MLP, fp32 weight-gradient tile products
+//                        accumulated in registers, table gradients by vector
 //                        atomics.
 // Sample positions and encodings live only in registers and shared memory.
 #include <algorithm>
 
-#include "mlp_simt.cuh"
+#include "mlp_tile.cuh"
 #include "train_common.cuh"
 
 namespace nectb {
@@ -199,63 +199,72 @@ order_compact_kernel(const int32_t* __restrict__ slot, const RayRec* __restrict_
 
 namespace {
 
-constexpr int kPlainFwdThreads = 128;
+constexpr int kPlainFwdSamples = 128;
 
-template <int D, int F, int IN, int H>
-__global__ void __launch_bounds__(kPlainFwdThreads)
+// Bound by shared-memory wavefronts (78 % of their rate) in the products and by
+// the gathers' latency between them.  16,384 rays x 256 samples, 16 x 2 levels,
+// 2 x 64: 2.49 -> 1.45 ms against one sample a thread, 0.91 ms of it the MLP (its
+// multiply-adds take 0.49 ms).
+template <int D, int F, int L, int H>
+__global__ void __launch_bounds__(kTileThreads)
 fwd_plain_kernel(GridDev grid, const float* __restrict__ table, const float* __restrict__ W, TrainArgs a,
                  RayRec* __restrict__ recs, const int32_t* __restrict__ slot, unsigned int* __restrict__ ctrl,
                  int act, int out_act, float* __restrict__ y_pred, float* __restrict__ loss) {
-  constexpr int NT = kPlainFwdThreads;
+  constexpr int IN = L * F, NT = kPlainFwdSamples, LD = NT + 4;
   const bool by_pixel = !(ctrl[3] & kFlagDuplicatePixels);
-  constexpr int LD = NT + 4;
   extern __shared__ float4 smem4[];
   float* smem = reinterpret_cast<float*>(smem4);
   const SimtWeights sw = stage_weights<IN, H, false>(W, smem);
-  float* cols = smem + simt_weight_floats<IN, H, false>();
-  const int t = threadIdx.x;
-  float* x = cols + t;                 // [IN][LD]
-  float* hid = cols + IN * LD + t;     // two [64][LD] buffers, alternating between layers
-  __syncthreads();
-  const int lane = t & 31;
-  float loss_acc = 0.f;
+  TilePoints<NT>* pts = reinterpret_cast<TilePoints<NT>*>(smem + simt_weight_floats<IN, H, false>());
+  float* buf = reinterpret_cast<float*>(pts + 1);   // every layer's columns in turn
+  const int t = threadIdx.x, lane = t & 31;
+  const bool owner = t < NT;   // the first NT threads hold the tile's samples, a warp 32 of one ray
+  float loss_acc = 0.f, sum = 0.f;
+  int ray = -1, base = 0;
+  RayRec rec;
+  rec.count = 0;
   while (true) {
-    const int r = next_ray(ctrl, slot, recs, a.num_rays, a.n_pixels, by_pixel, lane);
-    if (r < 0) break;
-    const RayRec rec = load_ray(recs, r);
-    float sum = 0.f;
-    for (int base = 0; base < rec.count; base += 32) {
-      const int i = base + lane;
-      float p[4] = {0.f, 0.f, 0.f, 0.f};
-      bool valid = false;
-      if (i < rec.count) valid = sample_point(rec, i, p);
-      if (D == 4) p[3] = a.t;
-      if (valid) {
-        encode_point<D, F, float>(grid, table, p, x, LD);
-        const float* in = x;
-        if (H == 1) {
-          sum += act_fwd(gemv_dot<IN, LD>(sw.WT[0], in, sw.wout, act), out_act);
+    bool valid = false;
+    if (owner) {
+      if (ray < a.num_rays && (ray < 0 || base >= rec.count)) {
+        const int r = next_ray(ctrl, slot, recs, a.num_rays, a.n_pixels, by_pixel, lane);
+        if (r < 0) {
+          ray = a.num_rays;
+          rec.count = 0;
         } else {
-          gemv_cols<IN, kWidth, LD>(sw.WT[0], in, hid, act);
+          rec = load_ray(recs, r);
+          ray = r;
+          base = 0;
+          sum = 0.f;
+        }
+      }
+      float p[4] = {0.f, 0.f, 0.f, 0.f};
+      if (ray < a.num_rays && base + lane < rec.count) valid = sample_point(rec, base + lane, p);
 #pragma unroll
-          for (int k = 1; k < H - 1; ++k)
-            gemv_cols<kWidth, kWidth, LD>(sw.WT[k], hid + ((k - 1) & 1) * kWidth * LD, hid + (k & 1) * kWidth * LD,
-                                          act);
-          sum += act_fwd(gemv_dot<kWidth, LD>(sw.WT[H - 1], hid + ((H - 2) & 1) * kWidth * LD, sw.wout, act),
-                         out_act);
+      for (int k = 0; k < 3; ++k) pts->p[k * NT + t] = p[k];
+      pts->valid[t] = valid ? 1 : 0;
+    }
+    if (!__syncthreads_or(owner && ray < a.num_rays)) break;
+    encode_tile<D, F, L, NT, kTileThreads, float>(grid, table, pts->p, pts->valid, a.t, buf);
+    __syncthreads();
+    tile_hidden<IN, H, NT, kTileThreads>(sw, buf, buf, act);
+    __syncthreads();
+    if (owner && ray < a.num_rays) {
+      if (valid) sum += act_fwd(dot_col<kWidth, LD>(sw.wout, buf + t), out_act);
+      base += 32;
+      if (base >= rec.count) {
+        const float s = warp_sum(sum);
+        if (lane == 0) {
+          const float yp = s * rec.scale;
+          y_pred[ray] = yp;
+          recs[ray].gsig = loss_grad(yp, rec.y, a.loss_type, a.num_rays, rec.scale) * a.loss_scale;
+          loss_acc += loss_term(yp, rec.y, a.loss_type);
         }
       }
     }
-    sum = warp_sum(sum);
-    if (lane == 0) {
-      const float yp = sum * rec.scale;
-      y_pred[r] = yp;
-      recs[r].gsig = loss_grad(yp, rec.y, a.loss_type, a.num_rays, rec.scale) * a.loss_scale;
-      loss_acc += loss_term(yp, rec.y, a.loss_type);
-    }
   }
   __shared__ float red[NT / 32];
-  if (lane == 0) red[t >> 5] = loss_acc;
+  if (owner && lane == 0) red[t >> 5] = loss_acc;
   __syncthreads();
   if (t == 0) {
     float s = 0.f;
@@ -264,316 +273,225 @@ fwd_plain_kernel(GridDev grid, const float* __restrict__ table, const float* __r
   }
 }
 
-// acc[a][b] += sum_t G[(4*jb + a)*LD + t] * A[(ib*IB + b)*LD + t] over the
-// tile's NT samples (weight gradient dW[j][i] = sum_t G[t][j] A[t][i]).
-// Thread p owns rows 4*jb..4*jb+3 and columns ib*IB..ib*IB+IB-1.
-template <int K, int NT, int LD>
-struct WGrad {
-  static constexpr int IBLK = NT / 16;
-  static constexpr int IB = K / IBLK;
-  static_assert(16 * IBLK == NT && IB * IBLK == K, "tile shape");
-  float acc[4][IB];
-  __device__ __forceinline__ void zero() {
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < IB; ++b) acc[a][b] = 0.f;
-  }
-  __device__ __forceinline__ void add(const float* __restrict__ G, const float* __restrict__ A) {
-    const int jb = threadIdx.x / IBLK, ib = threadIdx.x % IBLK;
-#pragma unroll 1
-    for (int t = 0; t < NT; t += 4) {
-      float4 g[4], v[IB];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) g[a] = *reinterpret_cast<const float4*>(G + (4 * jb + a) * LD + t);
-#pragma unroll
-      for (int b = 0; b < IB; ++b) v[b] = *reinterpret_cast<const float4*>(A + (ib * IB + b) * LD + t);
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < IB; ++b) {
-          acc[a][b] = fmaf(g[a].x, v[b].x, acc[a][b]);
-          acc[a][b] = fmaf(g[a].y, v[b].y, acc[a][b]);
-          acc[a][b] = fmaf(g[a].z, v[b].z, acc[a][b]);
-          acc[a][b] = fmaf(g[a].w, v[b].w, acc[a][b]);
-        }
-    }
-  }
-  __device__ __forceinline__ void flush(float* __restrict__ dst) const {  // dst [64][K]
-    const int jb = threadIdx.x / IBLK, ib = threadIdx.x % IBLK;
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < IB; ++b) atomicAdd(dst + (4 * jb + a) * K + ib * IB + b, acc[a][b]);
-  }
-};
-
-// Whether the layer-0 weight-gradient tile stays in registers across the
-// sample-tile loop.  A thread carries 4 * (IN + (H - 1) * 64) / (NT / 16)
-// accumulators when every tile stays; the 3-layer MLP over 64 inputs (192 of
-// them, the kernel at the 255-register limit) measured wrong first-layer and
-// table gradients on B200 in that form, and exact ones when its layer-0 tile
-// is added to W_grad after every sample tile (4096 atomics per tile of NT
-// samples, about 64 per sample) and only the hidden-layer tiles stay.
-template <int IN, int H, int NT>
-__host__ __device__ constexpr bool carry_layer0() {
-  return 4 * (IN + (H - 1) * kWidth) / (NT / 16) <= 160;
-}
-
-// Whether the hidden layers' weight-gradient tiles stay in registers across
-// the loop (at most 160 accumulators); otherwise each is computed and added
-// to W_grad per sample tile, one layer at a time (the deep models).
-template <int H, int NT>
-__host__ __device__ constexpr bool carry_hidden() {
-  return 4 * (H - 1) * kWidth / (NT / 16) <= 160;
-}
-
-// Shared-memory plan of the SIMT backward kernels for IN inputs and H hidden
-// layers: tiles of 128, 64 or 32 samples with both weight copies in shared
-// memory, or, when even 32 do not fit (the deep models), tiles of 32 with the
-// PyTorch-layout weights read from the global buffer through L1.
+// Shared-memory plan of the fp32 backward for IN inputs and H hidden layers:
+// both weight copies and tiles of 64 samples where two such blocks share an SM
+// (one block's gathers run beside the other's products), else 128, 64 or 32
+// samples in one block, the last with the PyTorch-layout weights read from the
+// global buffer through L1 (the deep models).
 template <int IN, int H>
-struct SimtBwdPlan {
+struct PlainBwdPlan {
   static constexpr size_t kBudget = 227 * 1024;
-  static constexpr size_t cols(int nt) { return (size_t)(IN + (H + 2) * kWidth) * (nt + 4) * 4; }
-  static constexpr size_t wbytes(bool both) {
-    return (size_t)(both ? simt_weight_floats<IN, H, true>() : simt_weight_floats<IN, H, false>()) * 4;
+  static constexpr int kRows = IN > kWidth ? IN : kWidth;   // rows of a_H, then of the gradients
+  static constexpr size_t bytes(int nt, bool both) {
+    return (size_t)(both ? simt_weight_floats<IN, H, true>() : simt_weight_floats<IN, H, false>()) * 4 +
+           (size_t)nt * 20 + (size_t)(IN + (H - 1) * kWidth + kRows) * (nt + 4) * 4;
   }
-  static constexpr bool kBoth = wbytes(true) + cols(32) <= kBudget;
+  static constexpr bool kTwo = bytes(64, true) <= 113 * 1024;
+  static constexpr bool kBoth = bytes(32, true) <= kBudget;
+  // rows of 76 inputs split into groups of 4 outputs only, which 32 samples need
   static constexpr int NT =
-      wbytes(kBoth) + cols(128) <= kBudget ? 128 : (wbytes(kBoth) + cols(64) <= kBudget ? 64 : 32);
-  static constexpr size_t smem = wbytes(kBoth) + cols(NT);
-  static_assert(smem <= kBudget, "SIMT backward does not fit shared memory");
+      IN % 8 != 0 ? 32 : (kTwo ? 64 : (bytes(128, kBoth) <= kBudget ? 128 : (bytes(64, kBoth) <= kBudget ? 64 : 32)));
+  // 4 x 8 products a thread; the deep models' tiles of 32 samples take 4 x 2 and 4 x 4
+  static constexpr int NTH = NT == 64 ? 128 : 256;
+  static constexpr size_t smem = bytes(NT, kBoth);
+  static_assert(smem <= kBudget, "fp32 backward does not fit shared memory");
+  static_assert(sizeof(TilePoints<32>) == 32 * 20, "tile points");
 };
 
-template <int D, int F, int IN, int H, int NT, bool kBoth>
-__global__ void __launch_bounds__(NT, 1)
+// The fp32 backward over tiles of NT samples.  next(pts) has the block's
+// threads write the next tile's points with their dL/dsigma and returns, after
+// a barrier, whether there is one.
+// Bound by shared-memory wavefronts (68 %) in the products, with the gathers and
+// the table reductions beside them.  16,384 rays x 256 samples, 16 x 2 levels, 2 x
+// 64: 10.96 -> 4.58 ms against one sample a thread (multiply-adds 1.96 ms;
+// without the gathers 3.95, without the scatter 3.9, without the weight gradients
+// 3.8 ms).  The gradients in a_H's place leave the L1 92 KB with two blocks an SM:
+// 4.77 -> 4.58 ms.
+template <int D, int F, int L, int H, typename T, typename Next>
+__device__ __forceinline__ void plain_backward(const GridDev& grid, const T* __restrict__ table,
+                                               const float* __restrict__ W, float tval, int act, int out_act,
+                                               float* __restrict__ table_grad, float* __restrict__ W_grad,
+                                               float* smem, Next&& next) {
+  constexpr int IN = L * F;
+  using Plan = PlainBwdPlan<IN, H>;
+  constexpr int NT = Plan::NT, NTH = Plan::NTH, LD = NT + 4;
+  const SimtWeights sw = stage_weights<IN, H, Plan::kBoth>(W, smem);
+  TilePoints<NT>& pts =
+      *reinterpret_cast<TilePoints<NT>*>(smem + simt_weight_floats<IN, H, Plan::kBoth>());
+  float* sX = reinterpret_cast<float*>(&pts + 1);   // [IN][LD]
+  float* sA = sX + IN * LD;                         // [H][64][LD]  a_1..a_H
+  float* sG = sA + (H - 1) * kWidth * LD;           // [max(64, IN)][LD]  the gradients, in a_H's place
+  const int t = threadIdx.x;
+  TileWGrad<IN, NT, NTH> g0;
+  g0.zero();
+  TileWGrad<kWidth, NT, NTH> gh[H - 1];
+#pragma unroll
+  for (int k = 0; k < H - 1; ++k) gh[k].zero();
+  constexpr int RT = NTH / kWidth;   // threads of a row
+  float dwout = 0.f;                 // of w_out[t / RT], over the thread's samples
+  while (next(pts)) {
+    encode_tile<D, F, L, NT, NTH, T>(grid, table, pts.p, pts.valid, tval, sX);
+    __syncthreads();
+    // forward: a_1..a_H into sA
+    {
+      TileProduct<IN, kWidth, NT, NTH> p;
+      p.run(sw.WT[0], sX);
+      p.store(sA, [&](float v, int) { return act_fwd(v, act); });
+    }
+#pragma unroll
+    for (int k = 1; k < H; ++k) {
+      __syncthreads();
+      TileProduct<kWidth, kWidth, NT, NTH> p;
+      p.run(sw.WT[k], sA + (k - 1) * kWidth * LD);
+      p.store(sA + k * kWidth * LD, [&](float v, int) { return act_fwd(v, act); });
+    }
+    __syncthreads();
+    const float* aH = sG;
+    if (t < NT) {
+      const float z = dot_col<kWidth, LD>(sw.wout, aH + t);
+      pts.d[t] = pts.valid[t] ? pts.d[t] * act_grad_z(z, out_act) : 0.f;
+    }
+    __syncthreads();
+    // w_out gradient, and G_H = dz * w_out * act'(a_H)
+    {
+      const int j = t / RT;
+      const float wj = sw.wout[j];
+#pragma unroll 4
+      for (int s = 4 * (t % RT); s < NT; s += 4 * RT) {
+        const float4 v = *reinterpret_cast<const float4*>(aH + j * LD + s);
+        const float4 dz = *reinterpret_cast<const float4*>(pts.d + s);
+        dwout = fmaf(dz.x, v.x, dwout);
+        dwout = fmaf(dz.y, v.y, dwout);
+        dwout = fmaf(dz.z, v.z, dwout);
+        dwout = fmaf(dz.w, v.w, dwout);
+        *reinterpret_cast<float4*>(sG + j * LD + s) =
+            make_float4(dz.x * wj * act_grad_a(v.x, act), dz.y * wj * act_grad_a(v.y, act),
+                        dz.z * wj * act_grad_a(v.z, act), dz.w * wj * act_grad_a(v.w, act));
+      }
+    }
+#pragma unroll
+    for (int k = H - 1; k >= 1; --k) {
+      __syncthreads();
+      const float* ak = sA + (k - 1) * kWidth * LD;
+      gh[k - 1].add(sG, ak);
+      // G_k = (W_k^T G_{k+1}) * act'(a_k); W_k is [64 out][64 in] = M[j][i]
+      TileProduct<kWidth, kWidth, NT, NTH> p;
+      p.run(sw.W[k], sG);
+      __syncthreads();
+      p.store(sG, [&](float v, int at) { return v * act_grad_a(ak[at], act); });
+    }
+    __syncthreads();
+    g0.add(sG, sX);
+    // dX = W_0^T G_1 (W_0 is [64][IN] = M[j][i]), then the scatter
+    {
+      TileProduct<kWidth, IN, NT, NTH> p;
+      p.run(sw.W[0], sG);
+      __syncthreads();
+      p.store(sG, [&](float v, int) { return v; });
+    }
+    __syncthreads();
+    {
+      const int s = t % NT;
+      if (pts.valid[s]) {
+        const float x[4] = {pts.p[s], pts.p[NT + s], pts.p[2 * NT + s], tval};
+#pragma unroll 1
+        for (int l = t / NT; l < L; l += NTH / NT) {
+          float d[F];
+#pragma unroll
+          for (int f = 0; f < F; ++f) d[f] = sG[(l * F + f) * LD + s];
+          scatter_level<D, F>(grid, table_grad, l, x, d);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  g0.flush(W_grad);
+#pragma unroll
+  for (int k = 0; k < H - 1; ++k) gh[k].flush(W_grad + kWidth * IN + k * kWidth * kWidth);
+#pragma unroll
+  for (int o = 1; o < RT; o <<= 1) dwout += __shfl_xor_sync(0xffffffffu, dwout, o);
+  if (t % RT == 0) atomicAdd(W_grad + kWidth * IN + (H - 1) * kWidth * kWidth + t / RT, dwout);
+}
+
+// Blocks of the fp32 backward: two to an SM where the plan fits twice.
+template <int IN, int H>
+__host__ __device__ constexpr int plain_bwd_per_sm() {
+  return PlainBwdPlan<IN, H>::kTwo ? 2 : 1;
+}
+
+// The training backward: tiles of 32 consecutive samples of each of NT / 32 rays.
+template <int D, int F, int L, int H>
+__global__ void __launch_bounds__(PlainBwdPlan<L * F, H>::NTH, plain_bwd_per_sm<L * F, H>())
 bwd_plain_kernel(GridDev grid, const float* __restrict__ table, const float* __restrict__ W, TrainArgs a,
                  const RayRec* __restrict__ recs, const int32_t* __restrict__ slot, unsigned int* __restrict__ ctrl,
                  int act, int out_act, float* __restrict__ table_grad, float* __restrict__ W_grad) {
-  constexpr int NW = NT / 32;
+  constexpr int NT = PlainBwdPlan<L * F, H>::NT;
   const bool by_pixel = !(ctrl[3] & kFlagDuplicatePixels);
-  constexpr int LD = NT + 4;
   extern __shared__ float4 smem4[];
-  float* smem = reinterpret_cast<float*>(smem4);
-  const SimtWeights sw = stage_weights<IN, H, kBoth>(W, smem);
-  float* cols = smem + simt_weight_floats<IN, H, kBoth>();
-  float* sX = cols;                      // [IN][LD]
-  float* sA = sX + IN * LD;              // [H][64][LD]  a_1..a_H
-  float* sG = sA + H * kWidth * LD;      // [64][LD]
-  float* sG2 = sG + kWidth * LD;         // [64][LD]
-  const int t = threadIdx.x;
-  const int lane = t & 31;
-  (void)NW;
-  constexpr bool kCarry0 = carry_layer0<IN, H, NT>();
-  constexpr bool kCarryH = carry_hidden<H, NT>();
-  WGrad<IN, NT, LD> g0;
-  g0.zero();
-  WGrad<kWidth, NT, LD> gh[kCarryH && H > 1 ? H - 1 : 1];
-#pragma unroll
-  for (int k = 0; k < (kCarryH ? H - 1 : 1); ++k) gh[k].zero();
-  float dwout[2] = {0.f, 0.f};  // lane owns w_out[lane] and w_out[lane + 32]
-
+  const int t = threadIdx.x, lane = t & 31;
   int ray = -1, base = 0;
   RayRec rec;
   rec.count = 0;
   rec.gsig = 0.f;
-  __syncthreads();
-  while (true) {
-    if (ray < a.num_rays && (ray < 0 || base >= rec.count)) {
-      const int r = next_ray(ctrl + 1, slot, recs, a.num_rays, a.n_pixels, by_pixel, lane);
-      if (r < 0) {
-        ray = a.num_rays;
-        rec.count = 0;
-      } else {
-        rec = load_ray(recs, r);
-        ray = r;
-        base = 0;
-      }
-    }
-    const bool warp_active = ray < a.num_rays;
-    if (!__syncthreads_or(warp_active)) break;
-
-    const int i = base + lane;
-    float p[4] = {0.f, 0.f, 0.f, 0.f};
-    bool valid = false;
-    if (warp_active && i < rec.count) valid = sample_point(rec, i, p);
-    if (D == 4) p[3] = a.t;
-    if (valid) {
-      encode_point<D, F, float>(grid, table, p, sX + t, LD);
-    } else {
-      for (int k = 0; k < IN; ++k) sX[k * LD + t] = 0.f;
-    }
-    // forward: a_1..a_H into sA
-    gemv_cols<IN, kWidth, LD>(sw.WT[0], sX + t, sA + t, act);
+  plain_backward<D, F, L, H>(
+      grid, table, W, a.t, act, out_act, table_grad, W_grad, reinterpret_cast<float*>(smem4),
+      [&](TilePoints<NT>& pts) -> bool {
+        bool active = false;
+        if (t < NT) {
+          if (ray < a.num_rays && (ray < 0 || base >= rec.count)) {
+            const int r = next_ray(ctrl + 1, slot, recs, a.num_rays, a.n_pixels, by_pixel, lane);
+            if (r < 0) {
+              ray = a.num_rays;
+              rec.count = 0;
+            } else {
+              rec = load_ray(recs, r);
+              ray = r;
+              base = 0;
+            }
+          }
+          active = ray < a.num_rays;
+          float p[4] = {0.f, 0.f, 0.f, 0.f};
+          const bool valid = active && base + lane < rec.count && sample_point(rec, base + lane, p);
 #pragma unroll
-    for (int k = 1; k < H; ++k)
-      gemv_cols<kWidth, kWidth, LD>(sw.WT[k], sA + (k - 1) * kWidth * LD + t, sA + k * kWidth * LD + t, act);
-    const float* aH = sA + (H - 1) * kWidth * LD + t;
-    const float z = dot_col<kWidth, LD>(sw.wout, aH);
-    const float dz = valid ? rec.gsig * act_grad_z(z, out_act) : 0.f;
-    // w_out gradient (sum over the warp's samples), and G_H = dz * w_out * act'(a_H)
-#pragma unroll 4
-    for (int j = 0; j < kWidth; ++j) {
-      const float aj = aH[j * LD];
-      const float v = warp_sum(dz * aj);
-      if ((j & 31) == lane) dwout[j >> 5] += v;
-      sG[j * LD + t] = dz * sw.wout[j] * act_grad_a(aj, act);
-    }
-    float* G = sG;
-    float* G2 = sG2;
-#pragma unroll
-    for (int k = H - 1; k >= 1; --k) {
-      __syncthreads();
-      if constexpr (kCarryH) {
-        gh[k - 1].add(G, sA + (k - 1) * kWidth * LD);
-      } else {  // this layer's tile, added to W_grad now
-        gh[0].zero();
-        gh[0].add(G, sA + (k - 1) * kWidth * LD);
-        gh[0].flush(W_grad + kWidth * IN + (k - 1) * kWidth * kWidth);
-      }
-      // G_k = (W_k^T G_{k+1}) * act'(a_k); W_k is [64 out][64 in] = M[j][i]
-      gemv_cols<kWidth, kWidth, LD>(sw.W[k], G + t, G2 + t, NECTB_ACT_NONE);
-      const float* ak = sA + (k - 1) * kWidth * LD + t;
-      for (int j = 0; j < kWidth; ++j) G2[j * LD + t] *= act_grad_a(ak[j * LD], act);
-      float* tmp = G;
-      G = G2;
-      G2 = tmp;
-    }
-    __syncthreads();
-    if constexpr (!kCarry0) g0.zero();
-    g0.add(G, sX);
-    if constexpr (!kCarry0) g0.flush(W_grad);
-    // dX = W_0^T G_1 (W_0 is [64][IN] = M[j][i]) into G2, then scatter
-    gemv_cols<kWidth, IN, LD>(sw.W[0], G + t, G2 + t, NECTB_ACT_NONE);
-    // per-sample atomics: the SIMT path is issue-bound and the run reduction's
-    // shuffles cost it more than the atomics they save (measured)
-    scatter_warp<D, F>(grid, table_grad, p, valid, G2 + t, (int64_t)F * LD, LD, 0u, 0, grid.n_levels);
-    __syncthreads();
-    base += 32;
-  }
-  if constexpr (kCarry0) g0.flush(W_grad);
-  if constexpr (kCarryH) {
-#pragma unroll
-    for (int k = 0; k < H - 1; ++k) gh[k].flush(W_grad + kWidth * IN + k * kWidth * kWidth);
-  }
-  const int nHidden = kWidth * IN + (H - 1) * kWidth * kWidth;
-  // combine the warps' w_out partials through shared memory (reuse sG)
-  __syncthreads();
-  float* red = sG;  // [NW][64]
-  red[(t >> 5) * kWidth + lane] = dwout[0];
-  red[(t >> 5) * kWidth + lane + 32] = dwout[1];
-  __syncthreads();
-  for (int j = t; j < kWidth; j += NT) {  // tiles of 32 samples: each thread adds two entries
-    float s = 0.f;
-    for (int w = 0; w < NT / 32; ++w) s += red[w * kWidth + j];
-    atomicAdd(W_grad + nHidden + j, s);
-  }
+          for (int k = 0; k < 3; ++k) pts.p[k * NT + t] = p[k];
+          pts.valid[t] = valid ? 1 : 0;
+          pts.d[t] = rec.gsig;
+          base += 32;
+        }
+        return __syncthreads_or(active) != 0;
+      });
 }
 
 // Backward of the model at n independent points (nectb_model_backward):
 // gradients of sum_i dsigma[i] * sigma(x_i) added to the table and weight
-// gradients.  The pipeline of bwd_plain_kernel (fp32 SIMT MLP, register tile
-// weight gradients, per-sample table reductions) with points read from x
-// (n x 3, (z, y, x); t broadcast in 4D) instead of regenerated along rays
-// and a per-point dL/dsigma.  Tables of either precision are gathered.
-template <int D, int F, int IN, int H, int NT, bool kBoth, typename T>
-__global__ void __launch_bounds__(NT, 1)
+// gradients, the points read from x (n x 3, (z, y, x); t broadcast in 4D).
+// Tables of either precision are gathered.
+template <int D, int F, int L, int H, typename T>
+__global__ void __launch_bounds__(PlainBwdPlan<L * F, H>::NTH, plain_bwd_per_sm<L * F, H>())
 model_bwd_kernel(GridDev grid, const T* __restrict__ table, const float* __restrict__ W, const float* __restrict__ x,
                  int64_t n, float tval, const float* __restrict__ t_dev, const float* __restrict__ dsigma, int act,
                  int out_act, float* __restrict__ table_grad, float* __restrict__ W_grad) {
-  constexpr int LD = NT + 4;
+  constexpr int NT = PlainBwdPlan<L * F, H>::NT;
   extern __shared__ float4 smem4[];
-  float* smem = reinterpret_cast<float*>(smem4);
-  const SimtWeights sw = stage_weights<IN, H, kBoth>(W, smem);
-  float* cols = smem + simt_weight_floats<IN, H, kBoth>();
-  float* sX = cols;                      // [IN][LD]
-  float* sA = sX + IN * LD;              // [H][64][LD]
-  float* sG = sA + H * kWidth * LD;      // [64][LD]
-  float* sG2 = sG + kWidth * LD;         // [64][LD]
   const int t = threadIdx.x;
-  const int lane = t & 31;
-  constexpr bool kCarry0 = carry_layer0<IN, H, NT>();
-  constexpr bool kCarryH = carry_hidden<H, NT>();
-  WGrad<IN, NT, LD> g0;
-  g0.zero();
-  WGrad<kWidth, NT, LD> gh[kCarryH && H > 1 ? H - 1 : 1];
-#pragma unroll
-  for (int k = 0; k < (kCarryH ? H - 1 : 1); ++k) gh[k].zero();
-  float dwout[2] = {0.f, 0.f};
   if (D == 4 && t_dev) tval = *t_dev;   // the broadcast timestep, read on the device
-  __syncthreads();
-  for (int64_t c0 = (int64_t)blockIdx.x * NT; c0 < n; c0 += (int64_t)gridDim.x * NT) {  // block-uniform
-    const int64_t i = c0 + t;
-    const bool valid = i < n;
-    float p[4] = {0.f, 0.f, 0.f, 0.f};
-    if (valid) {
+  int64_t c0 = (int64_t)blockIdx.x * NT;
+  plain_backward<D, F, L, H>(
+      grid, table, W, tval, act, out_act, table_grad, W_grad, reinterpret_cast<float*>(smem4),
+      [&](TilePoints<NT>& pts) -> bool {
+        if (c0 >= n) return false;
+        if (t < NT) {
+          const int64_t i = c0 + t;
+          const bool valid = i < n;
 #pragma unroll
-      for (int k = 0; k < 3; ++k) p[k] = x[i * 3 + k];
-    }
-    if (D == 4) p[3] = tval;
-    if (valid) {
-      encode_point<D, F, T>(grid, table, p, sX + t, LD);
-    } else {
-      for (int k = 0; k < IN; ++k) sX[k * LD + t] = 0.f;
-    }
-    gemv_cols<IN, kWidth, LD>(sw.WT[0], sX + t, sA + t, act);
-#pragma unroll
-    for (int k = 1; k < H; ++k)
-      gemv_cols<kWidth, kWidth, LD>(sw.WT[k], sA + (k - 1) * kWidth * LD + t, sA + k * kWidth * LD + t, act);
-    const float* aH = sA + (H - 1) * kWidth * LD + t;
-    const float z = dot_col<kWidth, LD>(sw.wout, aH);
-    const float dz = valid ? dsigma[i] * act_grad_z(z, out_act) : 0.f;
-#pragma unroll 4
-    for (int j = 0; j < kWidth; ++j) {
-      const float aj = aH[j * LD];
-      const float v = warp_sum(dz * aj);
-      if ((j & 31) == lane) dwout[j >> 5] += v;
-      sG[j * LD + t] = dz * sw.wout[j] * act_grad_a(aj, act);
-    }
-    float* G = sG;
-    float* G2 = sG2;
-#pragma unroll
-    for (int k = H - 1; k >= 1; --k) {
-      __syncthreads();
-      if constexpr (kCarryH) {
-        gh[k - 1].add(G, sA + (k - 1) * kWidth * LD);
-      } else {  // this layer's tile, added to W_grad now
-        gh[0].zero();
-        gh[0].add(G, sA + (k - 1) * kWidth * LD);
-        gh[0].flush(W_grad + kWidth * IN + (k - 1) * kWidth * kWidth);
-      }
-      gemv_cols<kWidth, kWidth, LD>(sw.W[k], G + t, G2 + t, NECTB_ACT_NONE);
-      const float* ak = sA + (k - 1) * kWidth * LD + t;
-      for (int j = 0; j < kWidth; ++j) G2[j * LD + t] *= act_grad_a(ak[j * LD], act);
-      float* tmp = G;
-      G = G2;
-      G2 = tmp;
-    }
-    __syncthreads();
-    if constexpr (!kCarry0) g0.zero();
-    g0.add(G, sX);
-    if constexpr (!kCarry0) g0.flush(W_grad);
-    gemv_cols<kWidth, IN, LD>(sw.W[0], G + t, G2 + t, NECTB_ACT_NONE);
-    scatter_warp<D, F>(grid, table_grad, p, valid, G2 + t, (int64_t)F * LD, LD, 0u, 0, grid.n_levels);
-    __syncthreads();
-  }
-  if constexpr (kCarry0) g0.flush(W_grad);
-  if constexpr (kCarryH) {
-#pragma unroll
-    for (int k = 0; k < H - 1; ++k) gh[k].flush(W_grad + kWidth * IN + k * kWidth * kWidth);
-  }
-  const int nHidden = kWidth * IN + (H - 1) * kWidth * kWidth;
-  __syncthreads();
-  float* red = sG;  // [NT/32][64]
-  red[(t >> 5) * kWidth + lane] = dwout[0];
-  red[(t >> 5) * kWidth + lane + 32] = dwout[1];
-  __syncthreads();
-  for (int j = t; j < kWidth; j += NT) {  // tiles of 32 samples: each thread adds two entries
-    float s = 0.f;
-    for (int w = 0; w < NT / 32; ++w) s += red[w * kWidth + j];
-    atomicAdd(W_grad + nHidden + j, s);
-  }
+          for (int k = 0; k < 3; ++k) pts.p[k * NT + t] = valid ? x[i * 3 + k] : 0.f;
+          pts.valid[t] = valid ? 1 : 0;
+          pts.d[t] = valid ? dsigma[i] : 0.f;
+        }
+        c0 += (int64_t)gridDim.x * NT;
+        __syncthreads();
+        return true;
+      });
 }
 
 template <int D, int F, int L, int H, typename T>
@@ -581,17 +499,17 @@ int launch_model_bwd(const GridDev& grid, const void* table, const float* W, con
                      const float* t_dev, const float* dsigma, int act, int out_act, float* table_grad, float* W_grad,
                      cudaStream_t s) {
   constexpr int IN = L * F;
-  using Plan = SimtBwdPlan<IN, H>;
-  constexpr int NT = Plan::NT;
-  auto k = model_bwd_kernel<D, F, IN, H, NT, Plan::kBoth, T>;
+  using Plan = PlainBwdPlan<IN, H>;
+  auto k = model_bwd_kernel<D, F, L, H, T>;
   const size_t smem = Plan::smem;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(sms, ceil_div(n, NT)));
+  const int blocks =
+      (int)std::max<int64_t>(1, std::min<int64_t>(plain_bwd_per_sm<IN, H>() * sms, ceil_div(n, Plan::NT)));
   ProfScope ps(kProfModel, s);
-  k<<<blocks, NT, smem, s>>>(grid, (const T*)table, W, x, n, tval, t_dev, dsigma, act, out_act, table_grad, W_grad);
+  k<<<blocks, Plan::NTH, smem, s>>>(grid, (const T*)table, W, x, n, tval, t_dev, dsigma, act, out_act, table_grad, W_grad);
   return launch_status("model_bwd_kernel");
 }
 
@@ -605,34 +523,32 @@ int run_plain(const NectbGeometry& geo, const GridDev& grid, const float* table,
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   (void)geo;
 
-  constexpr int FNT = kPlainFwdThreads;
-  auto fk = fwd_plain_kernel<D, F, IN, H>;
-  const size_t fsmem =
-      (size_t)(simt_weight_floats<IN, H, false>() + (IN + simt_hidden_buffers<H>() * kWidth) * (FNT + 4)) * 4;
+  auto fk = fwd_plain_kernel<D, F, L, H>;
+  const size_t fsmem = tile_forward_smem<IN, H, kPlainFwdSamples>();
   set_smem(fk, fsmem, a.max_blocks > 0);
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fk, FNT, fsmem);
-  int fblocks = std::max(1, std::min<int>(sms * std::max(per_sm, 1), (int)ceil_div(a.num_rays, FNT / 32)));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fk, kTileThreads, fsmem);
+  int fblocks = std::max(1, std::min<int>(sms * std::max(per_sm, 1), (int)ceil_div(a.num_rays, kPlainFwdSamples / 32)));
   if (a.max_blocks > 0) fblocks = std::min(fblocks, a.max_blocks);
   if (a.phase & kPhaseForward) {
     {
       ProfScope ps(kProfForward, s);
-      fk<<<fblocks, FNT, fsmem, s>>>(grid, table, W, a, ws.rays, ws.slot, ws.counters, act, out_act, y_pred, loss);
+      fk<<<fblocks, kTileThreads, fsmem, s>>>(grid, table, W, a, ws.rays, ws.slot, ws.counters, act, out_act, y_pred, loss);
     }
     if (int rc = launch_status("fwd_plain_kernel")) return rc;
   }
   if (!table_grad || !(a.phase & kPhaseBackward)) return NECTB_OK;  // forward only (queries, split step)
 
-  using Plan = SimtBwdPlan<IN, H>;
-  constexpr int NT = Plan::NT;
-  auto bk = bwd_plain_kernel<D, F, IN, H, NT, Plan::kBoth>;
+  using Plan = PlainBwdPlan<IN, H>;
+  auto bk = bwd_plain_kernel<D, F, L, H>;
   const size_t bsmem = Plan::smem;
   cudaFuncSetAttribute(bk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem);
-  const int bblocks = std::max(1, std::min<int>(sms, (int)ceil_div(a.num_rays, NT / 32)));
+  const int bblocks =
+      std::max(1, std::min<int>(plain_bwd_per_sm<IN, H>() * sms, (int)ceil_div(a.num_rays, Plan::NT / 32)));
   {
     ProfScope ps(kProfBackward, s);
-    bk<<<bblocks, NT, bsmem, s>>>(grid, table, W, a, ws.rays, ws.slot, ws.counters, act, out_act, table_grad,
-                                  W_grad);
+    bk<<<bblocks, Plan::NTH, bsmem, s>>>(grid, table, W, a, ws.rays, ws.slot, ws.counters, act, out_act,
+                                            table_grad, W_grad);
   }
   return launch_status("bwd_plain_kernel");
 }
