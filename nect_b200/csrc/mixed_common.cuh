@@ -24,6 +24,27 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
   return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
 }
 
+// TMEM columns of a block of n_wg warpgroups: 64 each, allocated as a power of two.
+__host__ __device__ constexpr uint32_t wg_tmem_cols(int n_wg) {
+  return n_wg <= 1 ? 64u : (n_wg == 2 ? 128u : (n_wg <= 4 ? 256u : 512u));
+}
+
+// Barrier over the 128 threads of warpgroup wg (named barrier wg + 1; 0 is
+// __syncthreads'), and its OR-reduction form.
+__device__ __forceinline__ void wg_sync(int wg) { asm volatile("bar.sync %0, 128;" ::"r"(wg + 1) : "memory"); }
+__device__ __forceinline__ bool wg_or(int wg, bool p) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred pi, po;\n\t"
+      "setp.ne.u32 pi, %1, 0;\n\t"
+      "bar.red.or.pred po, %2, 128, pi;\n\t"
+      "selp.u32 %0, 1, 0, po;\n\t}\n"
+      : "=r"(r)
+      : "r"((uint32_t)p), "r"(wg + 1)
+      : "memory");
+  return r != 0;
+}
+
 // fp32 weights (PyTorch layout) -> bf16 swizzled tiles: W0 rows o over KT
 // tiles (input columns beyond IN are zero), W1..W_{H-1} rows o in the tiles
 // after them; w_out fp32.

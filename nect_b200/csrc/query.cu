@@ -28,9 +28,6 @@ int launch_time_slice(const GridDev& grid, const __half* table, float t, __half*
 namespace {
 
 constexpr int kQThreads = 128;
-constexpr uint32_t kQTile = 128 * 128;
-constexpr uint32_t kQWTile = 64 * 128;
-
 __device__ __forceinline__ int find_item(const NectbQueryItem* __restrict__ items, int n, int64_t chunk) {
   int lo = 0, hi = n - 1;
   while (lo < hi) {
@@ -69,15 +66,18 @@ __device__ __forceinline__ QPoint query_point(const NectbQueryItem& it, int64_t 
   return q;
 }
 
-__device__ __forceinline__ uint8_t* qalign1024(uint8_t* p) {
-  return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
-}
-
-// At most 128 registers so that three blocks share an SM under the 164 KB
-// shared split (a background block beside two slice blocks, or three blocks of
-// one query).
-template <int D, int F, int L, int H, int ACT>
-__global__ void __launch_bounds__(kQThreads, 4)
+// A block is n_wg = blockDim / 128 independent warpgroups sharing one copy of
+// the weight tiles; each takes chunks of 128 points on its own, with its own X
+// tiles (which the layers' activations overwrite), 64 TMEM columns, mbarrier and
+// named barrier.  kMaxWg = 1: one warpgroup a block, at most 128 registers, so
+// that three blocks share an SM with other kernels (capped grids: a server's
+// lanes).  kMaxWg > 1: one block an SM for a launch that has the GPU to itself.
+// Waits on the gathers and on the layers' chain of products, so the more
+// warpgroups an SM holds the better: 256^3 points of the 19 x 4 model with 6
+// layers (one 107 KB block an SM before) 17.8 -> 12.5 ms, a 256^2 slice of the 4D
+// 16 x 2 model 49.5 -> 35.7 us.
+template <int D, int F, int L, int H, int ACT, int kMaxWg>
+__global__ void __launch_bounds__(kQThreads * kMaxWg, kMaxWg == 1 ? 4 : 1)
 query_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __restrict__ W,
                    const NectbQueryItem* __restrict__ items, int n_items, int64_t total_chunks,
                    unsigned int* __restrict__ counter, int out_act) {
@@ -85,103 +85,127 @@ query_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* 
   constexpr int KT = S::KT;
   constexpr int act = ACT;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* base = qalign1024(smem_raw);
+  uint8_t* base = align1024(smem_raw);
+  const int n_wg = blockDim.x / kQThreads;
   uint8_t* sW = base;                   // KT + H - 1 weight tiles
-  uint8_t* sX = sW + (KT + H - 1) * kQWTile;
-  uint8_t* sA = sX + KT * kQTile;       // every hidden layer's activations in turn
-  float* sWout = reinterpret_cast<float*>(sA + kQTile);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sWout + 64);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
-  long long* s_chunk = reinterpret_cast<long long*>(tslot + 2);
-  int* s_item = reinterpret_cast<int*>(s_chunk + 1);
+  float* sWout = reinterpret_cast<float*>(sW + (KT + H - 1) * kWTile + n_wg * KT * kTile);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sWout + 64);              // [kMaxWg]
+  long long* chunks = reinterpret_cast<long long*>(bars + kMaxWg);       // [kMaxWg]
+  int* item = reinterpret_cast<int*>(chunks + kMaxWg);                   // [kMaxWg]
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(item + kMaxWg);
 
   const int t = threadIdx.x, warp = t >> 5;
+  const int wg = t / kQThreads, r = t % kQThreads;
+  uint8_t* sX = sW + (KT + H - 1) * kWTile + wg * KT * kTile;
+  uint64_t* bar = bars + wg;
   // fp32 weights -> bf16 swizzled tiles (same layout as the training kernels)
   stage_mixed_weights<L, F, H>(W, sW, sWout);
+  const uint32_t ncols = wg_tmem_cols(n_wg);
   if (warp == 0) {
-    tc::tmem_alloc(tslot, 128);
+    tc::tmem_alloc(tslot, ncols);
     tc::tmem_relinquish();
   }
-  if (t == 0) tc::mbar_init(bar, 1);
+  if (r == 0) tc::mbar_init(bar, 1);
   tc::fence_async_smem();
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
-  const uint32_t tm = *tslot;
-  const uint32_t my_lanes = tm + ((uint32_t)(32 * warp) << 16);
-  const uint32_t sX_a = tc::smem_u32(sX), sA_a = tc::smem_u32(sA), sW_a = tc::smem_u32(sW);
+  const uint32_t tm = *tslot + 64u * wg;   // this warpgroup's columns
+  const uint32_t my_lanes = tm + ((uint32_t)(32 * (warp & 3)) << 16);
+  const uint32_t sX_a = tc::smem_u32(sX), sW_a = tc::smem_u32(sW);
   constexpr uint32_t idesc = tc::idesc_bf16(128, 64, false, false);
   uint32_t phase = 0;
   bool timed_out = false;
   while (true) {
-    if (t == 0) {
+    if (r == 0) {
       const long long c = (long long)atomicAdd(counter, 1u);
-      *s_chunk = c;
-      *s_item = c < total_chunks ? find_item(items, n_items, c) : 0;
+      chunks[wg] = c;
+      item[wg] = c < total_chunks ? find_item(items, n_items, c) : 0;
     }
-    __syncthreads();
-    const long long chunk = *s_chunk;
+    wg_sync(wg);
+    const long long chunk = chunks[wg];
     if (chunk >= total_chunks) break;
-    const QPoint q = query_point(items[*s_item], chunk, t);
-    encode_row<D, F, L>(grid, table, q.p, q.valid, sX, t);   // the encoder's row writer (fp16 gathers, bf16 row)
-    // layer k writes TMEM columns 64 * (k & 1); its input is X for k = 0, else
-    // the previous layer's activations in sA (written once the MMA that read
-    // sA before has completed)
-    float h[64];
+    const QPoint q = query_point(items[item[wg]], chunk, r);
+    encode_row<D, F, L>(grid, table, q.p, q.valid, sX, r);   // the encoder's row writer (fp16 gathers, bf16 row)
+    // every layer writes the warpgroup's 64 TMEM columns; its input is X for
+    // k = 0, else the previous layer's activations, which overwrite X's first
+    // tile once layer 0's product has completed
+    float z = 0.f;
 #pragma unroll
     for (int k = 0; k < H; ++k) {
-      if (k > 0) {
-        uint32_t mlo, mhi;
-        act_row(h, sA, t, act, mlo, mhi);
-      }
       tc::fence_async_smem();
       tc::fence_before();
-      __syncthreads();
-      if (t == 0) {
+      wg_sync(wg);
+      if (r == 0) {
         tc::fence_after();
         if (k == 0) {
 #pragma unroll
           for (int c = 0; c < S::INP / 16; ++c)
-            tc::mma(tm, tc::desc_k(sX_a + (c / 4) * kQTile, c % 4), tc::desc_k(sW_a + (c / 4) * kQWTile, c % 4),
-                    idesc, c > 0);
+            tc::mma(tm, tc::desc_k(sX_a + (c / 4) * kTile, c % 4), tc::desc_k(sW_a + (c / 4) * kWTile, c % 4), idesc,
+                    c > 0);
         } else {
 #pragma unroll
           for (int c = 0; c < 4; ++c)
-            tc::mma(tm + 64 * (k & 1), tc::desc_k(sA_a, c), tc::desc_k(sW_a + (KT + k - 1) * kQWTile, c), idesc,
-                    c > 0);
+            tc::mma(tm, tc::desc_k(sX_a, c), tc::desc_k(sW_a + (KT + k - 1) * kWTile, c), idesc, c > 0);
         }
         tc::commit(bar);
       }
       timed_out = !tc::mbar_wait(bar, phase);
       phase ^= 1;
-      if (__syncthreads_or(timed_out)) {
+      if (wg_or(wg, timed_out)) {
         timed_out = true;
         break;
       }
       tc::fence_after();
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tc::tmem_ld16(my_lanes + 64 * (k & 1) + 16 * c, h + 16 * c);
-      tc::tmem_wait_ld();
+      for (int half = 0; half < 2; ++half) {   // 32 columns at a time
+        float v[32];
+        tc::tmem_ld16(my_lanes + 32 * half, v);
+        tc::tmem_ld16(my_lanes + 32 * half + 16, v + 16);
+        tc::tmem_wait_ld();
+        if (k + 1 < H) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            float a8[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a8[j] = hidden_act(v[8 * c + j], act);
+            tc::st_chunk_bf16(sX, r, 4 * half + c, a8);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) z = fmaf(sWout[32 * half + j], hidden_act(v[j], act), z);
+        }
+      }
     }
     if (timed_out) break;
-    float z = 0.f;
-#pragma unroll
-    for (int j = 0; j < 64; ++j) z = fmaf(sWout[j], hidden_act(h[j], act), z);
     if (q.valid) *q.dst = fmaf(act_fwd(z, out_act), q.scale, q.offset);
     tc::fence_before();
-    __syncthreads();
   }
   if (timed_out) {
     tc::mbar_wait(bar, phase);  // let the MMA in flight finish before TMEM is freed
-    if (t == 0) atomicOr(counter + 1, 1u);
+    if (r == 0) atomicOr(counter + 1, 1u);
   }
   tc::fence_before();
   __syncthreads();
   if (warp == 0) {
     tc::fence_after();
-    tc::tmem_dealloc(tm, 128);
+    tc::tmem_dealloc(*tslot, ncols);
   }
 }
+
+// Warpgroups of the wide form: as many as the registers of the shape allow (80 a
+// thread for 3D grids of 16 levels and two layers, 102 for the deep model, 128
+// otherwise; the training forward's numbers) and the shared memory holds.
+template <int D, int L, int F, int H>
+struct QueryShape {
+  using S = InShape<L, F>;
+  static constexpr size_t bytes(int n_wg) {
+    return 1024 + (S::KT + H - 1) * kWTile + (size_t)n_wg * S::KT * kTile + 64 * 4 + 6 * 20 + 16;
+  }
+  static constexpr int kRegWg = D == 3 ? (H == 2 ? 6 : (L == 16 ? 4 : 5)) : 4;
+  static constexpr int kMaxWg = bytes(kRegWg) <= 227 * 1024 ? kRegWg : 4;
+  static_assert(bytes(kMaxWg) <= 227 * 1024 && kMaxWg * 64 <= 512, "query block");
+};
 
 // fp32: a chunk is a tile of 128 points (mlp_tile.cuh).
 template <int D, int F, typename T, int L, int H>
@@ -236,16 +260,25 @@ int sm_count() {
 template <int D, int F, int L, int H, int ACT>
 int launch_query_mixed(const GridDev& g, const void* table, const float* W, const NectbQueryItem* items, int n,
                        int64_t chunks, unsigned int* counter, int oact, int max_blocks, cudaStream_t s) {
-  using S = InShape<L, F>;
-  auto k = query_mixed_kernel<D, F, L, H, ACT>;
-  const size_t smem = 1024 + (S::KT + H - 1) * kQWTile + (S::KT + 1) * kQTile + 64 * 4 + 64;
-  set_smem(k, smem, true);
-  int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(chunks, 3 * sm_count()));
-  if (max_blocks > 0) blocks = std::min(blocks, max_blocks);
+  using Q = QueryShape<D, L, F, H>;
   GridDev gt = g;  // with a texture over the table for the gathers
   gt.tex = table_texture(table, (size_t)g.total_entries * F * sizeof(__half), F * (int)sizeof(__half));
   ProfScope ps(kProfModel, s);
-  k<<<blocks, kQThreads, smem, s>>>(gt, (const __half*)table, W, items, n, chunks, counter, oact);
+  if (max_blocks > 0) {
+    auto k = query_mixed_kernel<D, F, L, H, ACT, 1>;
+    set_smem(k, Q::bytes(1), true);
+    const int blocks =
+        (int)std::max<int64_t>(1, std::min<int64_t>({chunks, 3 * (int64_t)sm_count(), (int64_t)max_blocks}));
+    k<<<blocks, kQThreads, Q::bytes(1), s>>>(gt, (const __half*)table, W, items, n, chunks, counter, oact);
+  } else {
+    // a launch below one chunk a warpgroup spreads over the SMs first
+    auto k = query_mixed_kernel<D, F, L, H, ACT, Q::kMaxWg>;
+    const int sms = sm_count();
+    const int wgs = (int)std::max<int64_t>(1, std::min<int64_t>(Q::kMaxWg, ceil_div(chunks, sms)));
+    set_smem(k, Q::bytes(Q::kMaxWg), false);
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(chunks, wgs), sms));
+    k<<<blocks, kQThreads * wgs, Q::bytes(wgs), s>>>(gt, (const __half*)table, W, items, n, chunks, counter, oact);
+  }
   return launch_status("query_mixed_kernel");
 }
 

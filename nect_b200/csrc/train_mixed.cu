@@ -115,27 +115,6 @@ struct FwdShape {
       (D == 3 && H == 2) ? kFwdBlocksPerSM : (kFwdBlocksPerSM < 4 ? kFwdBlocksPerSM : 4);
 };
 
-// TMEM columns of a forward block of n_wg warpgroups: 64 each, allocated as a power of two.
-__host__ __device__ constexpr uint32_t fwd_tmem_cols(int n_wg) {
-  return n_wg <= 1 ? 64u : (n_wg == 2 ? 128u : (n_wg <= 4 ? 256u : 512u));
-}
-
-// Barrier over the 128 threads of warpgroup wg (named barrier wg + 1; 0 is
-// __syncthreads'), and its OR-reduction form.
-__device__ __forceinline__ void wg_sync(int wg) { asm volatile("bar.sync %0, 128;" ::"r"(wg + 1) : "memory"); }
-__device__ __forceinline__ bool wg_or(int wg, bool p) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred pi, po;\n\t"
-      "setp.ne.u32 pi, %1, 0;\n\t"
-      "bar.red.or.pred po, %2, 128, pi;\n\t"
-      "selp.u32 %0, 1, 0, po;\n\t}\n"
-      : "=r"(r)
-      : "r"((uint32_t)p), "r"(wg + 1)
-      : "memory");
-  return r != 0;
-}
-
 template <int D, int F, int L, int H, int ACT>
 __global__ void __launch_bounds__(FwdShape<D, L, F, H>::kMaxWarpgroups * kMixThreads, 1)
 fwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __restrict__ W, TrainArgs a,
@@ -168,7 +147,7 @@ fwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
   uint64_t* bar = bars + wg;
   if (xstore && blockIdx.x == 0 && t == 0) ctrl[7] = xcap;  // rows this forward fills, for the backward
   stage_mixed_weights<L, F, H>(W, sW, sWout);
-  const uint32_t ncols = fwd_tmem_cols(n_wg);
+  const uint32_t ncols = wg_tmem_cols(n_wg);
   if (warp == 0) {
     tc::tmem_alloc(tslot, ncols);
     tc::tmem_relinquish();

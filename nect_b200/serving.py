@@ -144,7 +144,8 @@ def _call_points_slice(model: _HashGridModel, slice_ptr: int, items_dev: int, n_
 def query_points(model: _HashGridModel, items: np.ndarray, stream: torch.cuda.Stream | None = None,
                  max_blocks: int = 0, slice: torch.Tensor | None = None):
     """Evaluate the items (any requests) in one launch (outputs written in place);
-    max_blocks > 0 caps the persistent grid.  With ``slice`` (time_slice at
+    max_blocks > 0 caps the persistent grid, in blocks that leave room on an SM for
+    other kernels; 0 takes the whole GPU.  With ``slice`` (time_slice at
     some t) every item is evaluated on it, at its t."""
     if items.size == 0:
         return
@@ -269,7 +270,7 @@ class _Lane:
     """One stream with graph-captured point launches (one graph per bucket).
 
     priority: CUDA stream priority (lower is higher priority); max_blocks caps
-    the persistent grid (0 = two blocks per SM)."""
+    the persistent grid of one-warpgroup blocks (0 = one wide block per SM)."""
 
     def __init__(self, dev, priority: int = 0, max_blocks: int = 0):
         self.stream = torch.cuda.Stream(device=dev, priority=priority)
@@ -389,7 +390,8 @@ class QueryServer:
             raise ValueError("slow_warpgroups must be 1..6 and piece_pixels positive")
         self.slow_warpgroups = slow_warpgroups
         lo, hi = torch.cuda.Stream.priority_range()
-        self.fast = [_Lane(self.dev, priority=hi) for _ in range(n_fast)]
+        # both kinds of lane run one-warpgroup blocks (a capped grid), which share SMs
+        self.fast = [_Lane(self.dev, priority=hi, max_blocks=3 * sms) for _ in range(n_fast)]
         self.slow = [_Lane(self.dev, priority=lo, max_blocks=self.slow_blocks) for _ in range(n_slow)]
         for ln in self.fast + self.slow:
             ln.capture(model)
