@@ -9,6 +9,7 @@
 // w_out stays fp32.
 #pragma once
 #include <cuda_fp16.h>
+#include <type_traits>
 
 #include "common.cuh"
 #include "hashgrid.cuh"
@@ -102,15 +103,119 @@ __device__ __forceinline__ void act_row(const float* h, uint8_t* tile, int r, in
   }
 }
 
+// The raw corner entries of one level at p (coordinates in [0, 1]) and the
+// fractions along the axes: the integers and fractions of level_corners, with the
+// index rule of the level (hash or strides) taken by one uniform branch instead of
+// a select per corner, and 32-bit entry offsets from the level's base.
+template <int D, int F>
+struct LevelFetch {
+  using Raw = std::conditional_t<F == 2, unsigned int, uint2>;   // an entry: F fp16 features
+  Raw raw[1 << D];
+  float f[D];
+
+  __device__ __forceinline__ void load(const GridDev& g, const __half* __restrict__ table, int l, const float* p) {
+    uint32_t c[D];
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      const int res = g.res[l][k];
+      const float q = __fmul_rn(p[k], (float)res);   // as level_corners
+      const int ci = min((int)floorf(q), res - 1);   // q >= 0
+      c[k] = (uint32_t)ci;
+      f[k] = q - (float)ci;
+    }
+    uint32_t idx[1 << D];
+    const bool hashed = (g.hashed_bits >> l) & 1u;
+    if (hashed) {
+      const uint32_t m = g.hash_mask;
+      const uint32_t t1[2] = {c[1] * kPrime1, c[1] * kPrime1 + kPrime1};
+      const uint32_t t2[2] = {c[2] * kPrime2, c[2] * kPrime2 + kPrime2};
+      uint32_t row[1 << (D - 1)];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) row[r] = t1[r & 1] ^ t2[r >> 1];
+      if constexpr (D == 4) {
+        const uint32_t t3[2] = {c[3] * kPrime3, c[3] * kPrime3 + kPrime3};
+#pragma unroll
+        for (int r = 4; r < 8; ++r) row[r] = row[r - 4] ^ t3[1];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) row[r] ^= t3[0];
+      }
+#pragma unroll
+      for (int i = 0; i < (1 << D); ++i) idx[i] = ((c[0] + (i & 1)) ^ row[i >> 1]) & m;
+    } else {
+      uint32_t row[1 << (D - 1)];
+      const uint32_t base = c[0] + c[1] * g.stride[l][1] + c[2] * g.stride[l][2] +
+                            (D == 4 ? c[D - 1] * g.stride[l][3] : 0u);
+#pragma unroll
+      for (int r = 0; r < (1 << (D - 1)); ++r) {
+        row[r] = base;
+#pragma unroll
+        for (int k = 1; k < D; ++k)
+          if ((r >> (k - 1)) & 1) row[r] += g.stride[l][k];
+      }
+#pragma unroll
+      for (int i = 0; i < (1 << D); ++i) idx[i] = row[i >> 1] + (i & 1);
+    }
+    // the odd hashed levels' corners through the texture path (a second L1 data
+    // pipe beside the load/store unit's), the others as loads
+    if (g.tex && hashed && (l & 1)) {
+      const int off = (int)g.offset[l];
+#pragma unroll
+      for (int i = 0; i < (1 << D); ++i) raw[i] = tex1Dfetch<Raw>((cudaTextureObject_t)g.tex, off + (int)idx[i]);
+    } else {
+      const Raw* at = reinterpret_cast<const Raw*>(table) + g.offset[l];
+#pragma unroll
+      for (int i = 0; i < (1 << D); ++i) raw[i] = __ldg(at + idx[i]);
+    }
+  }
+
+  // The level's F features (fused multiply-adds over the corners in order).
+  __device__ __forceinline__ void blend(float* out) const {
+    float w01[4], wt[D][2];
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      wt[k][0] = 1.f - f[k];
+      wt[k][1] = f[k];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) w01[q] = wt[0][q & 1] * wt[1][q >> 1];
+    float acc[F];
+#pragma unroll
+    for (int k = 0; k < F; ++k) acc[k] = 0.f;
+#pragma unroll
+    for (int i = 0; i < (1 << D); ++i) {
+      float w = w01[i & 3];
+#pragma unroll
+      for (int k = 2; k < D; ++k) w = w * wt[k][(i >> k) & 1];
+      if constexpr (F == 2) {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&raw[i]));
+        acc[0] = fmaf(w, v.x, acc[0]);
+        acc[1] = fmaf(w, v.y, acc[1]);
+      } else {
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw[i].x));
+        const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&raw[i].y));
+        acc[0] = fmaf(w, a.x, acc[0]);
+        acc[1] = fmaf(w, a.y, acc[1]);
+        acc[2] = fmaf(w, b.x, acc[2]);
+        acc[3] = fmaf(w, b.y, acc[3]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < F; ++k) out[k] = acc[k];
+  }
+};
+
 // Encodes one sample into row r of the swizzled X tiles (bf16), 8 features
 // (one 16-byte chunk) at a time, the padding after the last level zero;
-// invalid samples write zeros.  With xdst the row is also written there
-// (evict-first: the store streams past the L2 that holds the tables).
+// invalid samples write zeros.  The
+// corners of two levels of 2 features are fetched before the first is blended (four
+// spill at 80 registers: 512 x 512 rays x 512 samples 38.1 ms a step, two 37.7, one
+// 38.4), one level of 4 features (two spill in the deep model).
 template <int D, int F, int L>
 __device__ __forceinline__ void encode_row(const GridDev& g, const __half* __restrict__ table, const float* p,
-                                           bool valid, uint8_t* sX, int r, uint4* __restrict__ xdst = nullptr) {
+                                           bool valid, uint8_t* sX, int r) {
   using S = InShape<L, F>;
   constexpr int LPC = 8 / F;  // levels per 16-byte chunk
+  constexpr int kGroup = F == 2 ? 2 : 1;   // levels in flight
 #pragma unroll 1
   for (int j = 0; j < S::NCH; ++j) {
     float v[8];
@@ -118,49 +223,44 @@ __device__ __forceinline__ void encode_row(const GridDev& g, const __half* __res
     for (int q = 0; q < 8; ++q) v[q] = 0.f;
     if (valid) {
 #pragma unroll
-      for (int q = 0; q < LPC; ++q) {
-        const int l = j * LPC + q;
-        if (L % LPC != 0 && l >= L) break;   // the padding chunk after an odd last level
-        LevelCorners<D> lc;
-        level_corners<D>(g, l, p, lc);
-        float vals[1 << D][F];
-        // the odd hashed levels' corners through the texture path (a second
-        // L1 data pipe beside the load/store unit's), the others as loads
-        if (g.tex && ((g.hashed_bits >> l) & 1u) && (l & 1)) {
+      for (int q = 0; q < LPC; q += kGroup) {
+        LevelFetch<D, F> lv[kGroup];
 #pragma unroll
-          for (int c = 0; c < (1 << D); ++c) {
-            const int e = (int)(g.offset[l] + lc.idx[c]);
-            if constexpr (F == 2) {
-              const unsigned int raw = tex1Dfetch<unsigned int>((cudaTextureObject_t)g.tex, e);
-              const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&raw));
-              vals[c][0] = v.x;
-              vals[c][1] = v.y;
-            } else {
-              const uint2 raw = tex1Dfetch<uint2>((cudaTextureObject_t)g.tex, e);
-              const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
-              const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-              vals[c][0] = a.x;
-              vals[c][1] = a.y;
-              vals[c][2] = b.x;
-              vals[c][3] = b.y;
-            }
-          }
-        } else
+        for (int k = 0; k < kGroup; ++k) {
+          const int l = j * LPC + q + k;
+          if (L % LPC == 0 || l < L) lv[k].load(g, table, l, p);
+        }
 #pragma unroll
-        for (int c = 0; c < (1 << D); ++c) Feat<F, __half>::load(table, g.offset[l] + lc.idx[c], vals[c]);
-#pragma unroll
-        for (int f = 0; f < F; ++f) {
-          float acc = 0.f;
-#pragma unroll
-          for (int c = 0; c < (1 << D); ++c) acc = fmaf(lc.w[c], vals[c][f], acc);
-          v[q * F + f] = acc;
+        for (int k = 0; k < kGroup; ++k) {
+          const int l = j * LPC + q + k;   // (an odd last level leaves a chunk's second half zero)
+          if (L % LPC == 0 || l < L) lv[k].blend(v + (q + k) * F);
         }
       }
     }
-    const uint4 packed = tc::pack_bf16x8(v);
-    tc::st_chunk_raw(sX + (j / 8) * kTile, r, j % 8, packed);
-    if (xdst) __stcs(xdst + j, packed);
+    tc::st_chunk_bf16(sX + (j / 8) * kTile, r, j % 8, v);
   }
+}
+
+// Copies the warp's 32 encoded rows (rows row0.. of the X tiles) to the encoding
+// store, lane r's to row `to` of it (none: kNoRow), evict-first: the store streams
+// past the L2 that holds the tables.  Consecutive lanes write consecutive chunks
+// of a row: whole sectors, where a lane writing its own row fills half a sector
+// at a time.
+constexpr uint32_t kNoRow = 0xffffffffu;
+template <int L, int F>
+__device__ __forceinline__ void store_rows(const uint8_t* sX, int row0, uint32_t to, uint4* __restrict__ xstore) {
+  constexpr int NCH = InShape<L, F>::NCH;
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < NCH; ++k) {
+    const int e = 32 * k + lane, row = e / NCH, j = e % NCH;
+    const uint32_t dst = __shfl_sync(0xffffffffu, to, row);
+    if (dst != kNoRow)
+      __stcs(xstore + (size_t)dst * NCH + j,
+             *reinterpret_cast<const uint4*>(sX + (j / 8) * kTile + tc::sw128(row0 + row, j % 8)));
+  }
+  __syncwarp();
 }
 
 // Loads 64 fp32 TMEM columns [col, col+64) of this thread's lane.

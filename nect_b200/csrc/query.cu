@@ -448,6 +448,15 @@ int reproject_range(const NectbGeometry* geometry, const NectbHashGrid* grid, co
   a.loss_scale = 0.f;
   a.max_blocks = max_blocks;
   a.fwd_warpgroups = max_blocks > 0 ? 0 : warpgroups;
+  a.n_cols = geometry->nDetector[1];
+  // a whole view with room past the base size: the column form's sigmas, whole strips at a time
+  const size_t base = align256(workspace_bytes(count, count));
+  const int64_t strip = 32 * (int64_t)a.n_cols;
+  if (!stage && max_blocks <= 0 && workspace_size > base) {
+    const int64_t fit = (int64_t)((workspace_size - base) / ((size_t)num_points_per_ray * sizeof(float)));
+    a.col_rays = (int)std::min<int64_t>(fit / strip * strip, ceil_div(count, strip) * strip);
+    if (a.col_rays > 0) a.col_sigma = reinterpret_cast<float*>(static_cast<char*>(workspace) + base);
+  }
   Workspace ws = carve_workspace(workspace, count, count, stage ? workspace_size : 0);
   float* y = out + begin;
   float* loss = reinterpret_cast<float*>(ws.counters + 8);

@@ -51,6 +51,10 @@ struct TrainArgs {
   // > 0: the forward runs one block of this many warpgroups per SM under the
   // shared-SM carveout (re-projection pieces beside serving kernels); 0: the tuning's
   int fwd_warpgroups = 0;
+  // Re-projections: room for the column form's sigmas, of col_rays rays (whole
+  // strips of 32 detector rows) at a time; null: none.
+  float* col_sigma = nullptr;
+  int col_rays = 0;
   // the encoders may fetch corners through a texture object over the table
   // (false: loads only, no texture object created)
   bool texture = true;
@@ -306,6 +310,17 @@ __device__ __forceinline__ int next_ray(unsigned int* cursor, const int32_t* __r
       if (recs[idx].count > 0) return (int)idx;
     }
   }
+}
+
+// Slot of scheduling index idx: the detector in strips of 32 rows, a strip
+// column by column, so that 32 consecutive rays are vertical neighbours.
+// Their paths differ along axis 0 only (the rotation axis), whose vertices
+// share sectors of the tables.
+__device__ __forceinline__ int strip_slot(int idx, int P, int cols, int sub) {
+  const int rows = P / (cols * sub), strip = idx / (32 * cols * sub);
+  const int h = min(32, rows - 32 * strip), rem = idx - strip * 32 * cols * sub;
+  const int cj = rem / h, row = 32 * strip + rem - cj * h;   // cj = column * sub + sub-angle
+  return row * cols * sub + cj;
 }
 
 // The rays with samples in scheduling order, for the two-pass backward's

@@ -43,6 +43,7 @@ constexpr int kMixThreads = 128;
 // 2.55 / 2.67 ms (before the passes became one launch).
 constexpr int kScatterThreads = 128;
 constexpr int kScatterSegment = 32;
+constexpr int kColumnSegment = 32;   // samples of a column unit of the forward
 #ifndef UNR
 #define UNR 1
 #endif
@@ -115,13 +116,80 @@ struct FwdShape {
       (D == 3 && H == 2) ? kFwdBlocksPerSM : (kFwdBlocksPerSM < 4 ? kFwdBlocksPerSM : 4);
 };
 
-template <int D, int F, int L, int H, int ACT>
+// The forward has two forms.  Rows: a warp takes 32 consecutive samples of one ray.
+// Columns: a warp takes sample i of 32 vertically neighbouring rays (strip_slot).
+// Those lie along axis 0, whose vertices follow each other in memory, so a warp's
+// gathers touch a few lines of a hashed level where a row's touch 32: the row form
+// is bound by the L1's lines and the L2's sectors, the column form by instruction
+// issue (72 %, L1 50 %, L2 requests 38 %).
+// What the column form works on: the rays [lo, hi) of the
+// order (or of the strips' slots), in groups of 32, and where sigma goes.
+struct Columns {
+  int lo = 0, hi = 0;
+  float* sigma = nullptr;   // [(rank - lo) / 32][S][32]
+};
+// A sample that the ray's sum leaves out (the zero point).
+constexpr unsigned int kNoSample = 0x7fffdeadu;
+
+// A lane's place in the column form: one of 32 vertically neighbouring rays,
+// the warp at sample i of all of them.
+struct ColumnCursor {
+  int i = 0, end = 0;     // the warp's current and last sample (exclusive)
+  int64_t xrow = -1;      // as RayCursor
+  int64_t out = 0;        // index of the lane's sigma of sample 0
+  RayRec rec;
+};
+
+// Moves the warp to its next sample, or to its next unit (32 rays x
+// kColumnSegment samples); false when there is none left.
+__device__ __forceinline__ bool next_column(ColumnCursor& cur, const RayRec* recs, unsigned int* cursor,
+                                            const int32_t* slot, const TrainArgs& a, const Columns& c,
+                                            const int32_t* order, const uint64_t* offs, unsigned int n_valid,
+                                            uint32_t xcap, int lane) {
+  if (cur.i + 1 < cur.end) {
+    ++cur.i;
+    return true;
+  }
+  const int segs = (a.S + kColumnSegment - 1) / kColumnSegment;
+  const int hi = order ? min(c.hi, (int)n_valid) : c.hi;
+  while (true) {
+    unsigned int u = 0;
+    if (lane == 0) u = atomicAdd(cursor, 1u);
+    u = __shfl_sync(0xffffffffu, u, 0);
+    const int group = (int)(u / (unsigned)segs);
+    if (c.lo + group * 32 >= hi) {
+      cur.i = cur.end = 0;
+      cur.rec.count = 0;
+      return false;
+    }
+    const int rank = c.lo + group * 32 + lane;
+    int ray = -1;
+    if (rank < hi) ray = order ? order[rank] : slot[strip_slot(rank, a.n_pixels, a.n_cols, a.sub)];
+    if (ray >= 0)
+      cur.rec = load_ray(recs, ray);
+    else
+      cur.rec.count = 0;
+    const int first = (int)(u % (unsigned)segs) * kColumnSegment;
+    cur.i = first;
+    cur.end = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(0, min(first + kColumnSegment, cur.rec.count)));
+    if (first >= cur.end) continue;
+    cur.xrow = -1;
+    if (ray >= 0 && offs) {
+      const uint64_t o = offs[rank];
+      if (o + (uint64_t)cur.rec.count <= (uint64_t)xcap) cur.xrow = (int64_t)o;
+    }
+    cur.out = (int64_t)group * a.S * 32 + lane;
+    return true;
+  }
+}
+
+template <int D, int F, int L, int H, int ACT, bool kColumns>
 __global__ void __launch_bounds__(FwdShape<D, L, F, H>::kMaxWarpgroups * kMixThreads, 1)
 fwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __restrict__ W, TrainArgs a,
                  RayRec* __restrict__ recs, const int32_t* __restrict__ slot, unsigned int* __restrict__ ctrl,
                  int out_act, float* __restrict__ y_pred, float* __restrict__ loss,
                  const int32_t* __restrict__ order, const uint64_t* __restrict__ offs, uint4* __restrict__ xstore,
-                 uint32_t xcap) {
+                 uint32_t xcap, Columns cols) {
   using S = InShape<L, F>;
   constexpr int KT = S::KT;
   constexpr int act = ACT;  // hidden activation, a compile-time constant of the hot loops
@@ -165,19 +233,27 @@ fwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
   uint32_t phase = 0;
   float loss_acc = 0.f;
   float ksum = 0.f, kcomp = 0.f;  // Kahan sum of sigma along the warp's current ray (per lane)
-  RayCursor cur;
+  using Cursor = std::conditional_t<kColumns, ColumnCursor, RayCursor>;
+  Cursor cur;
+  if constexpr (kColumns) cur.rec.count = 0;
   bool timed_out = false;
   while (true) {
-    const bool active =
-        next_chunk(cur, recs, ctrl, slot, a, by_pixel, lane, 0, 0x7fffffff, order, n_valid, offs, xcap);
+    bool active;
+    int i;
+    if constexpr (kColumns) {
+      active = next_column(cur, recs, ctrl, slot, a, cols, order, offs, n_valid, xcap, lane);
+      i = cur.i;
+    } else {
+      active = next_chunk(cur, recs, ctrl, slot, a, by_pixel, lane, 0, 0x7fffffff, order, n_valid, offs, xcap);
+      i = cur.base + lane;
+    }
     if (!wg_or(wg, active)) break;
-    const int i = cur.base + lane;
     float p[4] = {0.f, 0.f, 0.f, 0.f};
     bool valid = false;
     if (active && i < cur.rec.count) valid = sample_point(cur.rec, i, p);
     if (D == 4) p[3] = a.t;
-    encode_row<D, F, L>(grid, table, p, valid, sX, r,
-                        valid && cur.xrow >= 0 ? xstore + (size_t)(cur.xrow + i) * S::NCH : nullptr);
+    encode_row<D, F, L>(grid, table, p, valid, sX, r);
+    const uint32_t to = valid && cur.xrow >= 0 ? (uint32_t)(cur.xrow + i) : kNoRow;
     // layer k (0-based) writes the warpgroup's 64 TMEM columns; its input is
     // X for k = 0, else the previous layer's activations in sA (which
     // overwrite X once layer 0's MMA has completed)
@@ -201,6 +277,8 @@ fwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
         }
         tc::commit(bar);
       }
+      // beside the first product, which reads the same rows
+      if (k == 0 && xstore) store_rows<L, F>(sX, r & ~31, to, xstore);
       timed_out = !tc::mbar_wait(bar, phase);
       phase ^= 1;
       if (wg_or(wg, timed_out)) {
@@ -231,25 +309,31 @@ fwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
       }
     }
     if (timed_out) break;
-    if (valid) {  // Kahan-compensated accumulation along the ray
-      const float y = act_fwd(z, out_act) - kcomp;
-      const float s = ksum + y;
-      kcomp = (s - ksum) - y;
-      ksum = s;
-    }
-    tc::fence_before();
-    if (active) {
-      cur.base += 32;
-      if (cur.base >= cur.rec.count) {
-        const float sum = warp_sum(ksum);
-        if (lane == 0) {
-          const float yp = sum * cur.rec.scale;
-          y_pred[cur.ray] = yp;
-          recs[cur.ray].gsig = loss_grad(yp, cur.rec.y, a.loss_type, a.num_rays, cur.rec.scale) * a.loss_scale;
-          loss_acc += loss_term(yp, cur.rec.y, a.loss_type);
+    if constexpr (kColumns) {
+      if (active && i < cur.rec.count)
+        cols.sigma[cur.out + (int64_t)i * 32] = valid ? act_fwd(z, out_act) : __uint_as_float(kNoSample);
+      tc::fence_before();
+    } else {
+      if (valid) {  // Kahan-compensated accumulation along the ray
+        const float y = act_fwd(z, out_act) - kcomp;
+        const float s = ksum + y;
+        kcomp = (s - ksum) - y;
+        ksum = s;
+      }
+      tc::fence_before();
+      if (active) {
+        cur.base += 32;
+        if (cur.base >= cur.rec.count) {
+          const float sum = warp_sum(ksum);
+          if (lane == 0) {
+            const float yp = sum * cur.rec.scale;
+            y_pred[cur.ray] = yp;
+            recs[cur.ray].gsig = loss_grad(yp, cur.rec.y, a.loss_type, a.num_rays, cur.rec.scale) * a.loss_scale;
+            loss_acc += loss_term(yp, cur.rec.y, a.loss_type);
+          }
+          ksum = 0.f;
+          kcomp = 0.f;
         }
-        ksum = 0.f;
-        kcomp = 0.f;
       }
     }
   }
@@ -257,7 +341,7 @@ fwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
   if (lane == 0) red[warp] = loss_acc;
   tc::fence_before();
   __syncthreads();
-  if (t == 0) {
+  if (!kColumns && t == 0) {
     float sum = 0.f;
     for (int w = 0; w < (int)(blockDim.x / 32); ++w) sum += red[w];
     atomicAdd(loss, sum / (float)a.num_rays);
@@ -266,6 +350,75 @@ fwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
     tc::fence_after();
     tc::tmem_dealloc(*tslot, ncols);
   }
+}
+
+// The line integrals of the column form, summed in the order of the other form (32
+// compensated partial sums, sample i in sum i mod 32, then the warp's tree), so
+// that both give the same bits: a block takes 32 rays, a warp four of them, lane l
+// the samples l mod 32; tiles of 32 samples x 32 rays turn in shared memory.
+constexpr int kColumnSumWarps = 8;
+__global__ void __launch_bounds__(kColumnSumWarps * 32)
+column_sum_kernel(TrainArgs a, RayRec* __restrict__ recs, const int32_t* __restrict__ slot,
+                  const unsigned int* __restrict__ ctrl, const int32_t* __restrict__ order, Columns c,
+                  float* __restrict__ y_pred, float* __restrict__ loss) {
+  constexpr int PER = 32 / kColumnSumWarps;
+  __shared__ float tile[32][33];
+  __shared__ int rays[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int hi = order ? min(c.hi, (int)ctrl[6]) : c.hi;
+  int longest = 0;
+  {   // every warp finds the group's rays and their longest count
+    const int rank = c.lo + (int)blockIdx.x * 32 + lane;
+    int ray = -1;
+    if (rank < hi) ray = order ? order[rank] : slot[strip_slot(rank, a.n_pixels, a.n_cols, a.sub)];
+    if (warp == 0) rays[lane] = ray;
+    longest = (int)__reduce_max_sync(0xffffffffu, ray >= 0 ? (unsigned)recs[ray].count : 0u);
+  }
+  __syncthreads();
+  int ray[PER], count[PER];
+  float sum[PER], comp[PER];
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    ray[q] = rays[warp * PER + q];
+    count[q] = ray[q] >= 0 ? recs[ray[q]].count : 0;
+    sum[q] = comp[q] = 0.f;
+  }
+  const float* src = c.sigma + (int64_t)blockIdx.x * a.S * 32;
+  for (int i0 = 0; i0 < longest; i0 += 32) {   // block-uniform
+    float v[PER];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      const int i = i0 + warp * PER + q;
+      v[q] = i < longest ? __ldcs(src + (int64_t)i * 32 + lane) : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < PER; ++q) tile[warp * PER + q][lane] = v[q];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      const float s = tile[lane][warp * PER + q];
+      if (i0 + lane < count[q] && __float_as_uint(s) != kNoSample) {
+        const float y = s - comp[q];
+        const float n = sum[q] + y;
+        comp[q] = (n - sum[q]) - y;
+        sum[q] = n;
+      }
+    }
+  }
+  float term = 0.f;
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const float total = warp_sum(sum[q]);
+    if (lane == 0 && ray[q] >= 0) {
+      const RayRec& rec = recs[ray[q]];
+      const float yp = total * rec.scale;
+      y_pred[ray[q]] = yp;
+      recs[ray[q]].gsig = loss_grad(yp, rec.y, a.loss_type, a.num_rays, rec.scale) * a.loss_scale;
+      term += loss_term(yp, rec.y, a.loss_type);
+    }
+  }
+  if (lane == 0) atomicAdd(loss, term / (float)a.num_rays);
 }
 
 // Staged mode (kStaged): instead of scattering, dL/d(encoding) of every sample
@@ -1111,16 +1264,51 @@ int run_mixed(const NectbGeometry& geo, const GridDev& grid, const __half* table
     // with an encoding store the forward runs the rays in rank order and keeps their rows
     if (SL.xstore)
       if (int rc = run_order()) return rc;
-    auto k = fwd_mixed_kernel<D, F, L, H, ACT>;
     const size_t smem = 1024 + (KT + H - 1) * kWTile + wgs * KT * kTile + 64 * 4 + kFwdBlocksPerSM * 8 + 16 +
                         4 * kFwdBlocksPerSM * 4;
-    set_smem(k, smem, shares_sms);
-    {
+    const int32_t* order_arg = SL.xstore ? SL.order : nullptr;
+    auto run = [&](auto columns, const Columns& cols) -> int {
+      auto k = fwd_mixed_kernel<D, F, L, H, ACT, columns()>;
+      set_smem(k, smem, shares_sms);
       ProfScope ps(kProfForward, s);
       k<<<fblocks, kMixThreads * wgs, smem, s>>>(gt, table, W, a, ws.rays, ws.slot, ws.counters, out_act, y_pred, loss,
-                                           SL.xstore ? SL.order : nullptr, SL.offs, SL.xstore, SL.xcap);
+                                                 order_arg, SL.offs, SL.xstore, SL.xcap, cols);
+      if (columns())
+        column_sum_kernel<<<(unsigned)ceil_div(cols.hi - cols.lo, 32), kColumnSumWarps * 32, 0, s>>>(
+            a, ws.rays, ws.slot, ws.counters, order_arg, cols, y_pred, loss);
+      return launch_status("fwd_mixed_kernel");
+    };
+    // The column form needs neighbouring rays in a warp, so a share of the
+    // detector's pixels in the batch, and units enough for the warps.  A line of
+    // the table holds 32 entries of 2 features, 16 of 4.  Step (training) or view
+    // with the one / the other form, 512 x 512 detector and 512 samples unless
+    // stated: 2 features, all pixels 37.3 / 40.0 ms, a half 20.3 / 21.9, an eighth
+    // 6.20 / 6.37, a sixteenth 4.07 / 3.77; 4D view 14.9 / 23.5, 128 x 128 x 256 (1.7
+    // units a warp) 0.83 / 1.03, 64 x 64 x 64 (0.1) 0.52 / 0.14.  4 features, 256 x
+    // 256 x 256: all pixels 15.8 / 16.3, a half 8.76 / 8.72, a quarter 5.20 / 4.86; 128
+    // x 128 x 512 (3.5 units) 8.07 / 7.80.
+    const int64_t units = ceil_div(R, 32) * ceil_div(a.S, kColumnSegment), warps = (int64_t)fblocks * wgs * 4;
+    const bool columns = F == 2 ? 2 * units >= 3 * warps && 5 * (int64_t)R >= a.n_pixels
+                                : units >= 4 * warps && 2 * (int64_t)R > a.n_pixels;
+    const size_t sigma_bytes = (size_t)ceil_div(R, 32) * 32 * a.S * sizeof(float);
+    Columns cols;
+    if (columns && a.col_sigma) {   // a re-projection, strips at a time
+      for (int lo = 0; lo < R; lo += a.col_rays) {
+        if (lo > 0)
+          if (int rc = cuda_status(cudaMemsetAsync(ws.counters, 0, sizeof(unsigned int), s), "memset cursor")) return rc;
+        cols.lo = lo;
+        cols.hi = std::min(R, lo + a.col_rays);
+        cols.sigma = a.col_sigma;
+        if (int rc = run(std::true_type{}, cols)) return rc;
+      }
+    } else if (columns && SL.xstore && SL.per_round > 0 && !shares_sms &&
+               sigma_bytes <= (size_t)SL.per_round * ray_slots(a.S) * IN * sizeof(float)) {
+      cols.hi = R;   // sigma in the staging buffer, which the backward fills later
+      cols.sigma = SL.stage;
+      if (int rc = run(std::true_type{}, cols)) return rc;
+    } else {
+      if (int rc = run(std::false_type{}, cols)) return rc;
     }
-    if (int rc = launch_status("fwd_mixed_kernel")) return rc;
   }
   if (!table_grad || !(a.phase & kPhaseBackward)) return NECTB_OK;  // forward only (queries, split step)
   // at least 80 KB keeps at most two blocks (2 x 256 TMEM columns) per SM;

@@ -79,17 +79,6 @@ __global__ void ray_prep_kernel(NectbGeometry g, TrainArgs a, RayRec* __restrict
   }
 }
 
-// Slot of scheduling index idx: the detector in strips of 32 rows, a strip
-// column by column, so that 32 consecutive rays are vertical neighbours.
-// Their paths differ along axis 0 only (the rotation axis), whose vertices
-// share sectors of the tables.
-__device__ __forceinline__ int strip_slot(int idx, int P, int cols, int sub) {
-  const int rows = P / (cols * sub), strip = idx / (32 * cols * sub);
-  const int h = min(32, rows - 32 * strip), rem = idx - strip * 32 * cols * sub;
-  const int cj = rem / h, row = 32 * strip + rem - cj * h;   // cj = column * sub + sub-angle
-  return row * cols * sub + cj;
-}
-
 __device__ __forceinline__ bool ordered_valid(const int32_t* __restrict__ slot, const RayRec* __restrict__ recs,
                                               bool by_pixel, int idx, int n, int cols, int sub, int* ray) {
   if (idx >= n) return false;

@@ -40,6 +40,7 @@ from . import _lib
 from .network import _HashGridModel
 
 CHUNK = 128
+VIEW_SIGMA_BYTES = 256 << 20   # of a re-projection's own workspace, for the forward's column form
 
 ITEM_DTYPE = np.dtype({
     "names": ["origin", "du", "dv", "nu", "nv", "t", "out_scale", "out_offset", "out", "out_stride", "chunk_begin"],
@@ -198,6 +199,13 @@ def reproject(model: _HashGridModel, geometry, angle: float, t: float = 0.0, poi
     if pixels is None and not warpgroups:
         need = _lib.lib.nectb_train_workspace_bytes(ctypes.byref(cg.c_struct), ctypes.byref(model.grid_desc),
                                                     ctypes.byref(model.mlp_desc), P)
+        if workspace is None:
+            # with room for the sigmas of some strips of 32 detector rows, a mixed model's view runs
+            # them column by column (at most VIEW_SIGMA_BYTES; results do not depend on it)
+            strip = 4 * 32 * geometry.nDetector[1] * S
+            rows = -(-geometry.nDetector[0] // 32)
+            if model.precision == "mixed" and max_blocks == 0:
+                need = (need + 255) // 256 * 256 + min(rows, max(VIEW_SIGMA_BYTES // strip, 1)) * strip
         if workspace is None or workspace.numel() < need:
             workspace = torch.empty(need, dtype=torch.uint8, device=dev)
         rc = _lib.lib.nectb_query_reproject(ctypes.byref(cg.c_struct), ctypes.byref(model.grid_desc),
