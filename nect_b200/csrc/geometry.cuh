@@ -317,7 +317,35 @@ __device__ __forceinline__ bool ray_lookup(const int64_t* perm, int64_t perm_len
 
 // Warp-cooperative count of written samples: the first i in [0,S) at which
 // the reference loop breaks (S when it never does).  All 32 lanes must call.
+//
+// In the voxel geometries every test is monotone in i (the fp64 position, its fp32
+// rounding and the eps step are monotone roundings of a linear function), so the
+// break is looked for around the index where the ray leaves its bounds: a window of
+// 32 samples that starts unbroken and ends broken holds it.  Otherwise, and for the
+// cylinder (whose z test is not monotone), the samples are scanned from 0.
 __device__ __forceinline__ int warp_sample_count(const NectbGeometry& g, const RaySetup& r, int S, int lane) {
+  if (S > 32 && (g.kind == NECTB_CONE_VOXEL || g.kind == NECTB_PARALLEL_VOXEL)) {
+    float last = (float)S;   // about the last unbroken index
+    const double start[3] = {r.start.x, r.start.y, r.start.z}, end[3] = {r.end.x, r.end.y, r.end.z};
+    const double step[3] = {r.step.x, r.step.y, r.step.z};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float d = (float)(end[k] - start[k]), s = (float)step[k];
+      if (s != 0.f) last = fminf(last, __fdividef(d + copysignf(1e-5f, s), s));
+    }
+    const int w0 = last > 16.f ? min((int)last, S) - 16 : 0;
+    const int i = w0 + lane;
+    bool ok = true;
+    if (i < S) {
+      float a, b, c;
+      ok = sample_at(g, r, i, a, b, c);
+    }
+    const unsigned fail = __ballot_sync(0xffffffffu, !ok);
+    if (!(fail & 1u) || w0 == 0) {
+      if (fail) return w0 + __ffs(fail) - 1;
+      if (w0 + 32 >= S) return S;
+    }
+  }
   for (int base = 0; base < S; base += 32) {
     int i = base + lane;
     bool ok = true;

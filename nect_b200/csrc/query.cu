@@ -464,7 +464,7 @@ int reproject_range(const NectbGeometry* geometry, const NectbHashGrid* grid, co
   if (int rc = cuda_status(cudaMemsetAsync(ws.slot, 0xFF, (size_t)count * 4, s), "memset slots")) return rc;
   {
     ProfScope ps(kProfRayPrep, s);
-    ray_prep_kernel<<<(unsigned)ceil_div(count, 8), 256, 0, s>>>(*geometry, a, ws.rays, ws.slot, ws.counters, y,
+    ray_prep_kernel<<<(unsigned)ceil_div(count, kRayPrepThreads / 32), kRayPrepThreads, 0, s>>>(*geometry, a, ws.rays, ws.slot, ws.counters, y,
                                                                   loss);
   }
   if (int rc = launch_status("ray_prep_kernel")) return rc;

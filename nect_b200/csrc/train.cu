@@ -267,7 +267,7 @@ int train_entry(const NectbGeometry* geometry, const NectbHashGrid* grid, const 
     if (int rc = cuda_status(cudaMemsetAsync(ws.counters, 0, 64, s), "memset counters")) return rc;
     if (int rc = cuda_status(cudaMemsetAsync(ws.slot, 0xFF, (size_t)a.n_pixels * 4, s), "memset slots")) return rc;
     ProfScope ps(kProfRayPrep, s);
-    ray_prep_kernel<<<(unsigned)ceil_div(a.num_rays, 8), 256, 0, s>>>(*geometry, a, ws.rays, ws.slot, ws.counters,
+    ray_prep_kernel<<<(unsigned)ceil_div(a.num_rays, kRayPrepThreads / 32), kRayPrepThreads, 0, s>>>(*geometry, a, ws.rays, ws.slot, ws.counters,
                                                                        fwd_y, fwd_loss);
   } else {
     // backward half: fresh backward cursor, the caller's loss gradient per ray

@@ -268,6 +268,7 @@ inline size_t slice_half_bytes(const GridDev& g) {
 // Warp per ray: set-up, sample count (warp ballot), measured value, scale;
 // claims the ray's detector pixel in slot[]; finalises rays without samples
 // (y_pred = 0, their loss term and gradient).
+constexpr int kRayPrepThreads = 256;
 __global__ void ray_prep_kernel(NectbGeometry g, TrainArgs a, RayRec* __restrict__ recs, int32_t* __restrict__ slot,
                                 unsigned int* __restrict__ ctrl, float* __restrict__ y_pred, float* __restrict__ loss);
 

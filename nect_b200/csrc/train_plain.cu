@@ -22,34 +22,50 @@ namespace nectb {
 __global__ void ray_prep_kernel(NectbGeometry g, TrainArgs a, RayRec* __restrict__ recs, int32_t* __restrict__ slot,
                                 unsigned int* __restrict__ ctrl, float* __restrict__ y_pred, float* __restrict__ loss) {
   const int lane = threadIdx.x & 31;
-  const int tid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (tid >= a.num_rays) return;
-  int ray_index = 0;
-  RaySetup r;
-  r.valid = 0;
-  r.distance = 0.f;
-  // continuous scan: virtual ray tid is pixel rb of the batch at sub-angle j
+  // The block's eight rays are set up by eight lanes: the fp64 divisions once per
+  // ray instead of on every lane of its warp (512 x 512 rays: 422 -> 229 us, 138 of
+  // that from the windowed count).
+  constexpr int kRays = kRayPrepThreads / 32;
+  __shared__ RaySetup setups[kRays];
+  __shared__ int indices[kRays], slots[kRays];   // detector pixel (-1: outside the batch), scheduling slot
   const int n_batch = a.num_rays / a.sub;
-  const int j = tid / n_batch, rb = tid - j * n_batch;
-  const float angle = a.sub > 1 ? a.sub_angle[j] : a.angle;
-  // perm == nullptr: the detector pixels start, start + 1, ... in order
-  // (re-projection queries, whole views or pieces of them; the slots are
-  // indexed from the first pixel); jitter / detector offsets default to 0
-  // when absent.
-  bool ok;
-  int sidx;  // scheduling slot of the ray's pixel
-  if (a.perm) {
-    ok = ray_lookup(a.perm, a.perm_len, a.start, rb, n_batch, g, ray_index);
-    sidx = ray_index;
-  } else {
-    ray_index = (int)a.start + tid;
-    ok = tid < a.n_pixels;
-    sidx = tid;
+  if (threadIdx.x < kRays) {
+    const int v = blockIdx.x * kRays + threadIdx.x;
+    RaySetup s;
+    s.valid = 0;
+    s.distance = 0.f;
+    int ray_index = 0, sidx = 0;
+    bool ok = false;
+    if (v < a.num_rays) {
+      // continuous scan: virtual ray v is pixel rb of the batch at sub-angle j
+      const int j = v / n_batch, rb = v - j * n_batch;
+      const float angle = a.sub > 1 ? a.sub_angle[j] : a.angle;
+      // perm == nullptr: the detector pixels start, start + 1, ... in order
+      // (re-projection queries, whole views or pieces of them; the slots are
+      // indexed from the first pixel); jitter / detector offsets default to 0
+      // when absent.
+      if (a.perm) {
+        ok = ray_lookup(a.perm, a.perm_len, a.start, rb, n_batch, g, ray_index);
+        sidx = ray_index;
+      } else {
+        ray_index = (int)a.start + v;
+        ok = v < a.n_pixels;
+        sidx = v;
+      }
+      if (ok)
+        ray_setup(g, ray_index, a.det_off ? a.det_off[2 * (int64_t)v] : 0.f,
+                  a.det_off ? a.det_off[2 * (int64_t)v + 1] : 0.f, a.jitter ? a.jitter[v] : 0.f, angle, a.S, a.maxd,
+                  a.uniform != 0, s);
+    }
+    setups[threadIdx.x] = s;
+    indices[threadIdx.x] = ok && ray_index >= 0 ? ray_index : -1;
+    slots[threadIdx.x] = sidx;
   }
-  if (ok)
-    ray_setup(g, ray_index, a.det_off ? a.det_off[2 * (int64_t)tid] : 0.f,
-              a.det_off ? a.det_off[2 * (int64_t)tid + 1] : 0.f, a.jitter ? a.jitter[tid] : 0.f, angle, a.S,
-              a.maxd, a.uniform != 0, r);
+  __syncthreads();
+  const int tid = blockIdx.x * kRays + (threadIdx.x >> 5);
+  if (tid >= a.num_rays) return;
+  const RaySetup r = setups[threadIdx.x >> 5];
+  const int ray_index = indices[threadIdx.x >> 5], sidx = slots[threadIdx.x >> 5], j = tid / n_batch;
   int count = 0;
   if (r.valid) count = warp_sample_count(g, r, a.S, lane);
   if (lane == 0) {
@@ -64,8 +80,7 @@ __global__ void ray_prep_kernel(NectbGeometry g, TrainArgs a, RayRec* __restrict
     rec.scale = r.distance / a.max_dist;
     // proj[perm[start:start+R]] (projector.py:130); rays past the end of the
     // permutation are not part of the reference batch and get y = 0 here.
-    const bool in_range = ok && ray_index >= 0;
-    rec.y = (in_range && a.projection) ? a.projection[ray_index] : 0.f;
+    rec.y = (ray_index >= 0 && a.projection) ? a.projection[ray_index] : 0.f;
     rec.gsig = 0.f;
     if (count > 0) {
       if (atomicCAS(slot + (int64_t)sidx * a.sub + j, -1, tid) != -1) atomicOr(ctrl + 3, kFlagDuplicatePixels);
