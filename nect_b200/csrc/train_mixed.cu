@@ -421,6 +421,17 @@ column_sum_kernel(TrainArgs a, RayRec* __restrict__ recs, const int32_t* __restr
   if (lane == 0) atomicAdd(loss, term / (float)a.num_rays);
 }
 
+// Tiles after which a block of the staged backward adds its weight gradients to
+// fp32 memory and starts them anew.  They gather in the tensor cores' accumulators,
+// which lose about 2e-8 of the sum per product: batches are split into `flushes`
+// stretches over the whole order (launches of R / staged_rounds rays measured the
+// same losses; three times the length 3e-5 of the gradient).
+__device__ __forceinline__ int flush_interval(const unsigned int* ctrl, float flushes) {
+  if (flushes <= 1.f) return 0x7fffffff;
+  const float tiles = (float)ctrl[9] * 0.25f;   // 32-sample chunks of the batch, four to a tile
+  return max(1, (int)ceilf(tiles / (flushes * (float)gridDim.x)));
+}
+
 // Staged mode (kStaged): instead of scattering, dL/d(encoding) of every sample
 // is written to the staging buffer, level-major: stage[(l * slots + s) * F + f]
 // with s = (scheduling index - lo) * ray_slots(S) + sample, for the rays whose
@@ -446,7 +457,7 @@ bwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
                  const RayRec* __restrict__ recs, const int32_t* __restrict__ slot, unsigned int* __restrict__ ctrl,
                  int out_act, float* __restrict__ table_grad, float* __restrict__ W_grad, int lo, int hi,
                  float* __restrict__ stage, int64_t slots, const int32_t* __restrict__ order,
-                 const uint64_t* __restrict__ offs, const uint4* __restrict__ xstore, uint32_t xcap) {
+                 const uint64_t* __restrict__ offs, const uint4* __restrict__ xstore, uint32_t xcap, float flushes) {
   using S = InShape<L, F>;
   using Plan = BwdPlan<L, F, H>;
   constexpr int IN = S::IN, KT = S::KT;
@@ -497,12 +508,46 @@ bwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
 
   uint32_t phase = 0;
   uint32_t wacc = 0;  // weight-gradient accumulators start at the first tile
+  int left = flush_interval(ctrl, flushes);   // tiles until the accumulators are added to memory
   float dwout0 = 0.f, dwout1 = 0.f;  // w_out gradient entries j0_out and j0_out + 1 of this lane
   int j0_out = 0;
   RayCursor cur;
   bool timed_out = false;
   uint4 xrow[S::NCH];    // stored rows of the current chunk (this thread's sample)
   bool pre_ok = false;   // xrow already holds them (prefetched during the previous tile)
+  // Adds the weight gradients to fp32 memory: TMEM lanes 0..63 (warps 0 and 1) hold rows o = 0..63.
+  auto flush = [&]() {
+    tc::fence_after();
+    if (warp < 2) {
+      const int o = t;
+#pragma unroll 1
+      for (int k = 1; k < H; ++k) {
+        float v[64];
+        ld64(my_lanes + Plan::T + 64 * (k - 1), v);
+        float* dst = W_grad + 64 * IN + (k - 1) * 64 * 64 + o * 64;
+#pragma unroll
+        for (int i2 = 0; i2 < 64; ++i2) atomicAdd(dst + i2, v[i2]);
+      }
+    }
+    if constexpr (KT == 1) {
+      if (warp < 2) {
+        const int o = t;
+        float w0[S::INP];
+#pragma unroll
+        for (int c = 0; c < S::INP / 16; ++c) tc::tmem_ld16(dw0 + ((uint32_t)(32 * warp) << 16) + 16 * c, w0 + 16 * c);
+        tc::tmem_wait_ld();
+#pragma unroll
+        for (int i2 = 0; i2 < IN; ++i2) atomicAdd(W_grad + o * IN + i2, w0[i2]);
+      }
+    } else if (32 * warp < IN) {  // dW0^T: lane i holds input i's 64 output columns
+      float v[64];
+      ld64(dw0 + ((uint32_t)(32 * warp) << 16), v);
+      if (t < IN) {
+#pragma unroll 8
+        for (int o = 0; o < 64; ++o) atomicAdd(W_grad + o * IN + t, v[o]);
+      }
+    }
+  };
   // Issues the MMAs of one phase (thread 0), waits for them; false on time-out.
   auto run_phase = [&](auto issue) -> bool {
     tc::fence_async_smem();
@@ -677,42 +722,19 @@ bwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
     tc::fence_before();
     __syncthreads();
     if (active) cur.base += 32;
+    if (--left == 0) {   // block-uniform
+      flush();
+      tc::fence_before();
+      __syncthreads();
+      left = flush_interval(ctrl, flushes);
+      wacc = 0;
+    }
   }
   if (timed_out) {
     if (t == 0) atomicOr(err, 2u);
     tc::mbar_wait(bar, phase);  // let the MMAs in flight retire (bounded) before freeing TMEM
   } else if (wacc) {
-    // flush the weight gradients: TMEM lanes 0..63 (warps 0 and 1) hold rows o = 0..63
-    tc::fence_after();
-    if (warp < 2) {
-      const int o = t;
-#pragma unroll 1
-      for (int k = 1; k < H; ++k) {
-        float v[64];
-        ld64(my_lanes + Plan::T + 64 * (k - 1), v);
-        float* dst = W_grad + 64 * IN + (k - 1) * 64 * 64 + o * 64;
-#pragma unroll
-        for (int i2 = 0; i2 < 64; ++i2) atomicAdd(dst + i2, v[i2]);
-      }
-    }
-    if constexpr (KT == 1) {
-      if (warp < 2) {
-        const int o = t;
-        float w0[S::INP];
-#pragma unroll
-        for (int c = 0; c < S::INP / 16; ++c) tc::tmem_ld16(dw0 + ((uint32_t)(32 * warp) << 16) + 16 * c, w0 + 16 * c);
-        tc::tmem_wait_ld();
-#pragma unroll
-        for (int i2 = 0; i2 < IN; ++i2) atomicAdd(W_grad + o * IN + i2, w0[i2]);
-      }
-    } else if (32 * warp < IN) {  // dW0^T: lane i holds input i's 64 output columns
-      float v[64];
-      ld64(dw0 + ((uint32_t)(32 * warp) << 16), v);
-      if (t < IN) {
-#pragma unroll 8
-        for (int o = 0; o < 64; ++o) atomicAdd(W_grad + o * IN + t, v[o]);
-      }
-    }
+    flush();
   }
   {
     float s0, s1;
@@ -746,13 +768,13 @@ bwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
 //   Shared memory: W0, W1 | G2 | zero block | A1, then G1 | X.
 //   Accumulator rows are read 16 columns at a time; the w_out gradient is a
 //   16-column butterfly reduce-scatter per chunk.
-template <int D, int F, int ACT>
+template <int D, int F, int ACT, bool kFlush>
 __global__ void __launch_bounds__(kMixThreads, 3)
 bwd_lean_kernel(GridDev grid, const __half* __restrict__ table, const float* __restrict__ W, TrainArgs a,
                 const RayRec* __restrict__ recs, const int32_t* __restrict__ slot, unsigned int* __restrict__ ctrl,
                 int out_act, float* __restrict__ W_grad, int lo, int hi, float* __restrict__ stage,
                 int64_t slots, const int32_t* __restrict__ order, const uint64_t* __restrict__ offs,
-                const uint4* __restrict__ xstore, uint32_t xcap) {
+                const uint4* __restrict__ xstore, uint32_t xcap, float flushes) {
   constexpr int IN = 16 * F;
   constexpr int H = 2;
   constexpr int act = ACT;
@@ -801,11 +823,31 @@ bwd_lean_kernel(GridDev grid, const __half* __restrict__ table, const float* __r
 
   uint32_t phase = 0;
   uint32_t wacc = 0;  // the first tile's dW1 product starts the accumulators
+  int left = kFlush ? flush_interval(ctrl, flushes) : 0;   // tiles until the accumulators are added to memory
   float dwacc[4] = {0.f, 0.f, 0.f, 0.f};  // w_out gradient, column 16c + (lane >> 1) of chunk c
   uint4 xn[IN / 8];                       // the stored row of this thread's sample (prefetched a tile ahead)
   bool pre_ok = false;
   RayCursor cur;
   bool timed_out = false;
+  // Adds the weight gradients to fp32 memory.
+  auto flush = [&]() {
+    tc::fence_after();
+    if (warp < 2) {  // dW1 rows o = t in lanes 0..63
+      float v[64];
+      ld64(my_lanes + 64, v);
+      float* dst = W_grad + 64 * IN + t * 64;
+#pragma unroll
+      for (int j = 0; j < 64; ++j) atomicAdd(dst + j, v[j]);
+    } else {  // dW0 rows o = t - 64 in lanes 64..127
+      float v[IN];
+#pragma unroll
+      for (int c = 0; c < IN / 16; ++c) tc::tmem_ld16(my_lanes + 64 + 16 * c, v + 16 * c);
+      tc::tmem_wait_ld();
+      float* dst = W_grad + (t - 64) * IN;
+#pragma unroll
+      for (int j = 0; j < IN; ++j) atomicAdd(dst + j, v[j]);
+    }
+  };
   auto run_phase = [&](auto issue) -> bool {
     tc::fence_async_smem();
     tc::fence_before();
@@ -981,27 +1023,19 @@ bwd_lean_kernel(GridDev grid, const __half* __restrict__ table, const float* __r
     tc::fence_before();
     __syncthreads();
     if (active) cur.base += 32;
+    if (kFlush && --left == 0) {   // block-uniform
+      flush();
+      tc::fence_before();
+      __syncthreads();
+      left = flush_interval(ctrl, flushes);
+      wacc = 0;
+    }
   }
   if (timed_out) {
     if (t == 0) atomicOr(err, 2u);
     tc::mbar_wait(bar, phase);  // let the MMAs in flight retire (bounded) before freeing TMEM
   } else if (wacc) {
-    tc::fence_after();
-    if (warp < 2) {  // dW1 rows o = t in lanes 0..63
-      float v[64];
-      ld64(my_lanes + 64, v);
-      float* dst = W_grad + 64 * IN + t * 64;
-#pragma unroll
-      for (int j = 0; j < 64; ++j) atomicAdd(dst + j, v[j]);
-    } else {  // dW0 rows o = t - 64 in lanes 64..127
-      float v[IN];
-#pragma unroll
-      for (int c = 0; c < IN / 16; ++c) tc::tmem_ld16(my_lanes + 64 + 16 * c, v + 16 * c);
-      tc::tmem_wait_ld();
-      float* dst = W_grad + (t - 64) * IN;
-#pragma unroll
-      for (int j = 0; j < IN; ++j) atomicAdd(dst + j, v[j]);
-    }
+    flush();
   }
   if (!(lane & 1)) {
 #pragma unroll
@@ -1320,7 +1354,7 @@ int run_mixed(const NectbGeometry& geo, const GridDev& grid, const __half* table
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem);
     ProfScope ps(kProfBackward, s);
     k<<<blocks, kMixThreads, bsmem, s>>>(gt, table, W, a, ws.rays, ws.slot, ws.counters, out_act, table_grad,
-                                         W_grad, 0, 0x7fffffff, nullptr, 0, nullptr, nullptr, nullptr, 0u);
+                                         W_grad, 0, 0x7fffffff, nullptr, 0, nullptr, nullptr, nullptr, 0u, 1.f);
     return launch_status("bwd_mixed_kernel");
   }
   // the order is a function of the prepared rays alone: computed again unless
@@ -1352,40 +1386,39 @@ int run_mixed(const NectbGeometry& geo, const GridDev& grid, const __half* table
   constexpr bool kLean = H == 2 && L == 16 && IN <= 64;
   const size_t lsmem = 1024 + 2 * kWTile + 3 * kTile + 2048 + 64 * 4 + 64 + 4 * 64 * 4;
   const int lblocks = std::max(1, std::min<int>(tune.backward_blocks_per_sm * sms, (int)ceil_div(a.num_rays, 4)));
-  if constexpr (kLean)
-    set_smem(bwd_lean_kernel<D, F, ACT>, lsmem, false);
-  else
+  // (the lean kernel without the adding inside: it costs 3 % in spilled registers)
+  if constexpr (kLean) {
+    set_smem(bwd_lean_kernel<D, F, ACT, true>, lsmem, false);
+    set_smem(bwd_lean_kernel<D, F, ACT, false>, lsmem, false);
+  } else
     cudaFuncSetAttribute(bwd_mixed_kernel<D, F, L, H, true, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)bsmem);
   auto ks = scatter_stage_kernel<D, F>;
   const int segs = (int)ceil_div(a.S, kScatterSegment);
   const int64_t slots = per_round * ray_slots(a.S);
-  // a round stages in launches of at most R / staged_rounds rays: the weight
-  // gradients gather in the tensor cores' accumulators for the length of a
-  // launch and in fp32 memory between launches, and the accumulators lose about
-  // 2e-8 of the sum per product (three times the launch length: 3e-5)
-  const int64_t chunk = (R + tune.staged_rounds - 1) / tune.staged_rounds;
+  // the weight gradients leave the accumulators once per R / staged_rounds rays: at
+  // a launch's end when the rounds are that small, else inside it (flush_interval)
+  const float flushes = per_round * tune.staged_rounds < 2 * (int64_t)R ? 1.f : (float)tune.staged_rounds;
   for (int64_t lo = 0; lo < R; lo += per_round) {
     const int hi = (int)std::min<int64_t>(R, lo + per_round);
-    for (int64_t c0 = lo; c0 < hi; c0 += chunk) {
-      const int c1 = (int)std::min<int64_t>(hi, c0 + chunk);
-      if (int rc = cuda_status(cudaMemsetAsync(ws.counters + 1, 0, sizeof(unsigned int), s), "memset cursor"))
-        return rc;
-      {
-        ProfScope ps(kProfBackward, s);
-        float* at = stage + (c0 - lo) * ray_slots(a.S) * F;
-        if constexpr (kLean)
-          bwd_lean_kernel<D, F, ACT><<<lblocks, kMixThreads, lsmem, s>>>(gt, table, W, a, ws.rays, ws.slot,
-                                                                         ws.counters, out_act, W_grad, (int)c0, c1,
-                                                                         at, slots, order, SL.offs, SL.xstore,
-                                                                         SL.xcap);
+    if (int rc = cuda_status(cudaMemsetAsync(ws.counters + 1, 0, sizeof(unsigned int), s), "memset cursor")) return rc;
+    {
+      ProfScope ps(kProfBackward, s);
+      if constexpr (kLean) {
+        auto lean = [&](auto k) {
+          k<<<lblocks, kMixThreads, lsmem, s>>>(gt, table, W, a, ws.rays, ws.slot, ws.counters, out_act, W_grad, (int)lo,
+                                                hi, stage, slots, order, SL.offs, SL.xstore, SL.xcap, flushes);
+        };
+        if (flushes > 1.f)
+          lean(bwd_lean_kernel<D, F, ACT, true>);
         else
-          bwd_mixed_kernel<D, F, L, H, true, ACT><<<blocks, kMixThreads, bsmem, s>>>(
-              gt, table, W, a, ws.rays, ws.slot, ws.counters, out_act, table_grad, W_grad, (int)c0, c1, at, slots,
-              order, SL.offs, SL.xstore, SL.xcap);
-      }
-      if (int rc = launch_status("bwd_mixed_kernel")) return rc;
+          lean(bwd_lean_kernel<D, F, ACT, false>);
+      } else
+        bwd_mixed_kernel<D, F, L, H, true, ACT><<<blocks, kMixThreads, bsmem, s>>>(
+            gt, table, W, a, ws.rays, ws.slot, ws.counters, out_act, table_grad, W_grad, (int)lo, hi, stage, slots,
+            order, SL.offs, SL.xstore, SL.xcap, flushes);
     }
+    if (int rc = launch_status("bwd_mixed_kernel")) return rc;
     {
       ProfScope ps(kProfScatter, s);
       const int64_t warps = ceil_div(hi - lo, 32) * segs * grid.n_levels;

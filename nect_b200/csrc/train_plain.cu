@@ -175,7 +175,10 @@ order_scan_kernel(unsigned int* __restrict__ block_sums, unsigned long long* __r
     carry64 += total64;
     __syncthreads();
   }
-  if (threadIdx.x == 0) ctrl[6] = carry;  // rays with samples
+  if (threadIdx.x == 0) {
+    ctrl[6] = carry;                        // rays with samples
+    ctrl[9] = (unsigned)(carry64 / 32 + carry / 2);   // about their chunks of 32 samples
+  }
 }
 
 __global__ void __launch_bounds__(kOrderBlock)
