@@ -271,7 +271,10 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 
 def stream_ptr(device: torch.device | None = None) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """The current stream's handle (without the Stream object: a sixth of its time, which the
+    smallest calls feel)."""
+    index = device.index if device is not None else None
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def require_cuda(t: torch.Tensor, name: str) -> None:

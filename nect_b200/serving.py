@@ -150,21 +150,27 @@ def query_points(model: _HashGridModel, items: np.ndarray, stream: torch.cuda.St
     some t) every item is evaluated on it, at its t."""
     if items.size == 0:
         return
-    stream = stream or torch.cuda.current_stream()
-    items = items.copy()
+    if stream is not None:   # the buffer belongs to the stream that reads it
+        with torch.cuda.stream(stream):
+            return query_points(model, items, None, max_blocks, slice)
     ch = item_chunks(items)
-    items["chunk_begin"] = np.concatenate([[0], np.cumsum(ch)[:-1]])
-    dev = model.table.device
-    buf = torch.empty(items.nbytes + 16, dtype=torch.uint8, device=dev)
-    with torch.cuda.stream(stream):
-        buf[items.nbytes:].zero_()   # work cursor and error word
-        buf[:items.nbytes].copy_(torch.from_numpy(items.view(np.uint8)), non_blocking=False)
-        if slice is None:
-            _call_points(model, buf.data_ptr(), items.size, int(ch.sum()), buf.data_ptr() + items.nbytes,
-                         stream.cuda_stream, max_blocks)
-        else:
-            _call_points_slice(model, slice.data_ptr(), buf.data_ptr(), items.size, int(ch.sum()),
-                               buf.data_ptr() + items.nbytes, stream.cuda_stream, max_blocks)
+    ends = np.cumsum(ch)
+    # the items (with their chunk offsets), the work cursor and the error word go over in one
+    # asynchronous copy from pinned memory, which the host allocator keeps until the copy has run
+    host = torch.empty(items.nbytes + 16, dtype=torch.uint8, pin_memory=True)
+    raw = host.numpy()
+    table = raw[:items.nbytes].view(ITEM_DTYPE)
+    table[:] = items
+    table["chunk_begin"] = ends - ch
+    raw[items.nbytes:] = 0
+    buf = torch.empty(host.numel(), dtype=torch.uint8, device=model.table.device)
+    buf.copy_(host, non_blocking=True)
+    at, current = buf.data_ptr(), _lib.stream_ptr()
+    if slice is None:
+        _call_points(model, at, items.size, int(ends[-1]), at + items.nbytes, current, max_blocks)
+    else:
+        _call_points_slice(model, slice.data_ptr(), at, items.size, int(ends[-1]), at + items.nbytes, current,
+                           max_blocks)
 
 
 def reproject_workspace_bytes(model: _HashGridModel, geometry, pixels: int | None = None) -> int:
