@@ -13,6 +13,7 @@
 //                        atomics.
 // Sample positions and encodings live only in registers and shared memory.
 #include <algorithm>
+#include <type_traits>
 
 #include "mlp_tile.cuh"
 #include "train_common.cuh"
@@ -322,6 +323,7 @@ __device__ __forceinline__ void plain_backward(const GridDev& grid, const T* __r
   constexpr int IN = L * F;
   using Plan = PlainBwdPlan<IN, H>;
   constexpr int NT = Plan::NT, NTH = Plan::NTH, LD = NT + 4;
+  constexpr int kSegment = 8;   // samples of a thread in the 4D scatter
   const SimtWeights sw = stage_weights<IN, H, Plan::kBoth>(W, smem);
   TilePoints<NT>& pts =
       *reinterpret_cast<TilePoints<NT>*>(smem + simt_weight_floats<IN, H, Plan::kBoth>());
@@ -397,10 +399,35 @@ __device__ __forceinline__ void plain_backward(const GridDev& grid, const T* __r
       p.store(sG, [&](float v, int) { return v; });
     }
     __syncthreads();
-    {
+    if constexpr (D == 4) {
+      // A thread takes one level of kSegment consecutive samples and marches over
+      // them: 16 reductions a sample and level otherwise (300,007 points along rays:
+      // 0.89 -> 0.78 ms).  With the 8 of 3D, sample by sample is the faster (16,384
+      // rays x 256: 4.58 against 5.31 ms).
+      for (int e = t; e < L * (NT / kSegment); e += NTH) {
+        const int l = e / (NT / kSegment), first = e % (NT / kSegment) * kSegment;
+        auto march = [&](auto hashed) {
+          CellMarch<D, F, hashed()> m(grid, l, table_grad, tval);
+#pragma unroll 1
+          for (int s = first; s < first + kSegment; ++s) {
+            if (!pts.valid[s]) continue;
+            const float x[3] = {pts.p[s], pts.p[NT + s], pts.p[2 * NT + s]};
+            float d[F];
+#pragma unroll
+            for (int f = 0; f < F; ++f) d[f] = sG[(l * F + f) * LD + s];
+            m.add(x, d);
+          }
+          m.finish();
+        };
+        if ((grid.hashed_bits >> l) & 1u)
+          march(std::true_type{});
+        else
+          march(std::false_type{});
+      }
+    } else {
       const int s = t % NT;
       if (pts.valid[s]) {
-        const float x[4] = {pts.p[s], pts.p[NT + s], pts.p[2 * NT + s], tval};
+        const float x[3] = {pts.p[s], pts.p[NT + s], pts.p[2 * NT + s]};
 #pragma unroll 1
         for (int l = t / NT; l < L; l += NTH / NT) {
           float d[F];
