@@ -205,15 +205,17 @@ def reproject(model: _HashGridModel, geometry, angle: float, t: float = 0.0, poi
     if pixels is None and not warpgroups:
         need = _lib.lib.nectb_train_workspace_bytes(ctypes.byref(cg.c_struct), ctypes.byref(model.grid_desc),
                                                     ctypes.byref(model.mlp_desc), P)
-        if workspace is None:
-            # with room for the sigmas of some strips of 32 detector rows, a mixed model's view runs
-            # them column by column (at most VIEW_SIGMA_BYTES; results do not depend on it)
-            strip = 4 * 32 * geometry.nDetector[1] * S
-            rows = -(-geometry.nDetector[0] // 32)
-            if model.precision == "mixed" and max_blocks == 0:
-                need = (need + 255) // 256 * 256 + min(rows, max(VIEW_SIGMA_BYTES // strip, 1)) * strip
         if workspace is None or workspace.numel() < need:
-            workspace = torch.empty(need, dtype=torch.uint8, device=dev)
+            # with room for the sigmas of some strips of 32 detector rows, a mixed model's view runs
+            # them column by column (at most VIEW_SIGMA_BYTES, or one strip; results do not depend on it)
+            extra = 0
+            if model.precision == "mixed" and max_blocks == 0:
+                strip = 4 * 32 * geometry.nDetector[1] * S
+                extra = 256 + min(-(-geometry.nDetector[0] // 32), max(VIEW_SIGMA_BYTES // strip, 1)) * strip
+            try:
+                workspace = torch.empty(need + extra, dtype=torch.uint8, device=dev)
+            except torch.OutOfMemoryError:
+                workspace = torch.empty(need, dtype=torch.uint8, device=dev)
         rc = _lib.lib.nectb_query_reproject(ctypes.byref(cg.c_struct), ctypes.byref(model.grid_desc),
                                             ctypes.byref(model.mlp_desc), model.grid_table.data_ptr(),
                                             model.mlp.data_ptr(), float(angle), float(t), S,
