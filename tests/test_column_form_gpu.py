@@ -83,3 +83,24 @@ def test_training_predictions_are_the_same(cuda_device, F, rays, S, repeat):
     assert abs(got[0][3] - got[1][3]) <= 1e-5 * abs(got[1][3])
     for a, b in zip(got[0][1:3], got[1][1:3]):
         assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
+
+
+def test_loss_of_many_rays(cuda_device):
+    """The loss against float64 over the predictions.  A block adds its rays' terms once, so
+    at most 4 x 148 fp32 adds meet in one number, each off by 2^-24 of it at most: a random
+    walk of sqrt(592) steps of 2^-24 / 3 is 4.8e-7, and four times that is allowed."""
+    from nect_b200.trainer import RayBatch, Workspace, train_step
+
+    geo, m = build(3, 2, det=(256, 256), wide=0.5)
+    P, S = 65536, 128
+    g = torch.Generator(device="cuda").manual_seed(6)
+    batch = RayBatch(perm=torch.randperm(P, device="cuda", generator=g), start=0, num_rays=P, points_per_ray=S,
+                     angle=0.3, max_ray_distance_per_point=geo.max_distance_traveled / S,
+                     jitter=torch.rand(P, device="cuda", generator=g) - 0.5,
+                     detector_offset=torch.zeros(P, 2, device="cuda"),
+                     projection=torch.rand(P, device="cuda", generator=g))
+    tg, mg = torch.zeros_like(m.table), torch.zeros_like(m.mlp)
+    loss, y = train_step(m, geo.get_c_geometry(), batch, geo.max_distance_traveled, tg, mg,
+                         Workspace(staging=True), "l2")
+    want = float((y.double() - batch.projection[batch.perm].double()).square().mean())
+    assert abs(float(loss) - want) <= 2e-6 * want
