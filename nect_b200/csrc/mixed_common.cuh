@@ -103,7 +103,7 @@ __device__ __forceinline__ void act_row(const float* h, uint8_t* tile, int r, in
   }
 }
 
-// The raw corner entries of one level at p (coordinates in [0, 1]) and the
+// The raw corner entries of one level at p and the
 // fractions along the axes: the integers and fractions of level_corners, with the
 // index rule of the level (hash or strides) taken by one uniform branch instead of
 // a select per corner, and 32-bit entry offsets from the level's base.
@@ -117,11 +117,12 @@ struct LevelFetch {
     uint32_t c[D];
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-      const int res = g.res[l][k];
+      const uint32_t res = (uint32_t)g.res[l][k];
       const float q = __fmul_rn(p[k], (float)res);   // as level_corners
-      const int ci = min((int)floorf(q), res - 1);   // q >= 0
-      c[k] = (uint32_t)ci;
-      f[k] = q - (float)ci;
+      // clamp(floor(q), 0, res - 1): the conversion truncates and takes what is below 0
+      // (a t the caller passed as it was) to 0, so the lower end costs nothing
+      c[k] = min(__float2uint_rz(q), res - 1u);
+      f[k] = q - (float)c[k];
     }
     uint32_t idx[1 << D];
     const bool hashed = (g.hashed_bits >> l) & 1u;
