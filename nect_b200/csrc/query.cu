@@ -519,6 +519,7 @@ int reproject_range(const NectbGeometry* geometry, const NectbHashGrid* grid, co
   a.max_blocks = max_blocks;
   a.fwd_warpgroups = max_blocks > 0 ? 0 : warpgroups;
   a.n_cols = geometry->nDetector[1];
+  a.query = true;
   // a whole view with room past the base size: the column form's sigmas, whole strips at a time
   const size_t base = align256(workspace_bytes(count, count));
   const int64_t strip = 32 * (int64_t)a.n_cols;

@@ -1,0 +1,26 @@
+// The order in which a batch's rays are scheduled.  Host and device code without CUDA
+// types, so that it can be checked on the CPU.
+#pragma once
+
+#ifdef __CUDACC__
+#define NECTB_HD __host__ __device__ __forceinline__
+#else
+#define NECTB_HD inline
+#endif
+
+namespace nectb {
+
+// Slot of scheduling index idx: the detector in strips of 32 rows, a strip
+// column by column, so that 32 consecutive rays are vertical neighbours.
+// Their paths differ along axis 0 only (the rotation axis), whose vertices
+// share sectors of the tables.  A permutation of [0, P) for whole rows of
+// pixels; the pixels of a part of a row (a piece of a view) keep their order.
+NECTB_HD int strip_slot(int idx, int P, int cols, int sub) {
+  if (P % (cols * sub) != 0) return idx;
+  const int rows = P / (cols * sub), strip = idx / (32 * cols * sub);
+  const int left = rows - 32 * strip, h = left < 32 ? left : 32, rem = idx - strip * 32 * cols * sub;
+  const int cj = rem / h, row = 32 * strip + rem - cj * h;   // cj = column * sub + sub-angle
+  return row * cols * sub + cj;
+}
+
+}  // namespace nectb

@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "geometry.cuh"
 #include "hashgrid.cuh"
+#include "ray_plan.cuh"
 
 namespace nectb {
 
@@ -36,6 +37,9 @@ struct TrainArgs {
   int num_rays;
   int n_pixels;  // nDetector[0] * nDetector[1]
   int n_cols = 1;  // nDetector[1]
+  // a re-projection (a whole view or any range of its pixels): no backward follows, so
+  // no ray order is made and no rows are stored, whatever the workspace holds
+  bool query = false;
   int S;
   float angle;
   float t;
@@ -312,17 +316,6 @@ __device__ __forceinline__ int next_ray(unsigned int* cursor, const int32_t* __r
       if (recs[idx].count > 0) return (int)idx;
     }
   }
-}
-
-// Slot of scheduling index idx: the detector in strips of 32 rows, a strip
-// column by column, so that 32 consecutive rays are vertical neighbours.
-// Their paths differ along axis 0 only (the rotation axis), whose vertices
-// share sectors of the tables.
-__device__ __forceinline__ int strip_slot(int idx, int P, int cols, int sub) {
-  const int rows = P / (cols * sub), strip = idx / (32 * cols * sub);
-  const int h = min(32, rows - 32 * strip), rem = idx - strip * 32 * cols * sub;
-  const int cj = rem / h, row = 32 * strip + rem - cj * h;   // cj = column * sub + sub-angle
-  return row * cols * sub + cj;
 }
 
 // The rays with samples in scheduling order, for the two-pass backward's

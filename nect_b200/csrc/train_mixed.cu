@@ -1298,7 +1298,7 @@ int run_mixed(const NectbGeometry& geo, const GridDev& grid, const __half* table
   // per_round rays
   const StageLayout SL = stage_layout(ws, R, a.n_pixels, a.S, Shape::INP * sizeof(__nv_bfloat16),
                                       (size_t)ray_slots(a.S) * IN * sizeof(float), tune.staged_rounds,
-                                      tune.encoding_store != 0 && !shares_sms);
+                                      tune.encoding_store != 0 && !shares_sms && !a.query);
   auto run_order = [&]() -> int {
     ProfScope ps(kProfOrder, s);
     const int n_blocks = order_blocks(R, a.n_pixels);
