@@ -16,11 +16,12 @@ namespace nectb {
 // share sectors of the tables.  A permutation of [0, P) for whole rows of
 // pixels; the pixels of a part of a row (a piece of a view) keep their order.
 NECTB_HD int strip_slot(int idx, int P, int cols, int sub) {
-  if (P % (cols * sub) != 0) return idx;
-  const int rows = P / (cols * sub), strip = idx / (32 * cols * sub);
-  const int left = rows - 32 * strip, h = left < 32 ? left : 32, rem = idx - strip * 32 * cols * sub;
+  const int line = cols * sub;   // 32 of them may exceed an int, strip * 32 of them do not
+  if (P % line != 0) return idx;
+  const int rows = P / line, strip = idx / line / 32;
+  const int left = rows - 32 * strip, h = left < 32 ? left : 32, rem = idx - strip * 32 * line;
   const int cj = rem / h, row = 32 * strip + rem - cj * h;   // cj = column * sub + sub-angle
-  return row * cols * sub + cj;
+  return row * line + cj;
 }
 
 }  // namespace nectb

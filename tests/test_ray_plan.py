@@ -38,3 +38,14 @@ def test_strip_order_is_a_permutation(plan, P, cols, sub):
             assert slots[:32] == [r * cols * sub for r in range(32)]
     else:
         assert slots == list(range(P))
+
+
+@pytest.mark.parametrize("rows,cols,sub", [(1, (1 << 27) + 1, 1), (3, 300_000_001, 1), (1, 1 << 26, 4),
+                                           (40, (1 << 21) + 3, 25)])
+def test_strip_order_of_wide_detectors(plan, rows, cols, sub):
+    """Detectors whose strip of 32 rows has more than 2^31 - 1 slots."""
+    line = cols * sub
+    for i in [0, 1, 31, 32, line - 1, line // 3, rows * line // 2, rows * line - 32, rows * line - 1]:
+        strip = i // (32 * line)
+        h, rem = min(32, rows - 32 * strip), i - strip * 32 * line
+        assert plan.slot(i, rows * line, cols, sub) == (32 * strip + rem % h) * line + rem // h
