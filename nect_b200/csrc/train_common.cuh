@@ -1,6 +1,6 @@
 // Pieces shared by the plain (fp32 SIMT) and mixed (bf16 tcgen05) fused
 // training kernels: per-ray records, the ray-preparation kernel, the ray
-// scheduler, sample regeneration and the workspace layout.
+// scheduler and sample regeneration.
 #pragma once
 #include <algorithm>
 #include <cmath>
@@ -74,52 +74,7 @@ struct TrainArgs {
 
 enum : unsigned int { kFlagDuplicatePixels = 1u };
 
-// The two-pass mixed backward: the most rounds a staging buffer may need
-// before the fused single-pass backward is used instead (the recommended
-// staging is sized for NectbTuning::staged_rounds, 4 by default).
-constexpr int kMaxStagedRounds = 64;
-constexpr size_t kStagingCap = size_t(16) << 30;  // largest staging buffer recommended
-// A round staging less than this leaves part of the GPU idle in the scatter:
-// batches below it take one round (24,999 rays x 100 samples: the scatter of a
-// step 1.12 ms in four rounds of four level passes, 0.58 ms in one launch).
-constexpr size_t kStagedRoundMin = size_t(1) << 30;
-constexpr int kOrderBlock = 1024;                  // threads of the ray-order kernels
-
-// Stored encodings: the forward writes each sample's bf16 MLP input row, which
-// the backward reads back instead of gathering the tables again.  Largest
-// store the recommended staging size includes.
-constexpr size_t kEncodingStoreCap = size_t(80) << 30;
-
-// Staged samples per ray: S rounded up so that each run of four samples of a
-// ray's features is 16-byte aligned.
-__host__ __device__ inline int ray_slots(int S) { return (S + 3) & ~3; }
-
-inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
-inline int order_blocks(int R, int P) { return (std::max(R, P) + kOrderBlock - 1) / kOrderBlock; }
-
-// Bytes at the front of the staging region: the ray order, its block sums,
-// the sample offset of every ranked ray and their block sums.
-inline size_t order_bytes(int R, int P) {
-  const size_t nb = (size_t)order_blocks(R, P) + 1;
-  return align256((size_t)R * 4) + align256(nb * 4) + align256((size_t)R * 8) + align256(nb * 8);
-}
-
-// Workspace: RayRec[R] | slot[P] (int32: batch index of the ray through each
-// detector pixel, -1 if none) | 64-byte control block (scheduling cursors of
-// the forward and backward, error word, flags).
-// Any workspace bytes beyond workspace_bytes() (from a 256-byte boundary) are
-// the staging buffer of the two-pass mixed backward.
-struct Workspace {
-  RayRec* rays;
-  int32_t* slot;
-  unsigned int* counters;  // [0] forward cursor, [1] backward cursor, [2] error word, [3] flags,
-                           // [5] scatter cursor, [6] rays with samples, [7] encoding-store rows
-                           // the forward filled, [8] forward loss sum (split step),
-                           // [9] chunks of 32 samples (about)
-  float* stage = nullptr;
-  size_t stage_bytes = 0;
-};
-
+// Workspace (ray_plan.cuh) of R rays over P slots, without staging.
 inline size_t workspace_bytes(int R, int P) { return (size_t)R * sizeof(RayRec) + (size_t)P * 4 + 256; }
 
 inline Workspace carve_workspace(void* ws, int R, int P, size_t size = 0) {
@@ -133,70 +88,6 @@ inline Workspace carve_workspace(void* ws, int R, int P, size_t size = 0) {
     w.stage_bytes = size - base;
   }
   return w;
-}
-
-// Split of the staging region of the two-pass mixed backward:
-//   order[R] int32 | block sums | offs[R] uint64 (first stored row of each
-//   ranked ray) | block sums | encoding store [xcap rows of row_bytes] |
-//   staged dL/d(encoding) of one round of per_round rays (per_ray bytes each).
-// The staged rounds take the recommended size for `rounds` rounds (capped at
-// kStagingCap) and the encoding store the rest, up to R * S rows; when that
-// leaves less than one ray's rows there is no store and the rounds take the
-// whole region.  per_round == 0: no staging (the fused single-pass backward).
-// The store starts at the same address whatever the split, so a backward half
-// reading rows [0, min(its xcap, the forward's)) never reads its own staging.
-struct StageLayout {
-  int32_t* order = nullptr;
-  unsigned int* block_sums = nullptr;
-  uint64_t* offs = nullptr;
-  unsigned long long* block_samples = nullptr;
-  uint4* xstore = nullptr;
-  uint32_t xcap = 0;  // rows of the encoding store
-  float* stage = nullptr;
-  int64_t per_round = 0;
-};
-
-inline size_t staged_round_bytes(int R, int rounds, size_t per_ray) {
-  rounds = (int)std::max<int64_t>(1, std::min<int64_t>(rounds, (int64_t)((size_t)R * per_ray / kStagedRoundMin)));
-  const int64_t per_round = (R + rounds - 1) / rounds;
-  return std::min((size_t)per_round * per_ray, kStagingCap / per_ray * per_ray);
-}
-
-// store == false: no encoding store whatever the buffer size (the backward
-// recomputes every sample's encoding from the tables).
-inline StageLayout stage_layout(const Workspace& ws, int R, int P, int S, size_t row_bytes, size_t per_ray,
-                                int rounds, bool store = true) {
-  StageLayout L;
-  const size_t ob = order_bytes(R, P);
-  if (!ws.stage || ws.stage_bytes <= ob || R <= 0) return L;
-  char* p = reinterpret_cast<char*>(ws.stage);
-  const size_t nb = (size_t)order_blocks(R, P) + 1;
-  L.order = reinterpret_cast<int32_t*>(p);
-  L.block_sums = reinterpret_cast<unsigned int*>(p + align256((size_t)R * 4));
-  L.offs = reinterpret_cast<uint64_t*>(p + align256((size_t)R * 4) + align256(nb * 4));
-  L.block_samples = reinterpret_cast<unsigned long long*>(p + align256((size_t)R * 4) + align256(nb * 4) +
-                                                          align256((size_t)R * 8));
-  const size_t avail = ws.stage_bytes - ob;
-  const size_t want = staged_round_bytes(R, rounds, per_ray);
-  size_t xbytes = 0;
-  if (store && avail >= want + (size_t)S * row_bytes + 256) {
-    const size_t rows = std::min<size_t>({(avail - want - 256) / row_bytes, (size_t)R * S, 0xffffffffu});
-    if (rows >= (size_t)S) {
-      L.xcap = (uint32_t)rows;
-      xbytes = align256(rows * row_bytes);
-      L.xstore = reinterpret_cast<uint4*>(p + ob);
-    }
-  }
-  // 16-byte aligned rows whatever the caller's workspace pointer
-  const uintptr_t at = reinterpret_cast<uintptr_t>(p + ob + xbytes), pad = ((at + 15) & ~uintptr_t(15)) - at;
-  L.stage = reinterpret_cast<float*>(at + pad);
-  L.per_round = avail < xbytes + pad ? 0 : std::min<int64_t>((int64_t)((avail - xbytes - pad) / per_ray), R);
-  if (L.per_round <= 0 || (R + L.per_round - 1) / L.per_round > kMaxStagedRounds) {
-    L.per_round = 0;
-    L.xstore = nullptr;
-    L.xcap = 0;
-  }
-  return L;
 }
 
 // Time slice of a 4D grid at the batch's t (mixed training).  Along t a

@@ -1,5 +1,6 @@
-"""The scheduling order of a batch's rays (csrc/ray_plan.cuh), compiled for the CPU:
-every slot exactly once, whatever part of the detector the pixels are."""
+"""The scheduling order of a batch's rays and the split of its workspace
+(csrc/ray_plan.cuh), compiled for the CPU: every slot exactly once, whatever part of the
+detector the pixels are; the stored rows a workspace of a given size keeps."""
 import ctypes
 import shutil
 import subprocess
@@ -10,7 +11,27 @@ import pytest
 CSRC = Path(__file__).resolve().parents[1] / "nect_b200" / "csrc"
 SOURCE = """
 #include "ray_plan.cuh"
-extern "C" int slot(int i, int P, int cols, int sub) { return nectb::strip_slot(i, P, cols, sub); }
+using namespace nectb;
+extern "C" int slot(int i, int P, int cols, int sub) { return strip_slot(i, P, cols, sub); }
+extern "C" int64_t order(int R, int P) { return (int64_t)order_bytes(R, P); }
+extern "C" int64_t recommended(int R, int rounds, int64_t per_ray) {
+  return (int64_t)staged_round_bytes(R, rounds, (size_t)per_ray);
+}
+// rows of the store, rays of a round; every part of the region inside it, in order
+extern "C" int layout(int64_t at, int64_t bytes, int R, int P, int S, int64_t row, int64_t per_ray, int rounds,
+                      int64_t* rows, int64_t* per_round) {
+  Workspace ws;
+  ws.stage = (float*)at;
+  ws.stage_bytes = (size_t)bytes;
+  const StageLayout L = stage_layout(ws, R, P, S, (size_t)row, (size_t)per_ray, rounds);
+  *rows = L.xcap;
+  *per_round = L.per_round;
+  if (!L.per_round) return 1;
+  const int64_t o = (int64_t)L.order, f = (int64_t)L.offs, s = (int64_t)L.block_samples, g = (int64_t)L.stage;
+  const int64_t x = L.xstore ? (int64_t)L.xstore : g;
+  return o >= at && (int64_t)L.block_sums >= o + 4 * (int64_t)R && f > (int64_t)L.block_sums && s >= f + 8 * (int64_t)R &&
+         x > s && x % 16 == 0 && g % 16 == 0 && x + L.xcap * row <= g && g + L.per_round * per_ray <= at + bytes;
+}
 """
 
 
@@ -23,7 +44,18 @@ def plan(tmp_path_factory):
     (d / "plan.cpp").write_text(SOURCE)
     subprocess.run([cxx, "-std=c++17", "-O1", "-shared", "-fPIC", f"-I{CSRC}", str(d / "plan.cpp"), "-o",
                     str(d / "plan.so")], check=True)
-    return ctypes.CDLL(str(d / "plan.so"))
+    lib = ctypes.CDLL(str(d / "plan.so"))
+    i64, i32 = ctypes.c_int64, ctypes.c_int
+    lib.order.restype = lib.recommended.restype = i64
+    lib.recommended.argtypes = [i32, i32, i64]
+    lib.layout.argtypes = [i64, i64, i32, i32, i32, i64, i64, i32, ctypes.POINTER(i64), ctypes.POINTER(i64)]
+    return lib
+
+
+def layout(plan, bytes_, R, P, S, row, per_ray, rounds, at=1 << 40):
+    rows, per_round = ctypes.c_int64(), ctypes.c_int64()
+    assert plan.layout(at, bytes_, R, P, S, row, per_ray, rounds, ctypes.byref(rows), ctypes.byref(per_round))
+    return rows.value, per_round.value
 
 
 @pytest.mark.parametrize("P,cols,sub", [
@@ -49,3 +81,27 @@ def test_strip_order_of_wide_detectors(plan, rows, cols, sub):
         strip = i // (32 * line)
         h, rem = min(32, rows - 32 * strip), i - strip * 32 * line
         assert plan.slot(i, rows * line, cols, sub) == (32 * strip + rem % h) * line + rem // h
+
+
+@pytest.mark.parametrize("R,S,features", [(700, 64, 32), (24999, 100, 32), (16000, 64, 64), (4882, 512, 76),
+                                          (65536, 512, 32), (262144, 512, 32), (1, 1, 32)])
+@pytest.mark.parametrize("rounds", [1, 4, 16])
+def test_rows_come_before_large_rounds(plan, R, S, features, rounds):
+    """The recommended size keeps every row and its rounds; below it the store keeps the rows
+    that rounds of R / `rounds` rays leave it, and rounds grow only into what is left."""
+    row, per_ray, P = (features + 15) // 16 * 32, (S + 3) // 4 * 4 * features * 4, 512 * 512
+    ob, best = plan.order(R, P), plan.recommended(R, rounds, per_ray)
+    least = -(-R // rounds) * per_ray
+    full = ob + best + 256 + (R * S * row + 255) // 256 * 256
+    assert layout(plan, full, R, P, S, row, per_ray, rounds) == (R * S, min(R, (best + 256) // per_ray))
+    for k in range(1, 200):
+        size = ob + (full - ob) * k // 200
+        rows, per_round = layout(plan, size, R, P, S, row, per_ray, rounds)
+        if size - ob >= best + R * S * row + 256:
+            want = R * S
+        else:
+            want = max(0, min(R * S, (size - ob - least - 256) // row))
+            want = want if want >= S else 0
+        if per_round:   # (the fused single pass below 64 rounds)
+            assert rows == want
+            assert per_round >= (least // per_ray if rows else 1)

@@ -1,0 +1,58 @@
+"""The staged mixed step in workspaces below the recommended size: rounds of a quarter of
+the rays beside a store of every row, of a part of them and of none, against the single
+fused pass.  Predictions bit for bit (the same network on the same positions); gradients
+within 1e-5 of the largest entry, the bound of the other staged-against-single-pass tests
+(the same products, other fp32 sums)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dims,F", [(3, 2), (3, 4), (4, 2)])
+@pytest.mark.parametrize("store", [1.0, 0.4, 0.0])
+def test_rows_of_small_workspaces(cuda_device, dims, F, store):
+    from nect_b200 import autotune
+    from nect_b200.config import HashEncoderConfig, MLPNetConfig
+    from nect_b200.network import HashGrid, HashGrid4D
+    from nect_b200.sampling import Geometry
+    from nect_b200.trainer import RayBatch, Workspace, train_step
+
+    R, S, det = 3000, 65, (80, 96)
+    P, row, per_ray = det[0] * det[1], 16 * F * 2, 68 * 16 * F * 4
+    geo = Geometry(nDetector=list(det), dDetector=[0.8, 0.7], mode="cone", DSD=300.0, DSO=200.0, nVoxel=[32] * 3,
+                   dVoxel=[1.0] * 3)
+    enc = HashEncoderConfig(n_levels=16, n_features_per_level=F, log2_hashmap_size=12, base_resolution=4,
+                            finest_resolution=256, base_resolution_t=2 if dims == 4 else None)
+    m = (HashGrid if dims == 3 else HashGrid4D)(enc, MLPNetConfig(n_hidden_layers=2), precision="mixed",
+                                                device="cuda", seed=0)
+    with torch.no_grad():
+        m.table.normal_(0.0, 0.3, generator=torch.Generator(device="cuda").manual_seed(1))
+        m.refresh_half()
+
+    class Sized(Workspace):
+        def get(self, model, c_geometry, num_rays, device, points_per_ray=0):
+            ptr, n = super().get(model, c_geometry, num_rays, device, points_per_ray)
+            less = (R - -(-R // 4)) * per_ray + (R * S - int(store * R * S)) * row   # a quarter's round, fewer rows
+            return ptr, n - less - (256 if store == 0 else 0)
+
+    g = torch.Generator(device="cuda").manual_seed(2)
+    batch = RayBatch(perm=torch.randperm(P, device="cuda", generator=g), start=0, num_rays=R, points_per_ray=S,
+                     angle=0.7, max_ray_distance_per_point=geo.max_distance_traveled / S,
+                     jitter=torch.rand(R, device="cuda", generator=g) - 0.5,
+                     detector_offset=torch.zeros(R, 2, device="cuda"),
+                     projection=torch.rand(P, device="cuda", generator=g), t=0.3)
+    default = autotune.get_tuning()
+    got = []
+    try:
+        autotune.set_tuning(dict(default, time_slice=0))
+        for ws in (Sized(), Workspace(staging=False)):
+            tg, mg = torch.zeros_like(m.table), torch.zeros_like(m.mlp)
+            _, y = train_step(m, geo.get_c_geometry(), batch, geo.max_distance_traveled, tg, mg, ws, "l2")
+            assert ws.error_word() == 0
+            got.append((y, tg, mg))
+    finally:
+        autotune.set_tuning(default)
+    assert torch.equal(got[0][0], got[1][0])
+    for a, b in zip(got[0][1:], got[1][1:]):
+        assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
