@@ -154,4 +154,20 @@ inline StageLayout stage_layout(const Workspace& ws, int R, int P, int S, size_t
   return L;
 }
 
+// The staged backward's weight gradients gather in the tensor cores' accumulators,
+// which lose about 2e-8 of the sum per product (three times the length measured 3e-5 of
+// the gradient), so they are added to fp32 memory at least once per R / rounds rays,
+// however many rays a launch has: at its end where it has no more than that, else inside
+// it too.  The stretches of the batch (1: at the ends alone).
+NECTB_HD int accumulator_stretches(int64_t R, int64_t per_round, int rounds) {
+  return per_round <= (R + rounds - 1) / rounds ? 1 : rounds;
+}
+
+// Tiles (of four 32-sample chunks) of a stretch for each of the launch's blocks.
+NECTB_HD int stretch_tiles(unsigned int chunks, int stretches, int blocks) {
+  if (stretches <= 1) return 0x7fffffff;
+  const uint64_t per = ((uint64_t)chunks + 4 * (uint64_t)stretches * blocks - 1) / (4 * (uint64_t)stretches * blocks);
+  return per < 1 ? 1 : (int)per;
+}
+
 }  // namespace nectb

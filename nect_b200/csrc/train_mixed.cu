@@ -436,17 +436,6 @@ column_sum_kernel(TrainArgs a, RayRec* __restrict__ recs, const int32_t* __restr
   }
 }
 
-// Tiles after which a block of the staged backward adds its weight gradients to
-// fp32 memory and starts them anew.  They gather in the tensor cores' accumulators,
-// which lose about 2e-8 of the sum per product: batches are split into `flushes`
-// stretches over the whole order (launches of R / staged_rounds rays measured the
-// same losses; three times the length 3e-5 of the gradient).
-__device__ __forceinline__ int flush_interval(const unsigned int* ctrl, float flushes) {
-  if (flushes <= 1.f) return 0x7fffffff;
-  const float tiles = (float)ctrl[9] * 0.25f;   // 32-sample chunks of the batch, four to a tile
-  return max(1, (int)ceilf(tiles / (flushes * (float)gridDim.x)));
-}
-
 // Staged mode (kStaged): instead of scattering, dL/d(encoding) of every sample
 // is written to the staging buffer, level-major: stage[(l * slots + s) * F + f]
 // with s = (scheduling index - lo) * ray_slots(S) + sample, for the rays whose
@@ -472,7 +461,7 @@ bwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
                  const RayRec* __restrict__ recs, const int32_t* __restrict__ slot, unsigned int* __restrict__ ctrl,
                  int out_act, float* __restrict__ table_grad, float* __restrict__ W_grad, int lo, int hi,
                  float* __restrict__ stage, int64_t slots, const int32_t* __restrict__ order,
-                 const uint64_t* __restrict__ offs, const uint4* __restrict__ xstore, uint32_t xcap, float flushes) {
+                 const uint64_t* __restrict__ offs, const uint4* __restrict__ xstore, uint32_t xcap, int stretches) {
   using S = InShape<L, F>;
   using Plan = BwdPlan<L, F, H>;
   constexpr int IN = S::IN, KT = S::KT;
@@ -495,11 +484,12 @@ bwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
   float* sWout = reinterpret_cast<float*>(sX + KT * kTile);
   uint64_t* bar = reinterpret_cast<uint64_t*>(sWout + 64);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
-  float* red = reinterpret_cast<float*>(tslot + 4);  // [4][64]
+  float* red = reinterpret_cast<float*>(tslot + 4);  // [4][64]: the warps' w_out gradients of past stretches
   auto sAk = [&](int k) { return sG + (H - k) * kTile; };   // A_k (k = 1..H-1), later G_k
 
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   stage_mixed_weights<L, F, H>(W, sW, sWout);
+  for (int e = t; e < 4 * 64; e += kMixThreads) red[e] = 0.f;
   if (warp == 0) {
     tc::tmem_alloc(tslot, Plan::kCols);
     tc::tmem_relinquish();
@@ -522,8 +512,7 @@ bwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
   constexpr uint32_t id_dW0 = tc::idesc_bf16(128, S::INP, true, true);
 
   uint32_t phase = 0;
-  uint32_t wacc = 0;  // weight-gradient accumulators start at the first tile
-  int left = flush_interval(ctrl, flushes);   // tiles until the accumulators are added to memory
+  uint32_t wacc = 0;  // weight-gradient accumulators start at a stretch's first tile
   float dwout0 = 0.f, dwout1 = 0.f;  // w_out gradient entries j0_out and j0_out + 1 of this lane
   int j0_out = 0;
   RayCursor cur;
@@ -579,187 +568,188 @@ bwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
     tc::fence_after();
     return true;
   };
-  while (true) {
-    const bool active =
-        next_chunk(cur, recs, ctrl + 1, slot, a, by_pixel, lane, lo, hi, order, n_valid, offs, xrows);
-    if (!__syncthreads_or(active)) break;
-    const int i = cur.base + lane;
-    float p[4] = {0.f, 0.f, 0.f, 0.f};
-    bool valid = false;
-    if (active && i < cur.rec.count) valid = sample_point(cur.rec, i, p);
-    if (D == 4) p[3] = a.t;
-    if (cur.xrow >= 0) {  // the forward stored this ray's rows: stream them back (warp-uniform branch)
-      const uint4* src = xstore + (size_t)(cur.xrow + i) * S::NCH;
-      if (!pre_ok && valid) {  // not prefetched: the first chunk of a ray
-#pragma unroll
-        for (int j = 0; j < S::NCH; ++j) xrow[j] = __ldcs(src + j);
+  // a stretch: the tiles whose weight gradients stay in the accumulators
+  bool done = false;
+  do {
+    int left = stretch_tiles(ctrl[9], stretches, gridDim.x);
+    while (true) {
+      const bool active =
+          next_chunk(cur, recs, ctrl + 1, slot, a, by_pixel, lane, lo, hi, order, n_valid, offs, xrows);
+      if (!__syncthreads_or(active)) {
+        done = true;
+        break;
       }
+      const int i = cur.base + lane;
+      float p[4] = {0.f, 0.f, 0.f, 0.f};
+      bool valid = false;
+      if (active && i < cur.rec.count) valid = sample_point(cur.rec, i, p);
+      if (D == 4) p[3] = a.t;
+      if (cur.xrow >= 0) {  // the forward stored this ray's rows: stream them back (warp-uniform branch)
+        const uint4* src = xstore + (size_t)(cur.xrow + i) * S::NCH;
+        if (!pre_ok && valid) {  // not prefetched: the first chunk of a ray
 #pragma unroll
-      for (int j = 0; j < S::NCH; ++j)
-        tc::st_chunk_raw(sX + (j / 8) * kTile, t, j % 8, valid ? xrow[j] : make_uint4(0u, 0u, 0u, 0u));
-      // prefetch the rows of the warp's next chunk of this ray; they arrive
-      // while this tile's MMAs run (rows below the ray's count lie in its
-      // stored range)
-      pre_ok = cur.base + 32 < cur.rec.count;
-      if (pre_ok && i + 32 < cur.rec.count) {
+          for (int j = 0; j < S::NCH; ++j) xrow[j] = __ldcs(src + j);
+        }
 #pragma unroll
-        for (int j = 0; j < S::NCH; ++j) xrow[j] = __ldcs(src + 32 * S::NCH + j);
+        for (int j = 0; j < S::NCH; ++j)
+          tc::st_chunk_raw(sX + (j / 8) * kTile, t, j % 8, valid ? xrow[j] : make_uint4(0u, 0u, 0u, 0u));
+        // prefetch the rows of the warp's next chunk of this ray; they arrive
+        // while this tile's MMAs run (rows below the ray's count lie in its
+        // stored range)
+        pre_ok = cur.base + 32 < cur.rec.count;
+        if (pre_ok && i + 32 < cur.rec.count) {
+#pragma unroll
+          for (int j = 0; j < S::NCH; ++j) xrow[j] = __ldcs(src + 32 * S::NCH + j);
+        }
+      } else {
+        pre_ok = false;
+        encode_row<D, F, L>(grid, table, p, valid, sX, t);
       }
-    } else {
-      pre_ok = false;
-      encode_row<D, F, L>(grid, table, p, valid, sX, t);
-    }
-    // forward recompute: layer 0 from X, layer k from A_k (stored with its sign mask)
-    float h[64];
-    uint32_t mlo[H], mhi[H];
-    bool ok = run_phase([&] {
+      // forward recompute: layer 0 from X, layer k from A_k (stored with its sign mask)
+      float h[64];
+      uint32_t mlo[H], mhi[H];
+      bool ok = run_phase([&] {
 #pragma unroll
-      for (int q = 0; q < S::INP / 16; ++q)
-        tc::mma(tm, tc::desc_k(sX_a + (q / 4) * kTile, q % 4), tc::desc_k(sW_a + (q / 4) * kWTile, q % 4), id_fwd,
-                q > 0);
-    });
-    if (ok) ld64(my_lanes, h);
-#pragma unroll
-    for (int k = 1; k < H && ok; ++k) {
-      act_row(h, sAk(k), t, act, mlo[k], mhi[k]);
-      const uint32_t a_k = tc::smem_u32(sAk(k));
-      ok = run_phase([&] {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          tc::mma(tm, tc::desc_k(a_k, q), tc::desc_k(sW_a + (KT + k - 1) * kWTile, q), id_fwd, q > 0);
+        for (int q = 0; q < S::INP / 16; ++q)
+          tc::mma(tm, tc::desc_k(sX_a + (q / 4) * kTile, q % 4), tc::desc_k(sW_a + (q / 4) * kWTile, q % 4), id_fwd,
+                  q > 0);
       });
       if (ok) ld64(my_lanes, h);
-    }
-    if (!ok) {
-      timed_out = true;
-      break;
-    }
-    float z = 0.f;
 #pragma unroll
-    for (int j = 0; j < 64; ++j) z = fmaf(sWout[j], hidden_act(h[j], act), z);
-    const float dz = valid ? cur.rec.gsig * act_grad_z(z, out_act) : 0.f;
-    // w_out gradient over the warp's samples; G_H = dz * w_out * a'(h_H)
-    {
-      float v[64];
+      for (int k = 1; k < H && ok; ++k) {
+        act_row(h, sAk(k), t, act, mlo[k], mhi[k]);
+        const uint32_t a_k = tc::smem_u32(sAk(k));
+        ok = run_phase([&] {
 #pragma unroll
-      for (int j = 0; j < 64; ++j) v[j] = dz * hidden_act(h[j], act);
-      float s0, s1;
-      warp_reduce_scatter64(v, lane, s0, s1, j0_out);
-      dwout0 += s0;
-      dwout1 += s1;
-    }
+          for (int q = 0; q < 4; ++q)
+            tc::mma(tm, tc::desc_k(a_k, q), tc::desc_k(sW_a + (KT + k - 1) * kWTile, q), id_fwd, q > 0);
+        });
+        if (ok) ld64(my_lanes, h);
+      }
+      if (!ok) {
+        timed_out = true;
+        break;
+      }
+      float z = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float v[8];
+      for (int j = 0; j < 64; ++j) z = fmaf(sWout[j], hidden_act(h[j], act), z);
+      const float dz = valid ? cur.rec.gsig * act_grad_z(z, out_act) : 0.f;
+      // w_out gradient over the warp's samples; G_H = dz * w_out * a'(h_H)
+      {
+        float v[64];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) v[q] = hidden_grad(dz * sWout[8 * j + q], h[8 * j + q] > 0.f, act);
-      tc::st_chunk_bf16(sG, t, j, v);
-    }
-    // backward through the hidden layers: G_{k+1} (tile gt) gives
-    //   dA_k = G_{k+1} W_k        (A = G K-major, B = W_k MN-major) -> transient columns
-    //   dW_k += G_{k+1}^T A_k     (A = G MN-major, M = 128 padded; B = A_k MN-major; K = 128 samples)
-    // and G_k = dA_k * a'(a_k) replaces A_k once the dW_k product has completed.
-    uint32_t gt = sG_a;
-#pragma unroll
-    for (int k = H - 1; k >= 1 && ok; --k) {
-      const uint32_t a_k = tc::smem_u32(sAk(k));
-      const uint32_t wk = sW_a + (KT + k - 1) * kWTile;
-      const uint32_t dwk = tm + Plan::T + 64 * (k - 1);
-      ok = run_phase([&] {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) tc::mma(tm, tc::desc_k(gt, q), tc::desc_mn(wk, q, kWTile), id_dA, q > 0);
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          tc::mma(dwk, tc::desc_mn(gt, q, pad_lbo), tc::desc_mn(a_k, q, kTile), id_dW, (q > 0) | wacc);
-      });
-      if (!ok) break;
-      ld64(my_lanes, h);
+        for (int j = 0; j < 64; ++j) v[j] = dz * hidden_act(h[j], act);
+        float s0, s1;
+        warp_reduce_scatter64(v, lane, s0, s1, j0_out);
+        dwout0 += s0;
+        dwout1 += s1;
+      }
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         float v[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int c = 8 * j + q;
-          const uint32_t bit = c < 32 ? (mlo[k] >> c) & 1u : (mhi[k] >> (c - 32)) & 1u;
-          v[q] = hidden_grad(h[c], bit != 0, act);
-        }
-        tc::st_chunk_bf16(sAk(k), t, j, v);
+        for (int q = 0; q < 8; ++q) v[q] = hidden_grad(dz * sWout[8 * j + q], h[8 * j + q] > 0.f, act);
+        tc::st_chunk_bf16(sG, t, j, v);
       }
-      gt = a_k;
-    }
-    // dX = G_1 W0 (A = G_1 K-major, B = W0 MN-major over the KT tiles); the
-    // layer-0 weight gradient: dW0 += G_1^T X (one X tile), or
-    // dW0^T += X^T G_1 (two X tiles as the M = 128 operand, B = G_1 MN-major)
-    if (ok)
-      ok = run_phase([&] {
+      // backward through the hidden layers: G_{k+1} (tile gt) gives
+      //   dA_k = G_{k+1} W_k        (A = G K-major, B = W_k MN-major) -> transient columns
+      //   dW_k += G_{k+1}^T A_k     (A = G MN-major, M = 128 padded; B = A_k MN-major; K = 128 samples)
+      // and G_k = dA_k * a'(a_k) replaces A_k once the dW_k product has completed.
+      uint32_t gt = sG_a;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) tc::mma(tm, tc::desc_k(gt, q), tc::desc_mn(sW_a, q, kWTile), id_dX, q > 0);
-        if constexpr (KT == 1) {
+      for (int k = H - 1; k >= 1 && ok; --k) {
+        const uint32_t a_k = tc::smem_u32(sAk(k));
+        const uint32_t wk = sW_a + (KT + k - 1) * kWTile;
+        const uint32_t dwk = tm + Plan::T + 64 * (k - 1);
+        ok = run_phase([&] {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) tc::mma(tm, tc::desc_k(gt, q), tc::desc_mn(wk, q, kWTile), id_dA, q > 0);
 #pragma unroll
           for (int q = 0; q < 8; ++q)
-            tc::mma(dw0, tc::desc_mn(gt, q, pad_lbo), tc::desc_mn(sX_a, q, kTile), id_dW0, (q > 0) | wacc);
-        } else {
+            tc::mma(dwk, tc::desc_mn(gt, q, pad_lbo), tc::desc_mn(a_k, q, kTile), id_dW, (q > 0) | wacc);
+        });
+        if (!ok) break;
+        ld64(my_lanes, h);
 #pragma unroll
-          for (int q = 0; q < 8; ++q)
-            tc::mma(dw0, tc::desc_mn(sX_a, q, kTile), tc::desc_mn(gt, q, kTile), id_dW, (q > 0) | wacc);
+        for (int j = 0; j < 8; ++j) {
+          float v[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const int c = 8 * j + q;
+            const uint32_t bit = c < 32 ? (mlo[k] >> c) & 1u : (mhi[k] >> (c - 32)) & 1u;
+            v[q] = hidden_grad(h[c], bit != 0, act);
+          }
+          tc::st_chunk_bf16(sAk(k), t, j, v);
         }
-      });
-    if (!ok) {
-      timed_out = true;
-      break;
-    }
-    wacc = 1;
-    constexpr int NX = (IN + 15) / 16;  // 16-column chunks holding the IN values of dX
-    float dx[NX * 16];
-#pragma unroll
-    for (int c = 0; c < NX; ++c) tc::tmem_ld16(my_lanes + 16 * c, dx + 16 * c);
-    tc::tmem_wait_ld();
-    if constexpr (kStaged) {
-      if (valid) {
-        float* dst = stage + ((int64_t)(cur.sched - lo) * ray_slots(a.S) + i) * F;
-#pragma unroll
-        for (int l = 0; l < L; ++l) {
-          // evict-first: each staged value is read once, by the scatter pass
-          if constexpr (F == 2)
-            __stcs(reinterpret_cast<float2*>(dst + l * slots * F), make_float2(dx[2 * l], dx[2 * l + 1]));
-          else if constexpr (F == 4)
-            __stcs(reinterpret_cast<float4*>(dst + l * slots * F),
-                   make_float4(dx[4 * l], dx[4 * l + 1], dx[4 * l + 2], dx[4 * l + 3]));
-          else
-#pragma unroll
-            for (int f = 0; f < F; ++f) dst[l * slots * F + f] = dx[l * F + f];
-        }
+        gt = a_k;
       }
-    } else {
-      const uint32_t agg = active ? run_levels(grid, cur.rec.dx, cur.rec.dy, cur.rec.dz, a.run_threshold) : 0u;
-      scatter_warp<D, F>(grid, table_grad, p, valid, dx, F, 1, agg, 0, grid.n_levels);
-    }
-    tc::fence_before();
-    __syncthreads();
-    if (active) cur.base += 32;
-    if (--left == 0) {   // block-uniform
-      flush();
+      // dX = G_1 W0 (A = G_1 K-major, B = W0 MN-major over the KT tiles); the
+      // layer-0 weight gradient: dW0 += G_1^T X (one X tile), or
+      // dW0^T += X^T G_1 (two X tiles as the M = 128 operand, B = G_1 MN-major)
+      if (ok)
+        ok = run_phase([&] {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) tc::mma(tm, tc::desc_k(gt, q), tc::desc_mn(sW_a, q, kWTile), id_dX, q > 0);
+          if constexpr (KT == 1) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              tc::mma(dw0, tc::desc_mn(gt, q, pad_lbo), tc::desc_mn(sX_a, q, kTile), id_dW0, (q > 0) | wacc);
+          } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              tc::mma(dw0, tc::desc_mn(sX_a, q, kTile), tc::desc_mn(gt, q, kTile), id_dW, (q > 0) | wacc);
+          }
+        });
+      if (!ok) {
+        timed_out = true;
+        break;
+      }
+      wacc = 1;
+      constexpr int NX = (IN + 15) / 16;  // 16-column chunks holding the IN values of dX
+      float dx[NX * 16];
+#pragma unroll
+      for (int c = 0; c < NX; ++c) tc::tmem_ld16(my_lanes + 16 * c, dx + 16 * c);
+      tc::tmem_wait_ld();
+      if constexpr (kStaged) {
+        if (valid) {
+          float* dst = stage + ((int64_t)(cur.sched - lo) * ray_slots(a.S) + i) * F;
+#pragma unroll
+          for (int l = 0; l < L; ++l) {
+            // evict-first: each staged value is read once, by the scatter pass
+            if constexpr (F == 2)
+              __stcs(reinterpret_cast<float2*>(dst + l * slots * F), make_float2(dx[2 * l], dx[2 * l + 1]));
+            else if constexpr (F == 4)
+              __stcs(reinterpret_cast<float4*>(dst + l * slots * F),
+                     make_float4(dx[4 * l], dx[4 * l + 1], dx[4 * l + 2], dx[4 * l + 3]));
+            else
+#pragma unroll
+              for (int f = 0; f < F; ++f) dst[l * slots * F + f] = dx[l * F + f];
+          }
+        }
+      } else {
+        const uint32_t agg = active ? run_levels(grid, cur.rec.dx, cur.rec.dy, cur.rec.dz, a.run_threshold) : 0u;
+        scatter_warp<D, F>(grid, table_grad, p, valid, dx, F, 1, agg, 0, grid.n_levels);
+      }
       tc::fence_before();
       __syncthreads();
-      left = flush_interval(ctrl, flushes);
-      wacc = 0;
+      if (active) cur.base += 32;
+      if (--left == 0) break;   // block-uniform
     }
-  }
+    if (timed_out) break;
+    if (wacc) {
+      flush();
+      red[warp * 64 + j0_out] += dwout0;   // (this lane's own)
+      red[warp * 64 + j0_out + 1] += dwout1;
+      dwout0 = dwout1 = 0.f;
+    }
+    wacc = 0;
+    tc::fence_before();
+    __syncthreads();
+  } while (!done);
   if (timed_out) {
     if (t == 0) atomicOr(err, 2u);
     tc::mbar_wait(bar, phase);  // let the MMAs in flight retire (bounded) before freeing TMEM
-  } else if (wacc) {
-    flush();
   }
-  {
-    float s0, s1;
-    float zero[64];
-#pragma unroll
-    for (int j = 0; j < 64; ++j) zero[j] = 0.f;
-    warp_reduce_scatter64(zero, lane, s0, s1, j0_out);  // j0_out of this lane (also when no tile ran)
-  }
-  red[warp * 64 + j0_out] = dwout0;
-  red[warp * 64 + j0_out + 1] = dwout1;
   tc::fence_before();
   __syncthreads();
   if (t < 64)
@@ -783,13 +773,13 @@ bwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
 //   Shared memory: W0, W1 | G2 | zero block | A1, then G1 | X.
 //   Accumulator rows are read 16 columns at a time; the w_out gradient is a
 //   16-column butterfly reduce-scatter per chunk.
-template <int D, int F, int ACT, bool kFlush>
+template <int D, int F, int ACT>
 __global__ void __launch_bounds__(kMixThreads, 3)
 bwd_lean_kernel(GridDev grid, const __half* __restrict__ table, const float* __restrict__ W, TrainArgs a,
                 const RayRec* __restrict__ recs, const int32_t* __restrict__ slot, unsigned int* __restrict__ ctrl,
                 int out_act, float* __restrict__ W_grad, int lo, int hi, float* __restrict__ stage,
                 int64_t slots, const int32_t* __restrict__ order, const uint64_t* __restrict__ offs,
-                const uint4* __restrict__ xstore, uint32_t xcap, float flushes) {
+                const uint4* __restrict__ xstore, uint32_t xcap, int stretches) {
   constexpr int IN = 16 * F;
   constexpr int H = 2;
   constexpr int act = ACT;
@@ -809,7 +799,7 @@ bwd_lean_kernel(GridDev grid, const __half* __restrict__ table, const float* __r
   float* sWout = reinterpret_cast<float*>(sX + kTile);
   uint64_t* bar = reinterpret_cast<uint64_t*>(sWout + 64);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
-  float* red = reinterpret_cast<float*>(tslot + 4);  // [4][64]
+  float* red = reinterpret_cast<float*>(tslot + 4);  // [4][64]: the warps' w_out gradients of past stretches
 
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   stage_mixed_weights<16, F, H>(W, sW, sWout);
@@ -817,6 +807,7 @@ bwd_lean_kernel(GridDev grid, const __half* __restrict__ table, const float* __r
     uint4* z = reinterpret_cast<uint4*>(sZ);
     for (int e = t; e < (int)(kZero / 16); e += kMixThreads) z[e] = make_uint4(0u, 0u, 0u, 0u);
   }
+  for (int e = t; e < 4 * 64; e += kMixThreads) red[e] = 0.f;
   if (warp == 0) {
     tc::tmem_alloc(tslot, 128);
     tc::tmem_relinquish();
@@ -837,8 +828,7 @@ bwd_lean_kernel(GridDev grid, const __half* __restrict__ table, const float* __r
   constexpr uint32_t id_dW0 = tc::idesc_bf16(128, IN, true, true);
 
   uint32_t phase = 0;
-  uint32_t wacc = 0;  // the first tile's dW1 product starts the accumulators
-  int left = kFlush ? flush_interval(ctrl, flushes) : 0;   // tiles until the accumulators are added to memory
+  uint32_t wacc = 0;  // a stretch's first dW1 product starts the accumulators
   float dwacc[4] = {0.f, 0.f, 0.f, 0.f};  // w_out gradient, column 16c + (lane >> 1) of chunk c
   uint4 xn[IN / 8];                       // the stored row of this thread's sample (prefetched a tile ahead)
   bool pre_ok = false;
@@ -878,183 +868,193 @@ bwd_lean_kernel(GridDev grid, const __half* __restrict__ table, const float* __r
     tc::fence_after();
     return true;
   };
-  while (true) {
-    const bool active = next_chunk(cur, recs, ctrl + 1, slot, a, by_pixel, lane, lo, hi, order, n_valid, offs, xrows);
-    if (!__syncthreads_or(active)) break;
-    const int i = cur.base + lane;
-    float p[4] = {0.f, 0.f, 0.f, 0.f};
-    bool valid = false;
-    if (active && i < cur.rec.count) valid = sample_point(cur.rec, i, p);
-    if (D == 4) p[3] = a.t;
-    if (cur.xrow >= 0) {  // stored rows (warp-uniform branch)
-      const uint4* src = xstore + (size_t)(cur.xrow + i) * (IN / 8);
-      if (!pre_ok && valid) {
-#pragma unroll
-        for (int j = 0; j < IN / 8; ++j) xn[j] = __ldcs(src + j);
+  // a stretch: the tiles whose weight gradients stay in the accumulators.  A loop of its
+  // own: 262,144 rays x 512 samples 9.72 ms a step, 10.0 without stretches inside a
+  // launch; 32,764 x 384 in four stretches 1.01 ms, 1.10 with the adds inside the tile
+  // loop (registers).
+  bool done = false;
+  do {
+    int left = stretch_tiles(ctrl[9], stretches, gridDim.x);
+    while (true) {
+      const bool active = next_chunk(cur, recs, ctrl + 1, slot, a, by_pixel, lane, lo, hi, order, n_valid, offs, xrows);
+      if (!__syncthreads_or(active)) {
+        done = true;
+        break;
       }
+      const int i = cur.base + lane;
+      float p[4] = {0.f, 0.f, 0.f, 0.f};
+      bool valid = false;
+      if (active && i < cur.rec.count) valid = sample_point(cur.rec, i, p);
+      if (D == 4) p[3] = a.t;
+      if (cur.xrow >= 0) {  // stored rows (warp-uniform branch)
+        const uint4* src = xstore + (size_t)(cur.xrow + i) * (IN / 8);
+        if (!pre_ok && valid) {
 #pragma unroll
-      for (int j = 0; j < IN / 8; ++j) tc::st_chunk_raw(sX, t, j, valid ? xn[j] : make_uint4(0u, 0u, 0u, 0u));
-      pre_ok = cur.base + 32 < cur.rec.count;
-      if (pre_ok && i + 32 < cur.rec.count) {
+          for (int j = 0; j < IN / 8; ++j) xn[j] = __ldcs(src + j);
+        }
 #pragma unroll
-        for (int j = 0; j < IN / 8; ++j) xn[j] = __ldcs(src + 32 * (IN / 8) + j);
+        for (int j = 0; j < IN / 8; ++j) tc::st_chunk_raw(sX, t, j, valid ? xn[j] : make_uint4(0u, 0u, 0u, 0u));
+        pre_ok = cur.base + 32 < cur.rec.count;
+        if (pre_ok && i + 32 < cur.rec.count) {
+#pragma unroll
+          for (int j = 0; j < IN / 8; ++j) xn[j] = __ldcs(src + 32 * (IN / 8) + j);
+        }
+      } else {
+        pre_ok = false;
+        encode_row<D, F, 16>(grid, table, p, valid, sX, t);
       }
-    } else {
-      pre_ok = false;
-      encode_row<D, F, 16>(grid, table, p, valid, sX, t);
-    }
-    // layer 0: h1 = X W0^T
-    bool ok = run_phase([&] {
+      // layer 0: h1 = X W0^T
+      bool ok = run_phase([&] {
 #pragma unroll
-      for (int q = 0; q < IN / 16; ++q) tc::mma(tm, tc::desc_k(sX_a, q), tc::desc_k(sW_a, q), id_fwd, q > 0);
-    });
-    if (!ok) {
-      timed_out = true;
-      break;
-    }
-    uint32_t m1lo = 0, m1hi = 0;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float h[16];
-      tc::tmem_ld16(my_lanes + 16 * c, h);
-      tc::tmem_wait_ld();
-      float v[8], u[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        v[q] = hidden_act(h[q], act);
-        u[q] = hidden_act(h[8 + q], act);
+        for (int q = 0; q < IN / 16; ++q) tc::mma(tm, tc::desc_k(sX_a, q), tc::desc_k(sW_a, q), id_fwd, q > 0);
+      });
+      if (!ok) {
+        timed_out = true;
+        break;
       }
+      uint32_t m1lo = 0, m1hi = 0;
 #pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const uint32_t bit = h[q] > 0.f ? 1u : 0u;
-        const int col = 16 * c + q;
-        if (col < 32) m1lo |= bit << col; else m1hi |= bit << (col - 32);
-      }
-      tc::st_chunk_bf16(sA, t, 2 * c, v);
-      tc::st_chunk_bf16(sA, t, 2 * c + 1, u);
-    }
-    // layer 1: h2 = A1 W1^T
-    ok = run_phase([&] {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) tc::mma(tm, tc::desc_k(sA_a, q), tc::desc_k(sW_a + kWTile, q), id_fwd, q > 0);
-    });
-    if (!ok) {
-      timed_out = true;
-      break;
-    }
-    float z = 0.f;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float h[16];
-      tc::tmem_ld16(my_lanes + 16 * c, h);
-      tc::tmem_wait_ld();
-#pragma unroll
-      for (int q = 0; q < 16; ++q) z = fmaf(sWout[16 * c + q], hidden_act(h[q], act), z);
-    }
-    const float dz = valid ? cur.rec.gsig * act_grad_z(z, out_act) : 0.f;
-    // second pass over h2: the w_out gradient and G2 = dz * w_out * 1[h2 > 0]
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float h[16];
-      tc::tmem_ld16(my_lanes + 16 * c, h);
-      tc::tmem_wait_ld();
-      float v[16], g[16];
-#pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        v[q] = dz * hidden_act(h[q], act);
-        g[q] = hidden_grad(dz * sWout[16 * c + q], h[q] > 0.f, act);
-      }
-      tc::st_chunk_bf16(sG, t, 2 * c, g);
-      tc::st_chunk_bf16(sG, t, 2 * c + 1, g + 8);
-      float r8[8], r4[4], r2[2], r1[1];
-      detail::rs_step<8>(v, r8, lane, 16);
-      detail::rs_step<4>(r8, r4, lane, 8);
-      detail::rs_step<2>(r4, r2, lane, 4);
-      detail::rs_step<1>(r2, r1, lane, 2);
-      dwacc[c] += r1[0] + __shfl_xor_sync(0xffffffffu, r1[0], 1);
-    }
-    // dA1 = G2 W1 (transient); dW1 += [G2; 0]^T A1 (lanes 0..63 of [64, 128))
-    ok = run_phase([&] {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) tc::mma(tm, tc::desc_k(sG_a, q), tc::desc_mn(sW_a + kWTile, q, kWTile), id_dA, q > 0);
-#pragma unroll
-      for (int q = 0; q < 8; ++q)  // second M block: the zero block, for every K step
-        tc::mma(tm + 64, tc::desc_mn(sG_a, q, sZ_a - (sG_a + 2048u * q)), tc::desc_mn(sA_a, q, kTile), id_dW,
-                (q > 0) | wacc);
-    });
-    if (!ok) {
-      timed_out = true;
-      break;
-    }
-    wacc = 1;
-    // G1 = dA1 * 1[h1 > 0] replaces A1
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float h[16];
-      tc::tmem_ld16(my_lanes + 16 * c, h);
-      tc::tmem_wait_ld();
-#pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const int col = 16 * c + q;
-        const uint32_t bit = col < 32 ? (m1lo >> col) & 1u : (m1hi >> (col - 32)) & 1u;
-        h[q] = hidden_grad(h[q], bit != 0, act);
-      }
-      tc::st_chunk_bf16(sA, t, 2 * c, h);
-      tc::st_chunk_bf16(sA, t, 2 * c + 1, h + 8);
-    }
-    // dX = G1 W0 (transient); dW0 += [0; G1]^T X (lanes 64..127 of [64, 64 + IN))
-    ok = run_phase([&] {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) tc::mma(tm, tc::desc_k(sA_a, q), tc::desc_mn(sW_a, q, kWTile), id_dX, q > 0);
-#pragma unroll
-      for (int q = 0; q < 8; ++q)  // first M block: the zero block; second: K step q of G1
-        tc::mma(tm + 64, tc::desc_sw128(sZ_a, sA_a + 2048u * q - sZ_a, 1024u), tc::desc_mn(sX_a, q, kTile), id_dW0,
-                1u);
-    });
-    if (!ok) {
-      timed_out = true;
-      break;
-    }
-    {
-      float* dst = stage + ((int64_t)(cur.sched - lo) * ray_slots(a.S) + i) * F;
-#pragma unroll
-      for (int c = 0; c < IN / 16; ++c) {
-        float dx[16];
-        tc::tmem_ld16(my_lanes + 16 * c, dx);  // warp-collective: every lane loads
+      for (int c = 0; c < 4; ++c) {
+        float h[16];
+        tc::tmem_ld16(my_lanes + 16 * c, h);
         tc::tmem_wait_ld();
-        if (valid) {
+        float v[8], u[8];
 #pragma unroll
-          for (int k = 0; k < 16 / F; ++k) {
-            const int l = c * (16 / F) + k;  // level
-            if constexpr (F == 2)
-              __stcs(reinterpret_cast<float2*>(dst + l * slots * F), make_float2(dx[2 * k], dx[2 * k + 1]));
-            else
-              __stcs(reinterpret_cast<float4*>(dst + l * slots * F),
-                     make_float4(dx[4 * k], dx[4 * k + 1], dx[4 * k + 2], dx[4 * k + 3]));
+        for (int q = 0; q < 8; ++q) {
+          v[q] = hidden_act(h[q], act);
+          u[q] = hidden_act(h[8 + q], act);
+        }
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          const uint32_t bit = h[q] > 0.f ? 1u : 0u;
+          const int col = 16 * c + q;
+          if (col < 32) m1lo |= bit << col; else m1hi |= bit << (col - 32);
+        }
+        tc::st_chunk_bf16(sA, t, 2 * c, v);
+        tc::st_chunk_bf16(sA, t, 2 * c + 1, u);
+      }
+      // layer 1: h2 = A1 W1^T
+      ok = run_phase([&] {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) tc::mma(tm, tc::desc_k(sA_a, q), tc::desc_k(sW_a + kWTile, q), id_fwd, q > 0);
+      });
+      if (!ok) {
+        timed_out = true;
+        break;
+      }
+      float z = 0.f;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        float h[16];
+        tc::tmem_ld16(my_lanes + 16 * c, h);
+        tc::tmem_wait_ld();
+#pragma unroll
+        for (int q = 0; q < 16; ++q) z = fmaf(sWout[16 * c + q], hidden_act(h[q], act), z);
+      }
+      const float dz = valid ? cur.rec.gsig * act_grad_z(z, out_act) : 0.f;
+      // second pass over h2: the w_out gradient and G2 = dz * w_out * 1[h2 > 0]
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        float h[16];
+        tc::tmem_ld16(my_lanes + 16 * c, h);
+        tc::tmem_wait_ld();
+        float v[16], g[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          v[q] = dz * hidden_act(h[q], act);
+          g[q] = hidden_grad(dz * sWout[16 * c + q], h[q] > 0.f, act);
+        }
+        tc::st_chunk_bf16(sG, t, 2 * c, g);
+        tc::st_chunk_bf16(sG, t, 2 * c + 1, g + 8);
+        float r8[8], r4[4], r2[2], r1[1];
+        detail::rs_step<8>(v, r8, lane, 16);
+        detail::rs_step<4>(r8, r4, lane, 8);
+        detail::rs_step<2>(r4, r2, lane, 4);
+        detail::rs_step<1>(r2, r1, lane, 2);
+        dwacc[c] += r1[0] + __shfl_xor_sync(0xffffffffu, r1[0], 1);
+      }
+      // dA1 = G2 W1 (transient); dW1 += [G2; 0]^T A1 (lanes 0..63 of [64, 128))
+      ok = run_phase([&] {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          tc::mma(tm, tc::desc_k(sG_a, q), tc::desc_mn(sW_a + kWTile, q, kWTile), id_dA, q > 0);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)  // second M block: the zero block, for every K step
+          tc::mma(tm + 64, tc::desc_mn(sG_a, q, sZ_a - (sG_a + 2048u * q)), tc::desc_mn(sA_a, q, kTile), id_dW,
+                  (q > 0) | wacc);
+      });
+      if (!ok) {
+        timed_out = true;
+        break;
+      }
+      wacc = 1;
+      // G1 = dA1 * 1[h1 > 0] replaces A1
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        float h[16];
+        tc::tmem_ld16(my_lanes + 16 * c, h);
+        tc::tmem_wait_ld();
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          const int col = 16 * c + q;
+          const uint32_t bit = col < 32 ? (m1lo >> col) & 1u : (m1hi >> (col - 32)) & 1u;
+          h[q] = hidden_grad(h[q], bit != 0, act);
+        }
+        tc::st_chunk_bf16(sA, t, 2 * c, h);
+        tc::st_chunk_bf16(sA, t, 2 * c + 1, h + 8);
+      }
+      // dX = G1 W0 (transient); dW0 += [0; G1]^T X (lanes 64..127 of [64, 64 + IN))
+      ok = run_phase([&] {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) tc::mma(tm, tc::desc_k(sA_a, q), tc::desc_mn(sW_a, q, kWTile), id_dX, q > 0);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)  // first M block: the zero block; second: K step q of G1
+          tc::mma(tm + 64, tc::desc_sw128(sZ_a, sA_a + 2048u * q - sZ_a, 1024u), tc::desc_mn(sX_a, q, kTile), id_dW0,
+                  1u);
+      });
+      if (!ok) {
+        timed_out = true;
+        break;
+      }
+      {
+        float* dst = stage + ((int64_t)(cur.sched - lo) * ray_slots(a.S) + i) * F;
+#pragma unroll
+        for (int c = 0; c < IN / 16; ++c) {
+          float dx[16];
+          tc::tmem_ld16(my_lanes + 16 * c, dx);  // warp-collective: every lane loads
+          tc::tmem_wait_ld();
+          if (valid) {
+#pragma unroll
+            for (int k = 0; k < 16 / F; ++k) {
+              const int l = c * (16 / F) + k;  // level
+              if constexpr (F == 2)
+                __stcs(reinterpret_cast<float2*>(dst + l * slots * F), make_float2(dx[2 * k], dx[2 * k + 1]));
+              else
+                __stcs(reinterpret_cast<float4*>(dst + l * slots * F),
+                       make_float4(dx[4 * k], dx[4 * k + 1], dx[4 * k + 2], dx[4 * k + 3]));
+            }
           }
         }
       }
-    }
-    tc::fence_before();
-    __syncthreads();
-    if (active) cur.base += 32;
-    if (kFlush && --left == 0) {   // block-uniform
-      flush();
       tc::fence_before();
       __syncthreads();
-      left = flush_interval(ctrl, flushes);
-      wacc = 0;
+      if (active) cur.base += 32;
+      if (--left == 0) break;   // block-uniform
     }
-  }
+    if (timed_out) break;
+    if (wacc) flush();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (!(lane & 1)) red[warp * 64 + 16 * c + (lane >> 1)] += dwacc[c];   // (this lane's own)
+      dwacc[c] = 0.f;
+    }
+    wacc = 0;
+    tc::fence_before();
+    __syncthreads();
+  } while (!done);
   if (timed_out) {
     if (t == 0) atomicOr(err, 2u);
     tc::mbar_wait(bar, phase);  // let the MMAs in flight retire (bounded) before freeing TMEM
-  } else if (wacc) {
-    flush();
-  }
-  if (!(lane & 1)) {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) red[warp * 64 + 16 * c + (lane >> 1)] = dwacc[c];
   }
   tc::fence_before();
   __syncthreads();
@@ -1371,7 +1371,7 @@ int run_mixed(const NectbGeometry& geo, const GridDev& grid, const __half* table
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem);
     ProfScope ps(kProfBackward, s);
     k<<<blocks, kMixThreads, bsmem, s>>>(gt, table, W, a, ws.rays, ws.slot, ws.counters, out_act, table_grad,
-                                         W_grad, 0, 0x7fffffff, nullptr, 0, nullptr, nullptr, nullptr, 0u, 1.f);
+                                         W_grad, 0, 0x7fffffff, nullptr, 0, nullptr, nullptr, nullptr, 0u, 1);
     return launch_status("bwd_mixed_kernel");
   }
   // the order is a function of the prepared rays alone: computed again unless
@@ -1403,37 +1403,28 @@ int run_mixed(const NectbGeometry& geo, const GridDev& grid, const __half* table
   constexpr bool kLean = H == 2 && L == 16 && IN <= 64;
   const size_t lsmem = 1024 + 2 * kWTile + 3 * kTile + 2048 + 64 * 4 + 64 + 4 * 64 * 4;
   const int lblocks = std::max(1, std::min<int>(tune.backward_blocks_per_sm * sms, (int)ceil_div(a.num_rays, 4)));
-  // (the lean kernel without the adding inside: it costs 3 % in spilled registers)
-  if constexpr (kLean) {
-    set_smem(bwd_lean_kernel<D, F, ACT, true>, lsmem, false);
-    set_smem(bwd_lean_kernel<D, F, ACT, false>, lsmem, false);
-  } else
+  if constexpr (kLean)
+    set_smem(bwd_lean_kernel<D, F, ACT>, lsmem, false);
+  else
     cudaFuncSetAttribute(bwd_mixed_kernel<D, F, L, H, true, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)bsmem);
   auto ks = scatter_stage_kernel<D, F>;
   const int segs = (int)ceil_div(a.S, kScatterSegment);
   const int64_t slots = per_round * ray_slots(a.S);
-  // the weight gradients leave the accumulators once per R / staged_rounds rays: at
-  // a launch's end when the rounds are that small, else inside it (flush_interval)
-  const float flushes = per_round * tune.staged_rounds < 2 * (int64_t)R ? 1.f : (float)tune.staged_rounds;
+  const int stretches = accumulator_stretches(R, per_round, tune.staged_rounds);
   for (int64_t lo = 0; lo < R; lo += per_round) {
     const int hi = (int)std::min<int64_t>(R, lo + per_round);
     if (int rc = cuda_status(cudaMemsetAsync(ws.counters + 1, 0, sizeof(unsigned int), s), "memset cursor")) return rc;
     {
       ProfScope ps(kProfBackward, s);
-      if constexpr (kLean) {
-        auto lean = [&](auto k) {
-          k<<<lblocks, kMixThreads, lsmem, s>>>(gt, table, W, a, ws.rays, ws.slot, ws.counters, out_act, W_grad, (int)lo,
-                                                hi, stage, slots, order, SL.offs, SL.xstore, SL.xcap, flushes);
-        };
-        if (flushes > 1.f)
-          lean(bwd_lean_kernel<D, F, ACT, true>);
-        else
-          lean(bwd_lean_kernel<D, F, ACT, false>);
-      } else
+      if constexpr (kLean)
+        bwd_lean_kernel<D, F, ACT><<<lblocks, kMixThreads, lsmem, s>>>(
+            gt, table, W, a, ws.rays, ws.slot, ws.counters, out_act, W_grad, (int)lo, hi, stage, slots, order, SL.offs,
+            SL.xstore, SL.xcap, stretches);
+      else
         bwd_mixed_kernel<D, F, L, H, true, ACT><<<blocks, kMixThreads, bsmem, s>>>(
             gt, table, W, a, ws.rays, ws.slot, ws.counters, out_act, table_grad, W_grad, (int)lo, hi, stage, slots,
-            order, SL.offs, SL.xstore, SL.xcap, flushes);
+            order, SL.offs, SL.xstore, SL.xcap, stretches);
     }
     if (int rc = launch_status("bwd_mixed_kernel")) return rc;
     {

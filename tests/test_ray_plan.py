@@ -1,6 +1,7 @@
 """The scheduling order of a batch's rays and the split of its workspace
 (csrc/ray_plan.cuh), compiled for the CPU: every slot exactly once, whatever part of the
-detector the pixels are; the stored rows a workspace of a given size keeps."""
+detector the pixels are; the stored rows a workspace of a given size keeps; how long the
+weight gradients stay in the tensor cores' accumulators."""
 import ctypes
 import shutil
 import subprocess
@@ -17,6 +18,8 @@ extern "C" int64_t order(int R, int P) { return (int64_t)order_bytes(R, P); }
 extern "C" int64_t recommended(int R, int rounds, int64_t per_ray) {
   return (int64_t)staged_round_bytes(R, rounds, (size_t)per_ray);
 }
+extern "C" int stretches(int64_t R, int64_t per_round, int rounds) { return accumulator_stretches(R, per_round, rounds); }
+extern "C" int tiles(unsigned int chunks, int n, int blocks) { return stretch_tiles(chunks, n, blocks); }
 // rows of the store, rays of a round; every part of the region inside it, in order
 extern "C" int layout(int64_t at, int64_t bytes, int R, int P, int S, int64_t row, int64_t per_ray, int rounds,
                       int64_t* rows, int64_t* per_round) {
@@ -48,6 +51,7 @@ def plan(tmp_path_factory):
     i64, i32 = ctypes.c_int64, ctypes.c_int
     lib.order.restype = lib.recommended.restype = i64
     lib.recommended.argtypes = [i32, i32, i64]
+    lib.stretches.argtypes = [i64, i64, i32]
     lib.layout.argtypes = [i64, i64, i32, i32, i32, i64, i64, i32, ctypes.POINTER(i64), ctypes.POINTER(i64)]
     return lib
 
@@ -105,3 +109,25 @@ def test_rows_come_before_large_rounds(plan, R, S, features, rounds):
         if per_round:   # (the fused single pass below 64 rounds)
             assert rows == want
             assert per_round >= (least // per_ray if rows else 1)
+
+
+@pytest.mark.parametrize("R", [1, 5, 16, 4882, 50000, 262144])
+@pytest.mark.parametrize("rounds", [1, 3, 4, 16, 64])
+@pytest.mark.parametrize("launches", range(1, 17))
+def test_accumulators_hold_no_more_than_a_round(plan, R, rounds, launches):
+    """However many launches a batch takes, the accumulators hold at most R / `rounds` rays."""
+    per_round = -(-R // launches)
+    n = plan.stretches(R, per_round, rounds)
+    longest = per_round if n == 1 else min(per_round, -(-R // n))
+    assert longest <= -(-R // rounds)
+
+
+@pytest.mark.parametrize("chunks,stretches,blocks", [(0, 4, 444), (7, 4, 444), (525_000, 4, 444), (2**32 - 1, 2, 1),
+                                                     (525_000, 64, 148), (525_000, 1, 148)])
+def test_tiles_of_a_stretch(plan, chunks, stretches, blocks):
+    """The blocks' stretches add up to a share of the batch's tiles, rounded up to a whole tile a block."""
+    tiles = plan.tiles(chunks, stretches, blocks)
+    if stretches == 1:
+        assert tiles == 2**31 - 1
+    else:
+        assert tiles == max(1, -(-chunks // (4 * stretches * blocks)))
