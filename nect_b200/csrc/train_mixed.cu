@@ -436,6 +436,22 @@ column_sum_kernel(TrainArgs a, RayRec* __restrict__ recs, const int32_t* __restr
   }
 }
 
+// Adds a thread's N consecutive values to fp32 memory, four to a reduction where dst is
+// 16-byte aligned (`vec`).  A stretch of a small batch ends after a few tiles, and its
+// adds, all blocks' to the same 25 KB, are bound by the L2's reduction requests: 24,999
+// rays x 100 samples 357 -> 272 us for the backward, 2,000 x 100 258 -> 83 us.
+template <int N>
+__device__ __forceinline__ void add_row(float* dst, const float* v, bool vec) {
+  if (vec) {
+#pragma unroll
+    for (int j = 0; j < N; j += 4)
+      atomicAdd(reinterpret_cast<float4*>(dst + j), make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; ++j) atomicAdd(dst + j, v[j]);
+  }
+}
+
 // Staged mode (kStaged): instead of scattering, dL/d(encoding) of every sample
 // is written to the staging buffer, level-major: stage[(l * slots + s) * F + f]
 // with s = (scheduling index - lo) * ray_slots(S) + sample, for the rays whose
@@ -522,6 +538,7 @@ bwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
   // Adds the weight gradients to fp32 memory: TMEM lanes 0..63 (warps 0 and 1) hold rows o = 0..63.
   auto flush = [&]() {
     tc::fence_after();
+    const bool vec = (reinterpret_cast<uintptr_t>(W_grad) & 15u) == 0;
     if (warp < 2) {
       const int o = t;
 #pragma unroll 1
@@ -529,8 +546,7 @@ bwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
         float v[64];
         ld64(my_lanes + Plan::T + 64 * (k - 1), v);
         float* dst = W_grad + 64 * IN + (k - 1) * 64 * 64 + o * 64;
-#pragma unroll
-        for (int i2 = 0; i2 < 64; ++i2) atomicAdd(dst + i2, v[i2]);
+        add_row<64>(dst, v, vec);
       }
     }
     if constexpr (KT == 1) {
@@ -540,8 +556,7 @@ bwd_mixed_kernel(GridDev grid, const __half* __restrict__ table, const float* __
 #pragma unroll
         for (int c = 0; c < S::INP / 16; ++c) tc::tmem_ld16(dw0 + ((uint32_t)(32 * warp) << 16) + 16 * c, w0 + 16 * c);
         tc::tmem_wait_ld();
-#pragma unroll
-        for (int i2 = 0; i2 < IN; ++i2) atomicAdd(W_grad + o * IN + i2, w0[i2]);
+        add_row<IN>(W_grad + o * IN, w0, vec);
       }
     } else if (32 * warp < IN) {  // dW0^T: lane i holds input i's 64 output columns
       float v[64];
@@ -837,20 +852,19 @@ bwd_lean_kernel(GridDev grid, const __half* __restrict__ table, const float* __r
   // Adds the weight gradients to fp32 memory.
   auto flush = [&]() {
     tc::fence_after();
+    const bool vec = (reinterpret_cast<uintptr_t>(W_grad) & 15u) == 0;
     if (warp < 2) {  // dW1 rows o = t in lanes 0..63
       float v[64];
       ld64(my_lanes + 64, v);
       float* dst = W_grad + 64 * IN + t * 64;
-#pragma unroll
-      for (int j = 0; j < 64; ++j) atomicAdd(dst + j, v[j]);
+      add_row<64>(dst, v, vec);
     } else {  // dW0 rows o = t - 64 in lanes 64..127
       float v[IN];
 #pragma unroll
       for (int c = 0; c < IN / 16; ++c) tc::tmem_ld16(my_lanes + 64 + 16 * c, v + 16 * c);
       tc::tmem_wait_ld();
       float* dst = W_grad + (t - 64) * IN;
-#pragma unroll
-      for (int j = 0; j < IN; ++j) atomicAdd(dst + j, v[j]);
+      add_row<IN>(dst, v, vec);
     }
   };
   auto run_phase = [&](auto issue) -> bool {
