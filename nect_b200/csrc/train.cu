@@ -230,6 +230,7 @@ int train_entry(const NectbGeometry* geometry, const NectbHashGrid* grid, const 
   a.perm_len = batch->random_ray_index_len;
   a.start = batch->starting_ray_index;
   a.num_rays = n_batch * sub;
+  a.claim = slots_per_claim(a.num_rays, a.n_pixels);
   a.S = batch->num_points_per_ray;
   a.angle = batch->angle_rad;
   a.t = batch->t;

@@ -40,6 +40,7 @@ struct TrainArgs {
   // a re-projection (a whole view or any range of its pixels): no backward follows, so
   // no ray order is made and no rows are stored, whatever the workspace holds
   bool query = false;
+  int claim = 1;   // slots a warp claims at a time (slots_per_claim)
   int S;
   float angle;
   float t;
@@ -187,25 +188,35 @@ __device__ __forceinline__ RayRec load_ray(const RayRec* recs, int r) { return r
 // in detector-pixel order (neighbouring rays run together, so the blocks in
 // flight touch a compact part of the tables and the L2 keeps it), or in batch
 // order when the batch repeats a pixel.  Returns -1 when none are left.
-// The scheduling index (pixel, or batch position) of the returned ray is
-// written to *sched; only indices in [lo, hi) are handed out (a round of the
-// staged backward), the cursor counting from lo.
-__device__ __forceinline__ int next_ray(unsigned int* cursor, const int32_t* __restrict__ slot,
-                                        const RayRec* __restrict__ recs, int R, int P, bool by_pixel, int lane,
-                                        int lo = 0, int hi = 0x7fffffff, int* sched = nullptr) {
-  const unsigned int end = (unsigned)min(hi, by_pixel ? P : R);
+// A claim of one slot costs an atomic on one address, which bound batches of very few
+// rays; in pixel order a warp then claims several neighbouring slots at a time
+// (slots_per_claim) and is handed their rays one after the other.
+struct SlotClaim {
+  int ray = -1;            // of this lane's slot of the claim
+  unsigned int left = 0;   // lanes whose rays have not been handed out
+};
+__device__ __forceinline__ int next_ray(SlotClaim& claim, unsigned int* cursor, const int32_t* __restrict__ slot,
+                                        const RayRec* __restrict__ recs, const TrainArgs& a, bool by_pixel,
+                                        int lane) {
+  while (by_pixel && claim.left == 0) {
+    unsigned int at = 0;
+    if (lane == 0) at = atomicAdd(cursor, (unsigned)a.claim);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (at >= (unsigned)a.n_pixels) return -1;
+    claim.ray = lane < a.claim && at + lane < (unsigned)a.n_pixels ? slot[at + lane] : -1;
+    claim.left = __ballot_sync(0xffffffffu, claim.ray >= 0);
+  }
+  if (by_pixel) {
+    const int from = __ffs(claim.left) - 1;
+    claim.left &= claim.left - 1;
+    return __shfl_sync(0xffffffffu, claim.ray, from);
+  }
   while (true) {
     unsigned int idx = 0;
-    if (lane == 0) idx = (unsigned)lo + atomicAdd(cursor, 1u);
+    if (lane == 0) idx = atomicAdd(cursor, 1u);
     idx = __shfl_sync(0xffffffffu, idx, 0);
-    if (idx >= end) return -1;
-    if (sched) *sched = (int)idx;
-    if (by_pixel) {
-      const int r = slot[idx];
-      if (r >= 0) return r;
-    } else {
-      if (recs[idx].count > 0) return (int)idx;
-    }
+    if (idx >= (unsigned)a.num_rays) return -1;
+    if (recs[idx].count > 0) return (int)idx;
   }
 }
 

@@ -51,7 +51,8 @@ constexpr int kColumnSegment = 32;   // samples of a column unit of the forward
 struct RayCursor {
   int ray = -1;
   int base = 0;
-  int sched = 0;      // scheduling index (detector pixel, or batch position; rank with an order) of the ray
+  int sched = 0;      // rank of the ray (with an order)
+  SlotClaim claim;    // (without one)
   int64_t xrow = -1;  // encoding-store row of the ray's sample 0, -1 if its rows are not stored
   RayRec rec;
 };
@@ -60,7 +61,7 @@ struct RayCursor {
 // scheduler when the current one is done).  Returns false when no rays are
 // left.  Rays without samples were finalised by the preparation kernel.
 // With ``order`` the rays come from the ordered list, ranks [lo, hi) (one
-// round of the two-pass backward), else from the scheduling indices [lo, hi).
+// round of the two-pass backward), else from the slots.
 // With ``offs`` a ray whose rows all lie below xcap gets its store row.
 __device__ __forceinline__ bool next_chunk(RayCursor& cur, const RayRec* recs, unsigned int* cursor,
                                            const int32_t* slot, const TrainArgs& a, bool by_pixel, int lane,
@@ -70,7 +71,7 @@ __device__ __forceinline__ bool next_chunk(RayCursor& cur, const RayRec* recs, u
   if (cur.ray >= a.num_rays) return false;
   if (cur.ray >= 0 && cur.base < cur.rec.count) return true;
   const int r = order ? next_ray_ranked(cursor, order, n_valid, lo, hi, lane, &cur.sched)
-                      : next_ray(cursor, slot, recs, a.num_rays, a.n_pixels, by_pixel, lane, lo, hi, &cur.sched);
+                      : next_ray(cur.claim, cursor, slot, recs, a, by_pixel, lane);
   if (r < 0) {
     cur.ray = a.num_rays;
     cur.rec.count = 0;

@@ -229,13 +229,14 @@ fwd_plain_kernel(GridDev grid, const float* __restrict__ table, const float* __r
   const bool owner = t < NT;   // the first NT threads hold the tile's samples, a warp 32 of one ray
   float loss_acc = 0.f, sum = 0.f;
   int ray = -1, base = 0;
+  SlotClaim claim;
   RayRec rec;
   rec.count = 0;
   while (true) {
     bool valid = false;
     if (owner) {
       if (ray < a.num_rays && (ray < 0 || base >= rec.count)) {
-        const int r = next_ray(ctrl, slot, recs, a.num_rays, a.n_pixels, by_pixel, lane);
+        const int r = next_ray(claim, ctrl, slot, recs, a, by_pixel, lane);
         if (r < 0) {
           ray = a.num_rays;
           rec.count = 0;
@@ -464,6 +465,7 @@ bwd_plain_kernel(GridDev grid, const float* __restrict__ table, const float* __r
   extern __shared__ float4 smem4[];
   const int t = threadIdx.x, lane = t & 31;
   int ray = -1, base = 0;
+  SlotClaim claim;
   RayRec rec;
   rec.count = 0;
   rec.gsig = 0.f;
@@ -473,7 +475,7 @@ bwd_plain_kernel(GridDev grid, const float* __restrict__ table, const float* __r
         bool active = false;
         if (t < NT) {
           if (ray < a.num_rays && (ray < 0 || base >= rec.count)) {
-            const int r = next_ray(ctrl + 1, slot, recs, a.num_rays, a.n_pixels, by_pixel, lane);
+            const int r = next_ray(claim, ctrl + 1, slot, recs, a, by_pixel, lane);
             if (r < 0) {
               ray = a.num_rays;
               rec.count = 0;

@@ -18,6 +18,7 @@ extern "C" int64_t order(int R, int P) { return (int64_t)order_bytes(R, P); }
 extern "C" int64_t recommended(int R, int rounds, int64_t per_ray) {
   return (int64_t)staged_round_bytes(R, rounds, (size_t)per_ray);
 }
+extern "C" int claim(int R, int P) { return slots_per_claim(R, P); }
 extern "C" int stretches(int64_t R, int64_t per_round, int rounds) { return accumulator_stretches(R, per_round, rounds); }
 extern "C" int tiles(unsigned int chunks, int n, int blocks) { return stretch_tiles(chunks, n, blocks); }
 // rows of the store, rays of a round; every part of the region inside it, in order
@@ -131,3 +132,9 @@ def test_tiles_of_a_stretch(plan, chunks, stretches, blocks):
         assert tiles == 2**31 - 1
     else:
         assert tiles == max(1, -(-chunks // (4 * stretches * blocks)))
+
+
+@pytest.mark.parametrize("R,P,want", [(1, 1, 1), (1, 64, 1), (1, 128, 2), (1, 65536, 32), (256, 65536, 4),
+                                      (2000, 65536, 1), (65536, 65536, 1), (1, 2**31 - 1, 32), (0, 65536, 32)])
+def test_claims(plan, R, P, want):
+    assert plan.claim(R, P) == want
