@@ -1235,7 +1235,14 @@ int run_mixed(const NectbGeometry& geo, const GridDev& grid, const __half* table
     // the start of its staging region, and runs without staging.
     const bool piece = args.fwd_warpgroups > 0 && !table_grad;
     const size_t sb = piece ? slice_half_bytes(grid) : slice_bytes(grid);
-    const size_t need = piece ? sb + 512 : sb + order_bytes(args.num_rays, args.n_pixels) + (size_t(1) << 20);
+    // Beside the slice a step needs a round's room: 16,000 rays x 64 samples, 16 x 2 levels, in 80 MB
+    // take 41 rounds and 2.74 ms on the slice, 4 rounds and 1.19 ms on the 4D grid; 2,000 x 100 in
+    // 80 MB 8 rounds and 0.80 ms, 1 round and 0.34 ms.
+    const size_t rounds =
+        round_bytes(args.num_rays, tune.staged_rounds, (size_t)ray_slots(args.S) * L * F * sizeof(float));
+    const size_t need = piece ? sb + 512
+                              : sb + order_bytes(args.num_rays, args.n_pixels) +
+                                    std::max(size_t(1) << 20, args.query ? 0 : rounds);
     if (tune.time_slice && args.max_blocks == 0 && ws.stage && ws.stage_bytes >= need) {
       const TimeSlice ts = make_time_slice(grid, args.t);
       const int64_t n3 = ts.g3.total_entries;

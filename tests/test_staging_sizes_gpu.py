@@ -3,10 +3,72 @@ the rays beside a store of every row, of a part of them and of none, against the
 fused pass.  Predictions bit for bit (the same network on the same positions); gradients
 within 1e-5 of the largest entry, the bound of the other staged-against-single-pass tests
 (the same products, other fp32 sums)."""
+import ctypes
+
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+
+
+def test_no_time_slice_without_a_round_beside_it(cuda_device):
+    """A 4D step in a workspace with room for the time slice but not for a quarter of the
+    rays' round beside it works on the 4D grid: the predictions of the unsliced step bit for
+    bit, which the slice's fp16 rounding would change."""
+    from nect_b200 import _lib, autotune
+    from nect_b200.config import HashEncoderConfig, MLPNetConfig
+    from nect_b200.network import HashGrid4D
+    from nect_b200.sampling import Geometry
+    from nect_b200.trainer import RayBatch, Workspace, train_step
+
+    R, S, det = 3000, 65, (80, 96)
+    geo = Geometry(nDetector=list(det), dDetector=[0.8, 0.7], mode="cone", DSD=300.0, DSO=200.0, nVoxel=[32] * 3,
+                   dVoxel=[1.0] * 3)
+    enc = HashEncoderConfig(n_levels=16, n_features_per_level=2, log2_hashmap_size=12, base_resolution=4,
+                            finest_resolution=256, base_resolution_t=2)
+    m = HashGrid4D(enc, MLPNetConfig(n_hidden_layers=2), precision="mixed", device="cuda", seed=0)
+    with torch.no_grad():
+        m.table.normal_(0.0, 0.3, generator=torch.Generator(device="cuda").manual_seed(1))
+        m.refresh_half()
+    cg = geo.get_c_geometry()
+    args = (ctypes.byref(cg.c_struct), ctypes.byref(m.grid_desc), ctypes.byref(m.mlp_desc), R)
+    base = (int(_lib.lib.nectb_train_workspace_bytes(*args)) + 255) // 256 * 256
+    default = autotune.get_tuning()
+
+    def recommended(time_slice):
+        autotune.set_tuning(dict(default, time_slice=time_slice))
+        return int(_lib.lib.nectb_train_staging_bytes(*args, S))
+
+    class Sized(Workspace):
+        def get(self, *a, **k):
+            self.staging = False
+            super().get(*a, **k)
+            if self.buf.numel() < self.size:
+                self.buf = torch.empty(self.size, dtype=torch.uint8, device="cuda")
+            return self.buf.data_ptr(), self.size
+
+    g = torch.Generator(device="cuda").manual_seed(2)
+    P = det[0] * det[1]
+    batch = RayBatch(perm=torch.randperm(P, device="cuda", generator=g), start=0, num_rays=R, points_per_ray=S,
+                     angle=0.7, max_ray_distance_per_point=geo.max_distance_traveled / S,
+                     jitter=torch.rand(R, device="cuda", generator=g) - 0.5,
+                     detector_offset=torch.zeros(R, 2, device="cuda"),
+                     projection=torch.rand(P, device="cuda", generator=g), t=0.3)
+    got = []
+    try:
+        ws = Sized()
+        ws.size = base + recommended(1) - recommended(0) + (2 << 20)   # a quarter's round takes 6.5 MB
+        for time_slice, w in ((1, ws), (0, ws), (1, Workspace())):
+            autotune.set_tuning(dict(default, time_slice=time_slice))
+            tg, mg = torch.zeros_like(m.table), torch.zeros_like(m.mlp)
+            _, y = train_step(m, cg, batch, geo.max_distance_traveled, tg, mg, w, "l2")
+            assert w.error_word() == 0
+            got.append((y, tg))
+    finally:
+        autotune.set_tuning(default)
+    assert torch.equal(got[0][0], got[1][0])
+    assert not torch.equal(got[0][0], got[2][0])   # the slice, where there is room
+    assert float((got[0][1] - got[1][1]).abs().max()) <= 1e-5 * float(got[1][1].abs().max())
 
 
 @pytest.mark.parametrize("dims,F", [(3, 2), (3, 4), (4, 2)])
