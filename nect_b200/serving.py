@@ -118,6 +118,15 @@ def time_slice_bytes(model: _HashGridModel) -> int:
     return int(_lib.lib.nectb_time_slice_bytes(ctypes.byref(model.grid_desc)))
 
 
+def _empty_on(stream: torch.cuda.Stream, n: int, dtype: torch.dtype, device) -> torch.Tensor:
+    """A result of the caller's that ``stream`` writes first: it belongs to that stream (a block
+    of the current one may still be in use there) and outlives its use on the current one."""
+    with torch.cuda.stream(stream):
+        t = torch.empty(n, dtype=dtype, device=device)
+    t.record_stream(torch.cuda.current_stream())
+    return t
+
+
 def time_slice(model: _HashGridModel, t: float, out: torch.Tensor | None = None,
                stream: torch.cuda.Stream | None = None) -> torch.Tensor:
     """The model's fp16 table blended at t into a 3D slice (nectb_time_slice):
@@ -125,9 +134,9 @@ def time_slice(model: _HashGridModel, t: float, out: torch.Tensor | None = None,
     n = time_slice_bytes(model)
     if n == 0:
         raise ValueError("the model has no time slice (4D with an fp16 table only)")
-    if out is None:
-        out = torch.empty(n, dtype=torch.uint8, device=model.table.device)
     stream = stream or torch.cuda.current_stream()
+    if out is None:
+        out = _empty_on(stream, n, torch.uint8, model.table.device)
     rc = _lib.lib.nectb_time_slice(ctypes.byref(model.grid_desc), model.grid_table.data_ptr(), float(t),
                                    out.data_ptr(), out.numel() * out.element_size(), stream.cuda_stream)
     _lib.check(rc, "nectb_time_slice")
@@ -199,9 +208,9 @@ def reproject(model: _HashGridModel, geometry, angle: float, t: float = 0.0, poi
     S = points_per_ray or int(math.ceil(1.5 * max(geometry.nDetector)))
     P = geometry.nDetector[0] * geometry.nDetector[1]
     dev = model.table.device
-    if out is None:
-        out = torch.empty(P, device=dev)
     stream = stream or torch.cuda.current_stream()
+    if out is None:
+        out = _empty_on(stream, P, torch.float32, dev)
     if pixels is None and not warpgroups:
         need = _lib.lib.nectb_train_workspace_bytes(ctypes.byref(cg.c_struct), ctypes.byref(model.grid_desc),
                                                     ctypes.byref(model.mlp_desc), P)
@@ -212,10 +221,11 @@ def reproject(model: _HashGridModel, geometry, angle: float, t: float = 0.0, poi
             if model.precision == "mixed" and max_blocks == 0:
                 strip = 4 * 32 * geometry.nDetector[1] * S
                 extra = 256 + min(-(-geometry.nDetector[0] // 32), max(VIEW_SIGMA_BYTES // strip, 1)) * strip
-            try:
-                workspace = torch.empty(need + extra, dtype=torch.uint8, device=dev)
-            except torch.OutOfMemoryError:
-                workspace = torch.empty(need, dtype=torch.uint8, device=dev)
+            with torch.cuda.stream(stream):   # the workspace belongs to the stream that uses it
+                try:
+                    workspace = torch.empty(need + extra, dtype=torch.uint8, device=dev)
+                except torch.OutOfMemoryError:
+                    workspace = torch.empty(need, dtype=torch.uint8, device=dev)
         rc = _lib.lib.nectb_query_reproject(ctypes.byref(cg.c_struct), ctypes.byref(model.grid_desc),
                                             ctypes.byref(model.mlp_desc), model.grid_table.data_ptr(),
                                             model.mlp.data_ptr(), float(angle), float(t), S,
@@ -226,7 +236,9 @@ def reproject(model: _HashGridModel, geometry, angle: float, t: float = 0.0, poi
     else:
         begin, count = pixels or (0, P)
         if workspace is None:
-            workspace = torch.empty(reproject_workspace_bytes(model, geometry, count), dtype=torch.uint8, device=dev)
+            with torch.cuda.stream(stream):
+                workspace = torch.empty(reproject_workspace_bytes(model, geometry, count), dtype=torch.uint8,
+                                        device=dev)
         rc = _lib.lib.nectb_query_reproject_range(
             ctypes.byref(cg.c_struct), ctypes.byref(model.grid_desc), ctypes.byref(model.mlp_desc),
             model.grid_table.data_ptr(), model.mlp.data_ptr(), float(angle), float(t), S,
