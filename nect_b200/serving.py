@@ -156,12 +156,16 @@ def query_points(model: _HashGridModel, items: np.ndarray, stream: torch.cuda.St
     """Evaluate the items (any requests) in one launch (outputs written in place);
     max_blocks > 0 caps the persistent grid, in blocks that leave room on an SM for
     other kernels; 0 takes the whole GPU.  With ``slice`` (time_slice at
-    some t) every item is evaluated on it, at its t."""
+    some t) every item is evaluated on it, at its t.  Not under graph capture: the items
+    are copied from a host buffer of the call."""
     if items.size == 0:
         return
     if stream is not None:   # the buffer belongs to the stream that reads it
         with torch.cuda.stream(stream):
             return query_points(model, items, None, max_blocks, slice)
+    if torch.cuda.is_current_stream_capturing():
+        raise RuntimeError("query_points cannot be captured in a graph: it copies its items from a host buffer "
+                           "that lives as long as the call")
     ch = item_chunks(items)
     ends = np.cumsum(ch)
     # the items (with their chunk offsets), the work cursor and the error word go over in one
