@@ -296,10 +296,10 @@ int nectb_query_points_slice(const NectbHashGrid* grid, const NectbMLP* mlp, con
  * max_blocks > 0 caps the persistent grid of either query (a server keeps
  * SMs free for latency-critical launches on higher-priority streams; a point
  * query then runs one-warpgroup blocks, otherwise one wide block per SM).
- * A workspace with at least num_points_per_ray * 4 bytes per ray of 32
- * detector rows past the required size (from a 256-byte boundary) lets a mixed
- * model's uncapped view run 32 neighbouring rays a warp, as many such strips
- * at a time as fit: the same bits, faster. */
+ * A workspace with room past the required size (from a 256-byte boundary), at
+ * num_points_per_ray * 4 bytes a ray, lets a mixed model's uncapped view run 32
+ * neighbouring rays a warp, as many groups of 32 rays at a time as fit, where those
+ * fill the GPU: the same bits, faster. */
 int nectb_query_reproject(const NectbGeometry* geometry, const NectbHashGrid* grid,
                           const NectbMLP* mlp, const void* grid_params, const float* mlp_params,
                           float angle_rad, float t, int32_t num_points_per_ray,

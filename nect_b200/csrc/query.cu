@@ -520,12 +520,11 @@ int reproject_range(const NectbGeometry* geometry, const NectbHashGrid* grid, co
   a.fwd_warpgroups = max_blocks > 0 ? 0 : warpgroups;
   a.n_cols = geometry->nDetector[1];
   a.query = true;
-  // a whole view with room past the base size: the column form's sigmas, whole strips at a time
+  // a whole view with room past the base size: the column form's sigmas, groups of 32 rays at a time
   const size_t base = align256(workspace_bytes(count, count));
-  const int64_t strip = 32 * (int64_t)a.n_cols;
   if (!stage && max_blocks <= 0 && workspace_size > base) {
     const int64_t fit = (int64_t)((workspace_size - base) / ((size_t)num_points_per_ray * sizeof(float)));
-    a.col_rays = (int)std::min<int64_t>(fit / strip * strip, ceil_div(count, strip) * strip);
+    a.col_rays = (int)(std::min<int64_t>(fit, count + (int64_t)31) / 32 * 32);
     if (a.col_rays > 0) a.col_sigma = reinterpret_cast<float*>(static_cast<char*>(workspace) + base);
   }
   Workspace ws = carve_workspace(workspace, count, count, stage ? workspace_size : 0);

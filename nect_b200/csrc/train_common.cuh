@@ -56,8 +56,8 @@ struct TrainArgs {
   // > 0: the forward runs one block of this many warpgroups per SM under the
   // shared-SM carveout (re-projection pieces beside serving kernels); 0: the tuning's
   int fwd_warpgroups = 0;
-  // Re-projections: room for the column form's sigmas, of col_rays rays (whole
-  // strips of 32 detector rows) at a time; null: none.
+  // Re-projections: room for the column form's sigmas, of col_rays rays (groups of
+  // 32) at a time; null: none.
   float* col_sigma = nullptr;
   int col_rays = 0;
   // the encoders may fetch corners through a texture object over the table

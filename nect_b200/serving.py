@@ -219,12 +219,11 @@ def reproject(model: _HashGridModel, geometry, angle: float, t: float = 0.0, poi
         need = _lib.lib.nectb_train_workspace_bytes(ctypes.byref(cg.c_struct), ctypes.byref(model.grid_desc),
                                                     ctypes.byref(model.mlp_desc), P)
         if workspace is None or workspace.numel() < need:
-            # with room for the sigmas of some strips of 32 detector rows, a mixed model's view runs
-            # them column by column (at most VIEW_SIGMA_BYTES, or one strip; results do not depend on it)
+            # with room for the sigmas of many groups of 32 rays, a mixed model's view runs them column
+            # by column (at most VIEW_SIGMA_BYTES; results do not depend on it)
             extra = 0
             if model.precision == "mixed" and max_blocks == 0:
-                strip = 4 * 32 * geometry.nDetector[1] * S
-                extra = 256 + min(-(-geometry.nDetector[0] // 32), max(VIEW_SIGMA_BYTES // strip, 1)) * strip
+                extra = 256 + min(-(-P // 32) * 32 * S * 4, VIEW_SIGMA_BYTES)
             with torch.cuda.stream(stream):   # the workspace belongs to the stream that uses it
                 try:
                     workspace = torch.empty(need + extra, dtype=torch.uint8, device=dev)
