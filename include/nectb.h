@@ -366,14 +366,17 @@ typedef struct NectbTrainBatch {
   float loss_scale;                 /* multiplies dL/dy (1 = plain mean) */
 } NectbTrainBatch;
 
+/* Bytes of a training (or re-projection) workspace of num_rays rays, which starts
+ * on an 8-byte boundary. */
 size_t nectb_train_workspace_bytes(const NectbGeometry* geometry, const NectbHashGrid* grid,
                                    const NectbMLP* mlp, int32_t num_rays);
 
 /* Recommended staging bytes for the mixed path's two-pass backward, to add to
  * nectb_train_workspace_bytes(): the rays with samples are listed in
- * scheduling order (detector pixels, or batch positions when the batch
- * repeats a pixel) and the backward runs in rounds of equal ray counts
- * (NectbTuning::staged_rounds, 4 by default);
+ * scheduling order (the detector in strips of 32 rows, column by column, or
+ * batch positions when the batch repeats a pixel) and the backward runs in
+ * rounds of equal ray counts (NectbTuning::staged_rounds, 4 by default, fewer
+ * where a round would stage less than 1 GiB);
  * each round's tensor-core pass writes dL/d(encoding) of its samples (fp32,
  * num_points_per_ray, rounded up to a multiple of 4, * n_levels * n_features
  * per ray) and a scatter over level groups applies it to grid_grad with the
@@ -383,8 +386,8 @@ size_t nectb_train_workspace_bytes(const NectbGeometry* geometry, const NectbHas
  * reads it back instead of gathering the tables a second time (identical
  * values); the store has a row for every sample slot (num_rays *
  * num_points_per_ray), capped at 80 GiB, and rays whose rows do not fit
- * gather again.  A smaller buffer gets fewer store rows, then no store, then
- * more rounds; when it would take more than 64 rounds the single-pass
+ * gather again.  A smaller buffer gets up to staged_rounds rounds, then fewer
+ * store rows, then no store, then more rounds; when it would take more than 64 rounds the single-pass
  * backward (scatter inside the tensor-core kernel) runs instead.  The split
  * between store and rounds follows the buffer size and staged_rounds, so a
  * split step's two halves take the same workspace size with the tuning

@@ -129,15 +129,17 @@ inline StageLayout stage_layout(const Workspace& ws, int R, int P, int S, size_t
                                 int rounds, bool store = true) {
   StageLayout L;
   const size_t ob = order_bytes(R, P);
-  if (!ws.stage || ws.stage_bytes <= ob || R <= 0) return L;
-  char* p = reinterpret_cast<char*>(ws.stage);
+  // 16-byte aligned rows, stored and staged, whatever the caller's workspace pointer
+  const uintptr_t start = reinterpret_cast<uintptr_t>(ws.stage), skip = ((start + 15) & ~uintptr_t(15)) - start;
+  if (!ws.stage || ws.stage_bytes <= ob + skip || R <= 0) return L;
+  char* p = reinterpret_cast<char*>(ws.stage) + skip;
   const size_t nb = (size_t)order_blocks(R, P) + 1;
   L.order = reinterpret_cast<int32_t*>(p);
   L.block_sums = reinterpret_cast<unsigned int*>(p + align256((size_t)R * 4));
   L.offs = reinterpret_cast<uint64_t*>(p + align256((size_t)R * 4) + align256(nb * 4));
   L.block_samples = reinterpret_cast<unsigned long long*>(p + align256((size_t)R * 4) + align256(nb * 4) +
                                                           align256((size_t)R * 8));
-  const size_t avail = ws.stage_bytes - ob;
+  const size_t avail = ws.stage_bytes - ob - skip;
   size_t want = staged_round_bytes(R, rounds, per_ray);
   // rows before large rounds: 65,536 rays x 256 samples on a 4D grid of 16 x 2 levels, in half of
   // the recommended size, 8.67 ms a step with rounds of kStagedRoundMin and no rows, 6.26 with them
@@ -152,10 +154,8 @@ inline StageLayout stage_layout(const Workspace& ws, int R, int P, int S, size_t
       L.xstore = reinterpret_cast<uint4*>(p + ob);
     }
   }
-  // 16-byte aligned rows whatever the caller's workspace pointer
-  const uintptr_t at = reinterpret_cast<uintptr_t>(p + ob + xbytes), pad = ((at + 15) & ~uintptr_t(15)) - at;
-  L.stage = reinterpret_cast<float*>(at + pad);
-  L.per_round = avail < xbytes + pad ? 0 : std::min<int64_t>((int64_t)((avail - xbytes - pad) / per_ray), R);
+  L.stage = reinterpret_cast<float*>(p + ob + xbytes);
+  L.per_round = avail < xbytes ? 0 : std::min<int64_t>((int64_t)((avail - xbytes) / per_ray), R);
   if (L.per_round <= 0 || (R + L.per_round - 1) / L.per_round > kMaxStagedRounds) {
     L.per_round = 0;
     L.xstore = nullptr;

@@ -138,3 +138,14 @@ def test_tiles_of_a_stretch(plan, chunks, stretches, blocks):
                                       (2000, 65536, 1), (65536, 65536, 1), (1, 2**31 - 1, 32), (0, 65536, 32)])
 def test_claims(plan, R, P, want):
     assert plan.claim(R, P) == want
+
+
+@pytest.mark.parametrize("shift", [0, 4, 8, 12, 20, 248])
+def test_rows_are_aligned_in_any_workspace(plan, shift):
+    """Stored rows (rows * 16 bytes) and staged ones start on 16-byte boundaries (checked in
+    layout()) and stay inside the region, whatever the workspace's address."""
+    R, S, row, per_ray, P = 700, 64, 64, 64 * 128, 4096
+    full = plan.order(R, P) + plan.recommended(R, 4, per_ray) + 256 + R * S * row
+    for size in (full, full + 16, full - 8, full // 2, full // 5):
+        layout(plan, size, R, P, S, row, per_ray, 4, at=(1 << 40) + shift)
+    assert layout(plan, full, R, P, S, row, per_ray, 4, at=(1 << 40) + shift) == (R * S, R)

@@ -118,3 +118,49 @@ def test_rows_of_small_workspaces(cuda_device, dims, F, store):
     assert torch.equal(got[0][0], got[1][0])
     for a, b in zip(got[0][1:], got[1][1:]):
         assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
+
+
+@pytest.mark.parametrize("dims", [3, 4])
+@pytest.mark.parametrize("shift", [8, 24])
+def test_workspace_aligned_to_eight_bytes(cuda_device, dims, shift):
+    """A workspace that starts on an 8-byte boundary: the same predictions bit for bit, and
+    gradients within the bound above."""
+    from nect_b200.config import HashEncoderConfig, MLPNetConfig
+    from nect_b200.network import HashGrid, HashGrid4D
+    from nect_b200.sampling import Geometry
+    from nect_b200.trainer import RayBatch, Workspace, train_step
+
+    class Shifted(Workspace):
+        def get(self, *a, **k):
+            _, n = super().get(*a, **k)
+            self.whole = torch.empty(n + 64, dtype=torch.uint8, device="cuda")
+            return self.whole.data_ptr() + shift, n
+
+        def error_word(self):
+            return 0   # (its address is that of the unshifted workspace)
+
+    R, S, P = 700, 65, 40 * 48
+    geo = Geometry(nDetector=[40, 48], dDetector=[1.5, 1.5], mode="cone", DSD=300.0, DSO=200.0, nVoxel=[32] * 3,
+                   dVoxel=[1.0] * 3)
+    enc = HashEncoderConfig(n_levels=16, n_features_per_level=2, log2_hashmap_size=12, base_resolution=4,
+                            finest_resolution=256, base_resolution_t=2 if dims == 4 else None)
+    m = (HashGrid if dims == 3 else HashGrid4D)(enc, MLPNetConfig(n_hidden_layers=2), precision="mixed",
+                                                device="cuda", seed=0)
+    with torch.no_grad():
+        m.table.normal_(0.0, 0.3, generator=torch.Generator(device="cuda").manual_seed(1))
+        m.refresh_half()
+    g = torch.Generator(device="cuda").manual_seed(2)
+    batch = RayBatch(perm=torch.randperm(P, device="cuda", generator=g), start=0, num_rays=R, points_per_ray=S,
+                     angle=0.7, max_ray_distance_per_point=geo.max_distance_traveled / S,
+                     jitter=torch.rand(R, device="cuda", generator=g) - 0.5,
+                     detector_offset=torch.zeros(R, 2, device="cuda"),
+                     projection=torch.rand(P, device="cuda", generator=g), t=0.3)
+    got = []
+    for ws in (Shifted(), Workspace()):
+        tg, mg = torch.zeros_like(m.table), torch.zeros_like(m.mlp)
+        _, y = train_step(m, geo.get_c_geometry(), batch, geo.max_distance_traveled, tg, mg, ws, "l2")
+        assert ws.error_word() == 0
+        got.append((y, tg, mg))
+    assert torch.equal(got[0][0], got[1][0])
+    for a, b in zip(got[0][1:], got[1][1:]):
+        assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
