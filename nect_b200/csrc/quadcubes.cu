@@ -200,8 +200,9 @@ struct EncodeRows {
 };
 
 // Encodes the block's points level by level (level(l, acc) gives this thread's
-// features) and writes rows [col0, col0 + L * F) of its warp's points.
-template <int F, typename O, typename Level>
+// features) and writes rows [col0, col0 + L * F) of its warp's points.  kFew: the blocks
+// along grid y take kEncodeLevels levels each (encode_few).
+template <bool kFew, int F, typename O, typename Level>
 __device__ __forceinline__ void encode_rows(EncodeRows<F, O>& rows, int n_levels, int64_t n, O* __restrict__ out,
                                             int64_t ld, int col0, Level&& level) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -209,7 +210,7 @@ __device__ __forceinline__ void encode_rows(EncodeRows<F, O>& rows, int n_levels
   if (i0 >= n) return;   // warp-uniform
   const int here = (int)min((int64_t)32, n - i0);
   auto& mine = rows.unit[warp];
-  for (int l0 = 0; l0 < n_levels; l0 += kEncodeLevels) {
+  for (int l0 = kFew ? kEncodeLevels * blockIdx.y : 0; l0 < n_levels; l0 += kEncodeLevels * (kFew ? gridDim.y : 1)) {
     const int nl = min(kEncodeLevels, n_levels - l0);
     if (lane < here) {
 #pragma unroll 2   // two levels' gathers in flight
@@ -238,14 +239,14 @@ __device__ __forceinline__ void encode_rows(EncodeRows<F, O>& rows, int n_levels
 }
 
 // The plane grid's features of (zyx[ca], zyx[cb]) into out[i * ld + col0 + l * F + f].
-template <int F, typename P, typename O>
+template <int F, typename P, typename O, bool kFew>
 __global__ void __launch_bounds__(kEncodeThreads)
 plane_encode_kernel(Plane s, const P* __restrict__ plane, const float* __restrict__ zyx, int64_t n,
                     int ca, int cb, O* __restrict__ out, int64_t ld, int col0) {
   __shared__ EncodeRows<F, O> rows;
   const int64_t i = min(blockIdx.x * (int64_t)blockDim.x + threadIdx.x, n - 1);
   const float a = zyx[i * 3 + ca], b = zyx[i * 3 + cb];
-  encode_rows<F, O>(rows, s.n_levels, n, out, ld, col0, [&](int l, float* acc) {
+  encode_rows<kFew, F, O>(rows, s.n_levels, n, out, ld, col0, [&](int l, float* acc) {
     PlaneCorners pc;
     plane_corners(s, l, a, b, pc);
     float v[4][F];
@@ -263,14 +264,14 @@ plane_encode_kernel(Plane s, const P* __restrict__ plane, const float* __restric
 // The (z, y, x) grid's features into columns [0, L * F) of the rows, the raw inputs
 // (z, y, x, t) after the four grids when `identity`, and zeros from column `pad` to
 // the end of the row.
-template <int F, typename O>
+template <int F, typename O, bool kFew>
 __global__ void __launch_bounds__(kEncodeThreads)
 volume_encode_kernel(GridDev g, const float* __restrict__ table, const float* __restrict__ zyx,
                      const float* __restrict__ t, int64_t n, int identity, O* __restrict__ out, int64_t ld, int pad) {
   __shared__ EncodeRows<F, O> rows;
   const int64_t i = min(blockIdx.x * (int64_t)blockDim.x + threadIdx.x, n - 1);
   const float x[3] = {zyx[i * 3], zyx[i * 3 + 1], zyx[i * 3 + 2]};
-  encode_rows<F, O>(rows, g.n_levels, n, out, ld, 0, [&](int l, float* acc) {
+  encode_rows<kFew, F, O>(rows, g.n_levels, n, out, ld, 0, [&](int l, float* acc) {
     LevelCorners<3> lc;
     level_corners<3>(g, l, x, lc);
     float v[8][F];
@@ -283,7 +284,7 @@ volume_encode_kernel(GridDev g, const float* __restrict__ table, const float* __
       for (int c = 0; c < 8; ++c) acc[f] = fmaf(lc.w[c], v[c][f], acc[f]);
     }
   });
-  if (blockIdx.x * (int64_t)blockDim.x + threadIdx.x >= n) return;
+  if ((kFew && blockIdx.y > 0) || blockIdx.x * (int64_t)blockDim.x + threadIdx.x >= n) return;
   // the rest of the row, 16 bytes at a time where it starts on such a boundary
   constexpr int kPer = 16 / sizeof(O);
   const int col = 4 * g.n_levels * F;
@@ -304,7 +305,7 @@ volume_encode_kernel(GridDev g, const float* __restrict__ table, const float* __
     if (c < pad ? identity : true) row[c] = value(c);
 }
 
-// The scatters take kWalkPoints consecutive points a block, each of its warps some
+// The scatters take 32 * kWalkSegment consecutive points a block, each of its warps some
 // levels of all of them.  Where most points lie next to their predecessor (a ray's
 // samples, as the module loop passes them) a lane marches over kWalkSegment
 // consecutive points with its cell's vertex sums in registers (CellMarch,
@@ -312,8 +313,7 @@ volume_encode_kernel(GridDev g, const float* __restrict__ table, const float* __
 // points in one cell.  4,882 rays x 512 samples, 23 levels x 4 features, 2^19 entries,
 // against the merging form alone: the volume 1.25 -> 0.98 ms, the planes 1.68 -> 1.41
 // (bound by the L1's lines: every lane reads its own row and reduces its own entries).
-constexpr int kWalkSegment = 16;
-constexpr int kWalkPoints = 32 * kWalkSegment;
+constexpr int kWalkSegment = 16, kWalkSegmentFew = 4;   // (few points: walk_few)
 constexpr float kWalkStep = 1.f / 64.f;   // largest |dz| + |dy| + |dx| to a neighbour
 constexpr int kWalkWarps = 12;
 constexpr int kPlaneWarps = 6;   // of two levels each
@@ -321,21 +321,24 @@ constexpr int kPlaneWarps = 6;   // of two levels each
 // The block's points: point k of lane l's segment at [c][33 k + l], so that a warp
 // reads them without bank conflicts (the lanes' points are kWalkSegment apart in
 // memory, and the L1's lines are what bounds the walk).
+template <int kSegment>
 struct WalkPoints {
-  float c[3][kWalkSegment * 33];
+  float c[3][kSegment * 33];
 };
 
 // Loads the block's points; whether they are walked through (block-uniform).
-__device__ __forceinline__ bool walks(WalkPoints& pts, const float* __restrict__ zyx, int64_t p0, int64_t n) {
-  const int values = 3 * (int)min((int64_t)kWalkPoints, n - p0);
+template <int kSegment>
+__device__ __forceinline__ bool walks(WalkPoints<kSegment>& pts, const float* __restrict__ zyx, int64_t p0,
+                                      int64_t n) {
+  const int values = 3 * (int)min((int64_t)32 * kSegment, n - p0);
   for (int e = threadIdx.x; e < values; e += blockDim.x) {
     const int point = e / 3;
-    pts.c[e - 3 * point][point % kWalkSegment * 33 + point / kWalkSegment] = zyx[p0 * 3 + e];
+    pts.c[e - 3 * point][point % kSegment * 33 + point / kSegment] = zyx[p0 * 3 + e];
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
   bool next = false;
-  if (p0 + lane * kWalkSegment + 1 < n) {
+  if (p0 + lane * kSegment + 1 < n) {
     float d = 0.f;
 #pragma unroll
     for (int k = 0; k < 3; ++k) d += fabsf(pts.c[k][33 + lane] - pts.c[k][lane]);
@@ -346,16 +349,16 @@ __device__ __forceinline__ bool walks(WalkPoints& pts, const float* __restrict__
 
 // Gradient of levels [l0, l1) of the (z, y, x) grid: dL/d(features) in
 // columns [0, L * F) of the rows.
-template <int F, typename S>
+template <int F, typename S, int kSegment>
 __global__ void __launch_bounds__(kWalkWarps * 32, 2)
 volume_scatter_kernel(GridDev g, const float* __restrict__ zyx, int64_t n,
                       const S* __restrict__ dout, int64_t ld, float* __restrict__ grad, int l0, int l1) {
-  const int64_t p0 = blockIdx.x * (int64_t)kWalkPoints;
+  const int64_t p0 = blockIdx.x * (int64_t)(32 * kSegment);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  __shared__ WalkPoints pts;
+  __shared__ WalkPoints<kSegment> pts;
   if (walks(pts, zyx, p0, n)) {
-    const int64_t first = p0 + (int64_t)lane * kWalkSegment;
-    const int count = (int)max((int64_t)0, min((int64_t)kWalkSegment, n - first));
+    const int64_t first = p0 + (int64_t)lane * kSegment;
+    const int count = (int)max((int64_t)0, min((int64_t)kSegment, n - first));
     for (int l = l0 + warp; l < l1; l += warps) {
       auto march = [&](auto hashed) {
         CellMarch<3, F, hashed()> m(g, l, grad, 0.f);
@@ -381,7 +384,7 @@ volume_scatter_kernel(GridDev g, const float* __restrict__ zyx, int64_t n,
     return;
   }
   for (int l = l0 + warp; l < l1; l += warps)
-    for (int k = 0; k < kWalkSegment; ++k) {   // every lane takes part in the warp's shuffles
+    for (int k = 0; k < kSegment && p0 + 32 * k < n; ++k) {   // every lane takes part in the warp's shuffles
       const int64_t i = p0 + 32 * k + lane;
       const bool valid = i < n;
       float p[3];
@@ -504,19 +507,19 @@ struct PlaneMarch {
 // a warp takes two levels.  Points that do not walk: on levels where a warp's 32
 // points form at most 24 runs of equal cells, each run's sums are reduced once by
 // its first lane.
-template <int F, typename S>
+template <int F, typename S, int kSegment>
 __global__ void __launch_bounds__(kPlaneWarps * 32)
 plane_scatter_kernel(Plane s, const float* __restrict__ zyx, int64_t n, int ca, int cb,
                      const S* __restrict__ dout, int64_t ld, int col0, float* __restrict__ pgrad) {
-  const int64_t p0 = blockIdx.x * (int64_t)kWalkPoints;
+  const int64_t p0 = blockIdx.x * (int64_t)(32 * kSegment);
   const int lane = threadIdx.x & 31, l0 = 2 * (int)(blockIdx.y * kPlaneWarps + (threadIdx.x >> 5));
   const int nl = min(2, s.n_levels - l0);
-  __shared__ WalkPoints pts;
+  __shared__ WalkPoints<kSegment> pts;
   const bool walk = walks(pts, zyx, p0, n);
   if (nl <= 0) return;
   if (walk) {
-    const int64_t first = p0 + (int64_t)lane * kWalkSegment;
-    const int count = (int)max((int64_t)0, min((int64_t)kWalkSegment, n - first));
+    const int64_t first = p0 + (int64_t)lane * kSegment;
+    const int count = (int)max((int64_t)0, min((int64_t)kSegment, n - first));
     PlaneMarch<F> m[2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) m[q].init(s, min(l0 + q, s.n_levels - 1), pgrad);
@@ -543,7 +546,7 @@ plane_scatter_kernel(Plane s, const float* __restrict__ zyx, int64_t n, int ca, 
     m[1].finish();
     return;
   }
-  for (int k = 0; k < kWalkSegment; ++k) {
+  for (int k = 0; k < kSegment && p0 + 32 * k < n; ++k) {
     const int64_t i = p0 + 32 * k + lane;
     const bool valid = i < n;
     const float a = valid ? zyx[i * 3 + ca] : 0.f, b = valid ? zyx[i * 3 + cb] : 0.f;
@@ -668,19 +671,24 @@ int check_grid(const NectbHashGrid* grid, GridDev* g, Plane* s) {
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
-template <int F, typename P, typename O>
+// Whether the encoders' blocks take kEncodeLevels levels of their points in place of all:
+// where one of all would not give every SM a block (23 levels x 4 features, 2^17 entries,
+// the whole call: 10,240 points 147 -> 82 us, 30,720 142 -> 94; 37,888 at the line).
+bool encode_few(int64_t n) { return ceil_div(n, kEncodeThreads) < 148; }
+
+template <int F, typename P, typename O, bool kFew>
 int encode_all(const GridDev& g, const Plane& s, const float* const* tables, const float* zyx, int64_t n,
                const float* t, int identity, O* out, int64_t ld, P* plane, cudaStream_t st) {
-  const unsigned blocks = (unsigned)ceil_div(n, kEncodeThreads);
+  const dim3 blocks((unsigned)ceil_div(n, kEncodeThreads), kFew ? (unsigned)ceil_div(g.n_levels, kEncodeLevels) : 1u);
   const int LF = g.n_levels * F;
-  volume_encode_kernel<F, O><<<blocks, kEncodeThreads, 0, st>>>(g, tables[0], zyx, t, n, identity, out, ld,
-                                                     4 * LF + (identity ? 4 : 0));
+  volume_encode_kernel<F, O, kFew><<<blocks, kEncodeThreads, 0, st>>>(g, tables[0], zyx, t, n, identity, out, ld,
+                                                                      4 * LF + (identity ? 4 : 0));
   if (int rc = launch_status("volume_encode_kernel")) return rc;
   for (int k = 0; k < 3; ++k) {
     plane_build_kernel<F, P><<<plane_grid(s), 256, 0, st>>>(s, tables[k + 1], t, plane);
     if (int rc = launch_status("plane_build_kernel")) return rc;
-    plane_encode_kernel<F, P, O><<<blocks, kEncodeThreads, 0, st>>>(s, plane, zyx, n, kPlaneCols[k][0], kPlaneCols[k][1], out,
-                                                          ld, (k + 1) * LF);
+    plane_encode_kernel<F, P, O, kFew><<<blocks, kEncodeThreads, 0, st>>>(
+        s, plane, zyx, n, kPlaneCols[k][0], kPlaneCols[k][1], out, ld, (k + 1) * LF);
     if (int rc = launch_status("plane_encode_kernel")) return rc;
   }
   return NECTB_OK;
@@ -688,10 +696,16 @@ int encode_all(const GridDev& g, const Plane& s, const float* const* tables, con
 
 constexpr int64_t kScatterGroupBytes = int64_t(64) << 20;
 
-template <int F, typename S>
+// Whether the scatters' blocks take segments of kWalkSegmentFew points: where those of
+// kWalkSegment would give fewer than three blocks to two SMs (23 levels x 4 features, 2^17
+// entries, encode and backward: 10,240 points along rays 376 -> 232 us, loose 385 -> 247;
+// 76,800 421 -> 416 and 651 -> 583; 148,480 along rays 589 with 16 points, 596 with four).
+bool walk_few(int64_t n) { return 2 * ceil_div(n, 32 * kWalkSegment) < 3 * 148; }
+
+template <int F, typename S, int kSegment>
 int backward_all(const GridDev& g, const Plane& s, const float* zyx, int64_t n, const float* t, const S* dout,
                  int64_t ld, float* const* grads, float* pgrad, cudaStream_t st) {
-  const unsigned blocks = (unsigned)ceil_div(n, 256), walk_blocks = (unsigned)ceil_div(n, kWalkPoints);
+  const unsigned blocks = (unsigned)ceil_div(n, 256), walk_blocks = (unsigned)ceil_div(n, 32 * kSegment);
   const dim3 plane_blocks(walk_blocks, (unsigned)ceil_div(s.n_levels, 2 * kPlaneWarps));
   const int LF = g.n_levels * F;
   // One pass per group of consecutive levels whose gradient slice is at most
@@ -715,16 +729,16 @@ int backward_all(const GridDev& g, const Plane& s, const float* zyx, int64_t n, 
         if (int rc = launch_status("volume_scatter_half_kernel")) return rc;
       }
     } else {
-      volume_scatter_kernel<F, S><<<walk_blocks, 32 * std::min(l1 - l0, kWalkWarps), 0, st>>>(g, zyx, n, dout, ld,
-                                                                                              grads[0], l0, l1);
+      volume_scatter_kernel<F, S, kSegment><<<walk_blocks, 32 * std::min(l1 - l0, kWalkWarps), 0, st>>>(
+          g, zyx, n, dout, ld, grads[0], l0, l1);
       if (int rc = launch_status("volume_scatter_kernel")) return rc;
     }
     l0 = l1;
   }
   for (int k = 0; k < 3; ++k) {
     if (int rc = cuda_status(cudaMemsetAsync(pgrad, 0, (size_t)s.total2 * F * 4, st), "cudaMemsetAsync")) return rc;
-    plane_scatter_kernel<F, S><<<plane_blocks, 32 * kPlaneWarps, 0, st>>>(s, zyx, n, kPlaneCols[k][0], kPlaneCols[k][1], dout, ld,
-                                                        (k + 1) * LF, pgrad);
+    plane_scatter_kernel<F, S, kSegment><<<plane_blocks, 32 * kPlaneWarps, 0, st>>>(
+        s, zyx, n, kPlaneCols[k][0], kPlaneCols[k][1], dout, ld, (k + 1) * LF, pgrad);
     if (int rc = launch_status("plane_scatter_kernel")) return rc;
     plane_spread_kernel<F><<<plane_grid(s), 256, 0, st>>>(s, t, pgrad, grads[k + 1]);
     if (int rc = launch_status("plane_spread_kernel")) return rc;
@@ -766,16 +780,16 @@ extern "C" int nectb_quadcubes_encode(const NectbHashGrid* grid, const float* co
   cudaStream_t st = (cudaStream_t)stream;
   ProfScope ps(kProfModel, st);
   const int id = identity ? 1 : 0;
-  if (out_dtype == NECTB_F32) {
-    float* o = (float*)out;
-    float* pl = (float*)workspace;
-    return F == 2 ? encode_all<2>(g, s, tables, zyx, n, t, id, o, out_ld, pl, st)
-                  : encode_all<4>(g, s, tables, zyx, n, t, id, o, out_ld, pl, st);
-  }
-  __nv_bfloat16* o = (__nv_bfloat16*)out;
-  __half* pl = (__half*)workspace;
-  return F == 2 ? encode_all<2>(g, s, tables, zyx, n, t, id, o, out_ld, pl, st)
-                : encode_all<4>(g, s, tables, zyx, n, t, id, o, out_ld, pl, st);
+  auto run = [&](auto f, auto* o, auto* pl) {
+    using P = std::decay_t<decltype(*pl)>;
+    using O = std::decay_t<decltype(*o)>;
+    return encode_few(n) ? encode_all<f(), P, O, true>(g, s, tables, zyx, n, t, id, o, out_ld, pl, st)
+                         : encode_all<f(), P, O, false>(g, s, tables, zyx, n, t, id, o, out_ld, pl, st);
+  };
+  auto rows = [&](auto* o, auto* pl) {
+    return F == 2 ? run(std::integral_constant<int, 2>{}, o, pl) : run(std::integral_constant<int, 4>{}, o, pl);
+  };
+  return out_dtype == NECTB_F32 ? rows((float*)out, (float*)workspace) : rows((__nv_bfloat16*)out, (__half*)workspace);
 }
 
 extern "C" int nectb_quadcubes_encode_backward(const NectbHashGrid* grid, const float* zyx, int64_t n,
@@ -801,12 +815,14 @@ extern "C" int nectb_quadcubes_encode_backward(const NectbHashGrid* grid, const 
   cudaStream_t st = (cudaStream_t)stream;
   ProfScope ps(kProfModel, st);
   float* pg = (float*)workspace;
-  if (dout_dtype == NECTB_F32) {
-    const float* d = (const float*)dout;
-    return F == 2 ? backward_all<2>(g, s, zyx, n, t, d, dout_ld, grads, pg, st)
-                  : backward_all<4>(g, s, zyx, n, t, d, dout_ld, grads, pg, st);
-  }
-  const __nv_bfloat16* d = (const __nv_bfloat16*)dout;
-  return F == 2 ? backward_all<2>(g, s, zyx, n, t, d, dout_ld, grads, pg, st)
-                : backward_all<4>(g, s, zyx, n, t, d, dout_ld, grads, pg, st);
+  auto run = [&](auto f, const auto* d) {
+    return walk_few(n) ? backward_all<f(), std::decay_t<decltype(*d)>, kWalkSegmentFew>(g, s, zyx, n, t, d, dout_ld,
+                                                                                        grads, pg, st)
+                       : backward_all<f(), std::decay_t<decltype(*d)>, kWalkSegment>(g, s, zyx, n, t, d, dout_ld,
+                                                                                     grads, pg, st);
+  };
+  auto rows = [&](const auto* d) {
+    return F == 2 ? run(std::integral_constant<int, 2>{}, d) : run(std::integral_constant<int, 4>{}, d);
+  };
+  return dout_dtype == NECTB_F32 ? rows((const float*)dout) : rows((const __nv_bfloat16*)dout);
 }
