@@ -1351,17 +1351,21 @@ int run_mixed(const NectbGeometry& geo, const GridDev& grid, const __half* table
                                                           loss);
       return launch_status("fwd_mixed_kernel");
     };
-    // The column form needs neighbouring rays in a warp, so a share of the
-    // detector's pixels in the batch, and units enough for the warps.  A line of
-    // the table holds 32 entries of 2 features, 16 of 4.  Step (training) or view
-    // with the one / the other form, 512 x 512 detector and 512 samples unless
-    // stated: 2 features, all pixels 37.3 / 40.0 ms, a half 20.3 / 21.9, an eighth
-    // 6.20 / 6.37, a sixteenth 4.07 / 3.77; 4D view 14.9 / 23.5, 128 x 128 x 256 (1.7
-    // units a warp) 0.83 / 1.03, 64 x 64 x 64 (0.1) 0.52 / 0.14.  4 features, 256 x
-    // 256 x 256: all pixels 15.8 / 16.3, a half 8.76 / 8.72, a quarter 5.20 / 4.86; 128
-    // x 128 x 512 (3.5 units) 8.07 / 7.80.
-    const int64_t units = ceil_div(R, 32) * ceil_div(a.S, kColumnSegment), warps = (int64_t)fblocks * wgs * 4;
-    const bool columns = F == 2 ? 2 * units >= 3 * warps && 5 * (int64_t)R >= a.n_pixels
+    // The column form needs a warp's rays close together (a line of the table holds 32
+    // entries of 2 features, 16 of 4) and units enough for the warps.  2 features: the rays
+    // a 64th of the detector's height apart at most, and no more than every eighth pixel;
+    // steps of 512 samples with the one / the other form, ms, on 512 x 512 pixels: all 36.4 /
+    // 39.1, a half 19.3 / 20.5, an eighth 5.39 / 5.52, a twelfth 3.74 / 3.74, a sixteenth
+    // 2.99 / 2.88; on 256 x 256: all 10.0 / 10.6, a third 3.89 / 3.92, a quarter 3.10 / 3.06, a
+    // fifth 2.75 / 2.57, an eighth 1.84 / 1.80.  4D view, 512 x 512 x 512: 14.9 / 23.5, 128 x
+    // 128 x 256 (1.7 units a warp) 0.83 / 1.03, 64 x 64 x 64 (0.1) 0.52 / 0.14.  4 features, 3
+    // layers, 256 x 256 x 512: all 15.0 / 15.3, a half 7.88 / 8.00, a quarter 4.29 / 4.19; 2
+    // layers, 128 x 128 x 512 (3.5 units) 8.07 / 7.80.  A view counts the units of the rays its
+    // sigmas' room holds at a time.
+    const int64_t at_once = a.col_sigma ? std::min(R, a.col_rays) : R;
+    const int64_t units = ceil_div(at_once, 32) * ceil_div(a.S, kColumnSegment), warps = (int64_t)fblocks * wgs * 4;
+    const int64_t apart = std::max(1, std::min(8, a.n_pixels / (a.n_cols * a.sub) / 64));   // pixels to a ray
+    const bool columns = F == 2 ? 2 * units >= 3 * warps && apart * R >= a.n_pixels
                                 : units >= 4 * warps && 2 * (int64_t)R > a.n_pixels;
     const size_t sigma_bytes = (size_t)ceil_div(R, 32) * 32 * a.S * sizeof(float);
     Columns cols;
