@@ -111,7 +111,7 @@ __global__ void encode_backward_kernel(GridDev g, const float* __restrict__ x, i
 #pragma unroll
   for (int k = 0; k < D; ++k) p[k] = valid ? x[i * D + k] : 0.f;
   const int64_t row = valid ? i : 0;
-  scatter_warp<D, F, false, true>(g, grad, p, valid, dout + row * (int64_t)g.n_levels * F, F, 1, 0u, 0,
+  scatter_warp<D, F, true>(g, grad, p, valid, dout + row * (int64_t)g.n_levels * F, F, 1, 0u, 0,
                                   g.n_levels);
 }
 

@@ -295,10 +295,7 @@ __device__ __forceinline__ float run_sum(float v, int lane, int end) {
 // fp32 reassociation.
 //
 // dL/d(feature f of level l) is read at dsrc[l * lstride + f * fstride] (fp32,
-// or bf16 with S = __nv_bfloat16); only levels [l0, l1) are scattered.  kStreamSrc: dsrc is global memory read once
-// (the staging buffer, fstride 1, rows aligned to F floats): one vector load
-// per level, evict-first, so the streamed rows do not push the gradient slice
-// out of L2.
+// or bf16 with S = __nv_bfloat16); only levels [l0, l1) are scattered.
 //
 // kAdaptive: agg_levels is ignored; every level merges runs when the warp's
 // 32 points form at most 24 runs of equal cells (points in no known order,
@@ -306,29 +303,17 @@ __device__ __forceinline__ float run_sum(float v, int lane, int end) {
 //
 // kVecSrc: fstride is 1 and each level's F elements are one aligned vector
 // (load_grad_row).
-template <int D, int F, bool kStreamSrc = false, bool kAdaptive = false, typename S = float, bool kVecSrc = false>
+template <int D, int F, bool kAdaptive = false, typename S = float, bool kVecSrc = false>
 __device__ __forceinline__ void scatter_warp(const GridDev& g, float* __restrict__ grad, const float* x, bool valid,
                                              const S* dsrc, int64_t lstride, int fstride, uint32_t agg_levels,
                                              int l0, int l1) {
-  static_assert(!kStreamSrc || sizeof(S) == 4, "the streamed source is fp32");
   const int lane = threadIdx.x & 31;
 #pragma unroll 1
   for (int l = l0; l < l1; ++l) {
     LevelCorners<D> lc;
     level_corners<D>(g, l, x, lc);
     float d[F];
-    if constexpr (kStreamSrc && F == 2) {
-      const float2 v = valid ? __ldcs(reinterpret_cast<const float2*>(dsrc + l * lstride)) : make_float2(0.f, 0.f);
-      d[0] = v.x;
-      d[1] = v.y;
-    } else if constexpr (kStreamSrc && F == 4) {
-      const float4 v =
-          valid ? __ldcs(reinterpret_cast<const float4*>(dsrc + l * lstride)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      d[0] = v.x;
-      d[1] = v.y;
-      d[2] = v.z;
-      d[3] = v.w;
-    } else if constexpr (kVecSrc) {
+    if constexpr (kVecSrc) {
       if (valid) {
         load_grad_row<F, S>(dsrc + l * lstride, d);
       } else {

@@ -390,7 +390,7 @@ volume_scatter_kernel(GridDev g, const float* __restrict__ zyx, int64_t n,
       float p[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) p[c] = valid ? zyx[i * 3 + c] : 0.f;
-      scatter_warp<3, F, false, true, S, true>(g, grad, p, valid, dout + (valid ? i : 0) * ld, F, 1, 0u, l, l + 1);
+      scatter_warp<3, F, true, S, true>(g, grad, p, valid, dout + (valid ? i : 0) * ld, F, 1, 0u, l, l + 1);
     }
 }
 

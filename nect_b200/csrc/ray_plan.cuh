@@ -80,8 +80,8 @@ struct Workspace {
   RayRec* rays;
   int32_t* slot;
   unsigned int* counters;  // [0] forward cursor, [1] backward cursor, [2] error word, [3] flags,
-                           // [5] scatter cursor, [6] rays with samples, [7] encoding-store rows
-                           // the forward filled, [8] forward loss sum (split step),
+                           // [6] rays with samples, [7] encoding-store rows the forward
+                           // filled, [8] forward loss sum (split step),
                            // [9] chunks of 32 samples (about)
   float* stage = nullptr;
   size_t stage_bytes = 0;

@@ -223,9 +223,10 @@ __device__ __forceinline__ int next_ray(SlotClaim& claim, unsigned int* cursor, 
 // The rays with samples in scheduling order, for the two-pass backward's
 // rounds of equal ray counts: order[rank] = ray, ranks 0..ctrl[6]-1, and
 // offs[rank] = samples of the rays ranked before it (the ray's first row in
-// the encoding store).  Three launches over the scheduling indices (pixels,
-// or batch positions when the batch repeats a pixel): per-block counts, one
-// block scanning them, and the per-block compaction, so pixel order is kept.
+// the encoding store).  Three launches over the scheduling indices (strips of
+// the detector, strip_slot, or batch positions when the batch repeats a pixel):
+// per-block counts, one block scanning them, and the per-block compaction, so
+// that order is kept.
 __global__ void order_count_kernel(const int32_t* __restrict__ slot, const RayRec* __restrict__ recs,
                                    const unsigned int* __restrict__ ctrl, int R, int P, int cols, int sub,
                                    unsigned int* __restrict__ block_sums,

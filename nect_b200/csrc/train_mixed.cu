@@ -44,9 +44,6 @@ constexpr int kMixThreads = 128;
 constexpr int kScatterThreads = 128;
 constexpr int kScatterSegment = 32;
 constexpr int kColumnSegment = 32;   // samples of a column unit of the forward
-#ifndef UNR
-#define UNR 1
-#endif
 // Per-warp ray cursor shared by the mixed kernels.
 struct RayCursor {
   int ray = -1;
