@@ -19,17 +19,18 @@ bracketed by a barrier and cuda synchronize, CUDA events on the launching
 stream, max over ranks.  Per-step state (tables, gradients, Adam moments)
 exceeds the 126 MB L2, so consecutive steps do not hit a warm L2.
 
-Rooflines: the encoding's corner gathers and the gradient scatter's
-reductions are served by the L2 (the table and one scatter pass's gradient
-slice are L2-sized), so their roofs are measured here, before the timed
-region, by the library's probes: random gathers of the table's entry size
-from a buffer of the fp16 table's size, and random fp32 reductions of the
-gradient's entry size into a buffer of one scatter pass's slice.  Achieved =
-algorithmic bytes per launch (per valid sample: L * 2^d * F * 2 bytes for the
-forward, L * 2^d * F * 4 bytes for the scatter) / the kernel's mean CUDA-event
-launch time.  The tensor-core backward is reported against the measured bf16
-peak (MLP flops per sample: the forward recompute and the two backward
-products).
+Rooflines: the forward and the scatter share table lines between neighbouring
+rays and reduce a vertex once per visit, so neither moves the bytes of every
+sample's corners; what they move through DRAM is measured (an ncu capture,
+profiles/dram_bytes_per_sample.txt, scaled per valid sample) and reported
+against the measured copy bandwidth.  Both are bound by instruction issue, so
+that fraction says how far from the memory's roof they are.  The corners'
+bytes per second (``corner_gbs``: per valid sample L * 2^d * F * 2 bytes for the
+forward, * 4 for the scatter) and the L2's (``l2_gbs``) stand beside it without
+a roof; the L2's rates for random gathers and reductions are measured before
+the timed region (``probes``).  The tensor-core backward is reported against
+the measured bf16 peak (MLP flops per sample: the forward recompute and the two
+backward products).
 
 --impl reference times the reference path's CPU restatement (oracle/
 workloads.py: the C sampler, PyTorch-CPU fp32 hash grid, MLP, autograd and
@@ -506,43 +507,28 @@ def main():
             if len(f) == 4 and not line.startswith("#") and f[:2] == [args.workload, args.precision]:
                 l2_step[f[2]] = float(f[3]) * per_step_samples
 
-    # the 4D mixed step gathers and reduces on the time slice: 8 spatial corners per level, half of the
-    # 16 the 4D interpolation counts (the time blend runs once per table entry and step instead)
-    sliced = spec["n_dims"] == 4 and args.precision == "mixed" and bool(autotune.get_tuning()["time_slice"])
-    executed = {"forward": gather // 2 if sliced else gather, "scatter": scatter // 2 if sliced else scatter}
-
-    def roof(kind, per_sample, peak_name, bound, unit, scale, peak=None, peak_src=None):
+    def roof(kind, per_sample, bound):
         if kind not in kernel_ms:
             return None
         per_launch = per_step_samples * per_sample / launches_per_step[kind]
         secs = kernel_ms[kind] / 1e3
-        achieved = per_launch / secs / scale
-        if peak is None:
-            peak, peak_src = roofs[peak_name]["gbs"], f"measured in this run: {peak_name} probe ({roofs[peak_name]['pattern']}, {roofs[peak_name]['access_bytes']} B, {roofs[peak_name]['buffer_mb']:.0f} MB buffer)"
         tr = traffic_step.get(kind)
-        out = {"bound": bound, "kernel": kind, "achieved": achieved, "peak": peak, "unit": unit,
-               "frac": achieved / peak, "peak_source": peak_src,
-               "traffic": tr / launches_per_step[kind] if tr is not None else None,
-               "algorithmic_per_launch": per_launch, "launch_ms": kernel_ms[kind],
+        traffic = tr / launches_per_step[kind] if tr is not None else None
+        out = {"bound": bound, "kernel": kind, "traffic": traffic, "launch_ms": kernel_ms[kind],
                "launches_per_step": launches_per_step[kind]}
-        if kind in executed:   # the bytes the kernel's own algorithm moves (time slice: 8 corners)
-            ex = per_step_samples * executed[kind] / launches_per_step[kind]
-            out["executed_per_launch"] = ex
-            out["executed_frac"] = ex / secs / scale / peak
-        if tr is not None:
-            out["dram_gbs"] = tr / launches_per_step[kind] / secs / 1e9
-            out["dram_frac_of_hbm"] = out["dram_gbs"] / hbm
-        if kind in l2_step and bound == "l2":
-            out["l2_gbs"] = l2_step[kind] / launches_per_step[kind] / secs / 1e9
-            out["l2_frac"] = out["l2_gbs"] / peak
+        if bound == "tensor":
+            out.update(achieved=per_launch / secs / 1e12, peak=tensor_peak, unit="TFLOP/s",
+                       peak_source=f"{peak_src} bf16 dense, sustained", algorithmic_per_launch=per_launch)
+        else:
+            out.update(achieved=traffic / secs / 1e9 if traffic is not None else None, peak=hbm, unit="GB/s",
+                       peak_source=f"{peak_src} copy bandwidth", corner_gbs=per_launch / secs / 1e9)
+            if kind in l2_step:
+                out["l2_gbs"] = l2_step[kind] / launches_per_step[kind] / secs / 1e9
+        out["frac"] = out["achieved"] / out["peak"] if out["achieved"] is not None else None
         return out
 
-    rooflines = {
-        "forward": roof("forward", gather, "gather_line", "l2", "GB/s", 1e9),
-        "scatter": roof("scatter", scatter, "reduce_line", "l2", "GB/s", 1e9),
-        "backward": roof("backward", 3 * mlp_fwd, None, "tensor", "TFLOP/s", 1e12, tensor_peak,
-                         f"{peak_src} bf16 dense, sustained"),
-    }
+    rooflines = {"forward": roof("forward", gather, "hbm"), "scatter": roof("scatter", scatter, "hbm"),
+                 "backward": roof("backward", 3 * mlp_fwd, "tensor")}
     if args.precision == "plain_fp32":
         rooflines["backward"] = None   # the plain backward is SIMT, no tensor-core roof
     rooflines = {k: v for k, v in rooflines.items() if v}
