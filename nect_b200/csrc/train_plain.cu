@@ -403,9 +403,11 @@ __device__ __forceinline__ void plain_backward(const GridDev& grid, const T* __r
     __syncthreads();
     if constexpr (D == 4) {
       // A thread takes one level of kSegment consecutive samples and marches over
-      // them: 16 reductions a sample and level otherwise (300,007 points along rays:
-      // 0.89 -> 0.78 ms).  With the 8 of 3D, sample by sample is the faster (16,384
-      // rays x 256: 4.58 against 5.31 ms).
+      // them: 16 reductions a sample and level otherwise (300,007 points along rays, 16 x
+      // 2 levels: 0.91 -> 0.81 ms; 16 x 4: 1.43 -> 1.34).  Points in no order, which a
+      // training loop does not pass, lose 3 to 6 % by it (300,007: 1.46 -> 1.52, 16 x 4
+      // 2.24 -> 2.30 ms), 10,000 of either kind nothing.  With the 8 of 3D, sample by
+      // sample is the faster (16,384 rays x 256: 4.58 against 5.31 ms).
       for (int e = t; e < L * (NT / kSegment); e += NTH) {
         const int l = e / (NT / kSegment), first = e % (NT / kSegment) * kSegment;
         auto march = [&](auto hashed) {
