@@ -1232,14 +1232,20 @@ int run_mixed(const NectbGeometry& geo, const GridDev& grid, const __half* table
     // the start of its staging region, and runs without staging.
     const bool piece = args.fwd_warpgroups > 0 && !table_grad;
     const size_t sb = piece ? slice_half_bytes(grid) : slice_bytes(grid);
-    // Beside the slice a step needs a round's room: 16,000 rays x 64 samples, 16 x 2 levels, in 80 MB
-    // take 41 rounds and 2.74 ms on the slice, 4 rounds and 1.19 ms on the 4D grid; 2,000 x 100 in
-    // 80 MB 8 rounds and 0.80 ms, 1 round and 0.34 ms.
-    const size_t rounds =
-        round_bytes(args.num_rays, tune.staged_rounds, (size_t)ray_slots(args.S) * L * F * sizeof(float));
+    // A round costs some 50 us and a workspace allows 64 of them (then the single pass), the slice its
+    // build and spread; it halves the corners. So batches of 2^23 sample slots and more, four times the
+    // slice in staged bytes at least, take it whatever is left beside it; smaller ones where a round of
+    // R / staged_rounds rays fits too. 16 x 2 levels, ms on the slice and on the 4D grid: 262,144 rays x
+    // 512 samples with 12 MB beside the slice 91 and 116, with 3 GB 57 and 106; 65,536 x 256 with 12 MB
+    // 15.1 and 19.8; at the line, 32,768 x 256, with 12 / 24 / 48 / 96 / 192 MB 7.1 / 11.3 / 8.5 / 7.4 /
+    // 6.3 and 10.1 / 10.0 / 9.6 / 8.8 / 7.3; 16,384 x 256 with 12 / 48 / 96 MB 8.9 / 4.8 / 4.3 and 3.6 /
+    // 3.3 / 3.3; 24,999 x 100 with 12 / 48 MB 4.8 / 3.4 and 2.4 / 2.2.
+    const size_t per_ray = (size_t)ray_slots(args.S) * L * F * sizeof(float);
+    const size_t staged = (size_t)args.num_rays * per_ray;
+    const bool large = (int64_t)args.num_rays * args.S >= (int64_t(1) << 23) && staged >= 4 * sb;
+    const size_t round = args.query || large ? 0 : round_bytes(args.num_rays, tune.staged_rounds, per_ray);
     const size_t need = piece ? sb + 512
-                              : sb + order_bytes(args.num_rays, args.n_pixels) +
-                                    std::max(size_t(1) << 20, args.query ? 0 : rounds);
+                              : sb + order_bytes(args.num_rays, args.n_pixels) + std::max(size_t(1) << 20, round);
     if (tune.time_slice && args.max_blocks == 0 && ws.stage && ws.stage_bytes >= need) {
       const TimeSlice ts = make_time_slice(grid, args.t);
       const int64_t n3 = ts.g3.total_entries;
