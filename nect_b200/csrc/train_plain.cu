@@ -213,9 +213,10 @@ constexpr int kPlainFwdSamples = 128;
 // the gathers' latency between them.  16,384 rays x 256 samples, 16 x 2 levels,
 // 2 x 64: 2.49 -> 1.45 ms against one sample a thread, 0.91 ms of it the MLP (its
 // multiply-adds take 0.49 ms).
-// (Three blocks an SM: 80 registers a thread; at 100 the same step 1.49 ms.)
+// Three blocks an SM in 3D: 80 registers a thread; at 100 the same step 1.49 ms.  In 4D,
+// 80 registers spill: 262,144 rays x 512 samples 65.0 ms with three blocks, 54.0 with two.
 template <int D, int F, int L, int H>
-__global__ void __launch_bounds__(kTileThreads, 3)
+__global__ void __launch_bounds__(kTileThreads, D == 4 ? 2 : 3)
 fwd_plain_kernel(GridDev grid, const float* __restrict__ table, const float* __restrict__ W, TrainArgs a,
                  RayRec* __restrict__ recs, const int32_t* __restrict__ slot, unsigned int* __restrict__ ctrl,
                  int act, int out_act, float* __restrict__ y_pred, float* __restrict__ loss) {
